@@ -87,10 +87,8 @@ __global__ void __launch_bounds__(kBlock) k_adj_load(DevPtrs P, int cur, const d
     const unsigned int fx = to_frac(x, rs.frac_per_len[0]), fy = to_frac(y, rs.frac_per_len[1]),
                        fz = to_frac(z, rs.frac_per_len[2]);
     vmax = displacement(P.ref[i], fx, fy, fz, rs);
-    if constexpr (MIXED) {
-      const uint4 me = P.m4[cur][i];
-      P.m4[cur][i] = make_uint4(fx, fy, fz, me.w);
-    } else {
+    P.m4[cur][i] = make_uint4(fx, fy, fz, P.m4[cur][i].w);
+    if constexpr (!MIXED) {
       const double4 me = P.d4[cur][i];
       P.d4[cur][i] = make_double4(x, y, z, me.w);
     }

@@ -260,7 +260,7 @@ __global__ void k_graph_cond(const Global* g, unsigned long long cond) {
 int launch_rebuild(smd_system* h, cudaStream_t st, int cur, int in_graph) {
   auto& P = h->P;
   const int gb = h->bead_grid();
-  SMD_LAUNCH(h, k_bin<<<gb, kBeadBlock, 0, st>>>(P, cur, h->mixed ? 1 : 0, in_graph));
+  SMD_LAUNCH(h, k_bin<<<gb, kBeadBlock, 0, st>>>(P, cur, in_graph));
   if (h->n_cells <= kScanOneMax) {
     SMD_PDL(h, k_scan_one, 1, kScanOneThreads, st, P);
   } else {
@@ -271,13 +271,13 @@ int launch_rebuild(smd_system* h, cudaStream_t st, int cur, int in_graph) {
   if (h->mixed) {
     SMD_PDL(h, k_reorder<true>, gb, kBeadBlock, st, P, cur);
     switch (h->tune.list) {
-      case 1: SMD_PDL(h, k_nbr_cells_flat<256>, h->nbr_grid(), 256, st, P, cur); break;
+      case 1: SMD_PDL(h, (k_nbr_cells_flat<true, 256>), h->nbr_grid(), 256, st, P, cur); break;
       case 2: SMD_PDL(h, k_nbr_cells_oct, h->nbr_grid(), kOctThreads, st, P, cur); break;
-      default: SMD_PDL(h, k_nbr_cells_flat<128>, h->nbr_grid(), 128, st, P, cur); break;
+      default: SMD_PDL(h, (k_nbr_cells_flat<true, 128>), h->nbr_grid(), 128, st, P, cur); break;
     }
   } else {
     SMD_PDL(h, k_reorder<false>, gb, kBeadBlock, st, P, cur);
-    SMD_PDL(h, k_nbr_cells_plain, h->nbr_grid(), kNbrThreads, st, P, cur);
+    SMD_PDL(h, (k_nbr_cells_flat<false, 128>), h->nbr_grid(), 128, st, P, cur);
   }
   return 0;
 }
@@ -891,10 +891,9 @@ int smd_create_batch(const smd_system_desc* descs, int n_rep, int precision, smd
                     &P.tx, &P.ty, &P.tz, &P.tvx, &P.tvy, &P.tvz, &P.tax, &P.tay, &P.taz};
   for (double** q : dbl)
     if ((rc = h->alloc(q, total))) return rc;
-  if (h->mixed) {
-    if ((rc = h->alloc(&P.m4[0], total)) || (rc = h->alloc(&P.m4[1], total)) || (rc = h->alloc(&P.mt, total)))
-      return rc;
-  } else {
+  if ((rc = h->alloc(&P.m4[0], total)) || (rc = h->alloc(&P.m4[1], total)) || (rc = h->alloc(&P.mt, total)))
+    return rc;
+  if (!h->mixed) {
     if ((rc = h->alloc(&P.d4[0], total)) || (rc = h->alloc(&P.d4[1], total)) || (rc = h->alloc(&P.dt4, total)))
       return rc;
   }
@@ -984,7 +983,7 @@ int smd_create_batch(const smd_system_desc* descs, int n_rep, int precision, smd
   {
     std::vector<double> hx(total), hy(total), hz(total), hvx(total), hvy(total), hvz(total);
     std::vector<int> orig(total);
-    std::vector<uint4> m4(h->mixed ? total : 0);
+    std::vector<uint4> m4(total);
     std::vector<double4> d4(h->mixed ? 0 : total);
     std::vector<RepState> rs(n_rep);
     int b = 0;
@@ -1004,10 +1003,9 @@ int smd_create_batch(const smd_system_desc* descs, int n_rep, int precision, smd
         hvz[b] = d.vel[3 * i + 2];
         orig[b] = b;
         const unsigned w = (unsigned)type[b] | ((unsigned)r << 8);
-        if (h->mixed) {
-          auto fr = [](double x, double L) { return (unsigned int)(long long)(x * (1.0 / L) * 4294967296.0); };
-          m4[b] = make_uint4(fr(hx[b], d.box[0]), fr(hy[b], d.box[1]), fr(hz[b], d.box[2]), w);
-        } else {
+        auto fr = [](double x, double L) { return (unsigned int)(long long)(x * (1.0 / L) * 4294967296.0); };
+        m4[b] = make_uint4(fr(hx[b], d.box[0]), fr(hy[b], d.box[1]), fr(hz[b], d.box[2]), w);
+        if (!h->mixed) {
           long long wb = (long long)w;
           double wd;
           std::memcpy(&wd, &wb, sizeof wd);
@@ -1024,9 +1022,8 @@ int smd_create_batch(const smd_system_desc* descs, int n_rep, int precision, smd
     SMD_CUDA(cudaMemcpy(P.orig, orig.data(), total * sizeof(int), cudaMemcpyHostToDevice));
     SMD_CUDA(cudaMemcpy(P.inv, orig.data(), total * sizeof(int), cudaMemcpyHostToDevice));
     SMD_CUDA(cudaMemcpy(P.cinfo, cinfo.data(), total * sizeof(int), cudaMemcpyHostToDevice));
-    if (h->mixed)
-      SMD_CUDA(cudaMemcpy(P.m4[0], m4.data(), total * sizeof(uint4), cudaMemcpyHostToDevice));
-    else
+    SMD_CUDA(cudaMemcpy(P.m4[0], m4.data(), total * sizeof(uint4), cudaMemcpyHostToDevice));
+    if (!h->mixed)
       SMD_CUDA(cudaMemcpy(P.d4[0], d4.data(), total * sizeof(double4), cudaMemcpyHostToDevice));
     SMD_CUDA(cudaMemcpy(P.rp, h->rp.data(), n_rep * sizeof(RepParams), cudaMemcpyHostToDevice));
     SMD_CUDA(cudaMemcpy(P.rs, rs.data(), n_rep * sizeof(RepState), cudaMemcpyHostToDevice));

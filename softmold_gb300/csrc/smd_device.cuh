@@ -3,10 +3,11 @@
 // Per-bead state lives in HBM in cell-sorted order (beads of one replica are
 // contiguous; within a replica they are ordered by Verlet-list cell), FP64 SoA:
 //   x,y,z  vx,vy,vz  ax,ay,az        master state (8 B each)
-//   mirror[2]                        double-buffered 16 B position mirror read
-//                                    by the pair loop: MIXED = uint4 of 32-bit
-//                                    fractional coordinates + (type | replica<<8),
-//                                    PLAIN = double4 (x,y,z,type bits)
+//   m4[2]                            double-buffered 16 B position mirror read
+//                                    by the list build and the pair loop: uint4
+//                                    of 32-bit fractional coordinates +
+//                                    (type | replica<<8)
+//   d4[2]                            PLAIN also: double4 (x,y,z,type bits)
 //   orig / inv                       sorted -> file order and back
 //   cinfo                            CHAIN role of the bead (position, length, set)
 // The Verlet list is bead-major: nbr[i * kmax + k] is neighbour k of bead i.

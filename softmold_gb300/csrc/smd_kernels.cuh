@@ -9,6 +9,7 @@
 #pragma once
 
 #include "smd_device.cuh"
+#include "smd_pair64.cuh"
 
 namespace smd {
 
@@ -71,7 +72,7 @@ __device__ __forceinline__ float displacement(uint4 ref, unsigned int fx, unsign
 // beads are in the previous build's cell order, so the lanes of a warp mostly
 // share a few cells: the lanes of one cell take their slots from one atomic
 // add of the leader (the lowest lane), in lane order.
-__global__ void __launch_bounds__(kBeadBlock) k_bin(DevPtrs P, int cur, int mixed, int in_graph) {
+__global__ void __launch_bounds__(kBeadBlock) k_bin(DevPtrs P, int cur, int in_graph) {
   pdl_trigger();
   if (!P.g->rebuild) return;
   const int i = blockIdx.x * kBeadBlock + threadIdx.x;
@@ -81,19 +82,9 @@ __global__ void __launch_bounds__(kBeadBlock) k_bin(DevPtrs P, int cur, int mixe
   if (!active) return;
   const int r = rep_of(P, i);
   const RepState& rs = P.rs[r];
-  unsigned int f[3];
-  if (mixed) {
-    const uint4 m = P.m4[cur][i];
-    f[0] = m.x;
-    f[1] = m.y;
-    f[2] = m.z;
-  } else {
-    f[0] = to_frac(P.x[i], rs.frac_per_len[0]);
-    f[1] = to_frac(P.y[i], rs.frac_per_len[1]);
-    f[2] = to_frac(P.z[i], rs.frac_per_len[2]);
-  }
+  const uint4 m = P.m4[cur][i];
   const int n0 = rs.ncell[0], n1 = rs.ncell[1], n2 = rs.ncell[2];
-  const int cx = __umulhi(f[0], (unsigned)n0), cy = __umulhi(f[1], (unsigned)n1), cz = __umulhi(f[2], (unsigned)n2);
+  const int cx = __umulhi(m.x, (unsigned)n0), cy = __umulhi(m.y, (unsigned)n1), cz = __umulhi(m.z, (unsigned)n2);
   const int key = P.rp[r].cell_begin + cx + n0 * (cy + n1 * cz);
   P.key[i] = key;
   const unsigned int same = __match_any_sync(lanes, key);
@@ -307,11 +298,8 @@ __global__ void __launch_bounds__(kBeadBlock) k_reorder(DevPtrs P, int cur) {
   P.tcinfo[nw] = P.cinfo[i];
   P.tkey[nw] = P.key[i];
   P.inv[o] = nw;
-  if constexpr (MIXED) {
-    P.mt[nw] = P.m4[cur][i];
-  } else {
-    P.dt4[nw] = P.d4[cur][i];
-  }
+  P.mt[nw] = P.m4[cur][i];
+  if constexpr (!MIXED) P.dt4[nw] = P.d4[cur][i];
 }
 
 // ------------------------------------------------------------ Verlet lists
@@ -355,7 +343,7 @@ __device__ __forceinline__ CellCtx cell_ctx(const DevPtrs& P, int c, int s, int 
 
 // Copies the cell's reordered state back from the scratch arrays.
 template <bool MIXED, int NT>
-__device__ __forceinline__ void copy_back(const DevPtrs& P, int cur, const CellCtx& q, const RepState& rs) {
+__device__ __forceinline__ void copy_back(const DevPtrs& P, int cur, const CellCtx& q) {
   for (int i = q.s + threadIdx.x; i < q.e; i += NT) {
     P.x[i] = P.tx[i];
     P.y[i] = P.ty[i];
@@ -368,72 +356,10 @@ __device__ __forceinline__ void copy_back(const DevPtrs& P, int cur, const CellC
     P.az[i] = P.taz[i];
     P.orig[i] = P.torig[i];
     P.cinfo[i] = P.tcinfo[i];
-    if constexpr (MIXED) {
-      P.m4[cur][i] = P.mt[i];
-      P.ref[i] = P.mt[i];
-    } else {
-      const double4 d = P.dt4[i];
-      P.d4[cur][i] = d;
-      P.ref[i] = make_uint4(to_frac(d.x, rs.frac_per_len[0]), to_frac(d.y, rs.frac_per_len[1]),
-                            to_frac(d.z, rs.frac_per_len[2]), 0u);
-    }
+    P.m4[cur][i] = P.mt[i];
+    P.ref[i] = P.mt[i];
+    if constexpr (!MIXED) P.d4[cur][i] = P.dt4[i];
   }
-}
-
-// The stencil as contiguous bead ranges with prefix sums (one thread): cells
-// are ordered x-fastest, so each (dy,dz) row of 3 cells is one range unless
-// it wraps in x.  Axes with fewer than 3 cells take every cell once.
-__device__ __forceinline__ int stencil_segments(const DevPtrs& P, const CellCtx& q, int* seg_s, int* seg_p) {
-  int nseg = 0;
-  const int lo1 = q.n1 >= 3 ? -1 : 0, hi1 = q.n1 >= 2 ? 1 : 0;
-  const int lo2 = q.n2 >= 3 ? -1 : 0, hi2 = q.n2 >= 2 ? 1 : 0;
-  int xa = q.cx - 1, xb = q.cx + 1;
-  if (q.n0 < 3) {
-    xa = 0;
-    xb = q.n0 - 1;
-  }
-  int acc = 0;
-  for (int oz = lo2; oz <= hi2; ++oz) {
-    const int zz = (q.cz + oz + q.n2) % q.n2;
-    for (int oy = lo1; oy <= hi1; ++oy) {
-      const int yy = (q.cy + oy + q.n1) % q.n1;
-      const int row = q.cb + q.n0 * (yy + q.n1 * zz);
-      int a0, a1, b0 = 0, b1 = 0;
-      if (xa >= 0 && xb < q.n0) {
-        a0 = row + xa;
-        a1 = row + xb + 1;
-      } else if (xa < 0) {  // cells n0-1 | 0..xb
-        a0 = row + q.n0 - 1;
-        a1 = row + q.n0;
-        b0 = row;
-        b1 = row + xb + 1;
-      } else {  // cells xa..n0-1 | 0
-        a0 = row + xa;
-        a1 = row + q.n0;
-        b0 = row;
-        b1 = row + 1;
-      }
-      seg_s[nseg] = P.cell_start[a0];
-      seg_p[nseg] = acc;
-      acc += P.cell_start[a1] - seg_s[nseg];
-      ++nseg;
-      if (b1 > b0) {
-        seg_s[nseg] = P.cell_start[b0];
-        seg_p[nseg] = acc;
-        acc += P.cell_start[b1] - seg_s[nseg];
-        ++nseg;
-      }
-    }
-  }
-  seg_p[nseg] = acc;
-  return nseg;
-}
-
-// Bead of staged position g.
-__device__ __forceinline__ int seg_bead(const int* seg_s, const int* seg_p, int nseg, int g) {
-  int q = 0;
-  while (q + 1 < nseg && seg_p[q + 1] <= g) ++q;
-  return seg_s[q] + (g - seg_p[q]);
 }
 
 __device__ __forceinline__ void list_counts(const DevPtrs& P, const CellCtx& q, const int* cnt, int nt) {
@@ -472,83 +398,6 @@ __device__ __forceinline__ void list_build_begin(const DevPtrs& P) {
     P.g->slack = 0.0;
     P.g->n_rebuilds++;
   }
-}
-
-// ---- FP64 form: each warp takes one bead of the cell at a time and tests
-// 32 staged candidates per round with the minimum image of the box.
-constexpr int kNbrThreads = 128;
-constexpr int kNbrChunkD = 768;  // 24 KB of staged double4
-
-__device__ __forceinline__ void nbr_cell_plain(const DevPtrs& P, int cur, int c) {
-  const int s0 = P.cell_start[c], e0 = P.cell_start[c + 1];
-  if (s0 >= e0) return;
-  const CellCtx q = cell_ctx(P, c, s0, e0);
-  const RepState& rs = P.rs[q.r];
-  copy_back<false, kNbrThreads>(P, cur, q, rs);
-  __shared__ int seg_s[18], seg_p[19];
-  __shared__ int nseg_sh;
-  __shared__ int cnt[kNbrMaxCell];
-  __shared__ int cidx[kNbrChunkD];
-  __shared__ double4 cposd[kNbrChunkD];
-  __syncthreads();  // the previous cell of this CTA is done with the shared arrays
-  const int nb = q.e - q.s;
-  if (nb > kNbrMaxCell) {
-    if (threadIdx.x == 0) atomicOr(&P.g->error, 2);
-    return;
-  }
-  if (threadIdx.x == 0) nseg_sh = stencil_segments(P, q, seg_s, seg_p);
-  for (int k = threadIdx.x; k < nb; k += kNbrThreads) cnt[k] = 0;
-  __syncthreads();
-  const int nseg = nseg_sh;
-  const int M = seg_p[nseg];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned int below = (1u << lane) - 1u;
-  const int kmax = P.kmax;
-  const double lc2 = P.tab->list_cut2;
-  for (int base = 0; base < M; base += kNbrChunkD) {
-    const int m = min(kNbrChunkD, M - base);
-    __syncthreads();
-    for (int k = threadIdx.x; k < m; k += kNbrThreads) {
-      const int j = seg_bead(seg_s, seg_p, nseg, base + k);
-      cidx[k] = j;
-      cposd[k] = P.dt4[j];
-    }
-    __syncthreads();
-    for (int b = warp; b < nb; b += kNbrThreads / 32) {
-      const int i = q.s + b;
-      int count = cnt[b];
-      int* out = P.nbr + (size_t)i * kmax;
-      const double4 di = P.dt4[i];
-      for (int k0 = 0; k0 < m; k0 += 32) {
-        const int k = k0 + lane;
-        bool hit = false;
-        if (k < m) {
-          const double4 dj = cposd[k];
-          double dx = di.x - dj.x, dy = di.y - dj.y, dz = di.z - dj.z;
-          dx -= rs.box[0] * rint(dx * (1.0 / 4294967296.0) * rs.frac_per_len[0]);
-          dy -= rs.box[1] * rint(dy * (1.0 / 4294967296.0) * rs.frac_per_len[1]);
-          dz -= rs.box[2] * rint(dz * (1.0 / 4294967296.0) * rs.frac_per_len[2]);
-          hit = (dx * dx + dy * dy + dz * dz < lc2) && (cidx[k] != i);
-        }
-        const unsigned int hits = __ballot_sync(0xffffffffu, hit);
-        if (hit) {
-          const int slot = count + __popc(hits & below);
-          if (slot < kmax) out[slot] = cidx[k];
-        }
-        count += __popc(hits);
-      }
-      if (lane == 0) cnt[b] = count;
-    }
-  }
-  __syncthreads();
-  list_counts(P, q, cnt, kNbrThreads);
-}
-
-__global__ void __launch_bounds__(kNbrThreads) k_nbr_cells_plain(DevPtrs P, int cur) {
-  pdl_wait();  // the reordered state
-  if (!P.g->rebuild) return;
-  list_build_begin(P);
-  for (int r = 0, c = list_cell(P, 0); c >= 0; c = list_cell(P, ++r)) nbr_cell_plain(P, cur, c);
 }
 
 // ---- Mixed form, octant-filtered.  Candidates are staged as FP32 offsets
@@ -705,7 +554,7 @@ __device__ __forceinline__ void nbr_cell_oct(const DevPtrs& P, int cur, int c) {
     if (threadIdx.x == 0) atomicOr(&P.g->error, 2);
     return;
   }
-  copy_back<true, kOctThreads>(P, cur, q, rs);
+  copy_back<true, kOctThreads>(P, cur, q);
   stencil_rows(P, q, seg_s, seg_len);
   for (int b = threadIdx.x; b < nb; b += kOctThreads) cnt[b] = 0;
   if (threadIdx.x == 0) stage[kOctChunk] = make_float4(1e30f, 1e30f, 1e30f, __int_as_float(-1));
@@ -836,13 +685,19 @@ __global__ void __launch_bounds__(kOctThreads) k_nbr_cells_oct(DevPtrs P, int cu
   for (int r = 0, c = list_cell(P, 0); c >= 0; c = list_cell(P, ++r)) nbr_cell_oct(P, cur, c);
 }
 
-// ---- Mixed form, flat stencil.  The CTA stages the stencil's beads as FP32
+// ---- Flat stencil.  The CTA stages the stencil's beads as FP32
 // offsets from the cell centre (exact 32-bit fractional differences, scaled
 // once), one x-row segment after another with no per-candidate search, and
 // each warp tests one bead of the cell against every staged candidate.  Few
 // barriers and 16 KB of shared memory per CTA: at the ~30 beads of an
 // occupied membrane cell this costs fewer instructions than filtering the
 // stencil per octant first.
+//
+// Both forms build their lists here.  The plain form's list is a filter only
+// (its pair passes test every entry's FP64 distance), so FP32 tests of the
+// fractional mirror serve it with a cut widened by the mirror's resolution and
+// the FP32 rounding of the offsets.  Testing in FP64 took 594 us per build of
+// an 18,003-bead vesicle, bound by the FP64 pipe.
 constexpr int kFlatChunk = 1024;  // staged candidates per pass (16 KB)
 
 // One bead (one warp) against mpad staged candidates (a multiple of 32):
@@ -912,7 +767,7 @@ __device__ __forceinline__ void flat_scan2(const float4* stage, int mpad, float 
   }
 }
 
-template <int NT>
+template <bool MIXED, int NT>
 __device__ __forceinline__ void nbr_cell_flat(const DevPtrs& P, int cur, int c) {
   const int s0 = P.cell_start[c], e0 = P.cell_start[c + 1];
   if (s0 >= e0) return;
@@ -930,7 +785,7 @@ __device__ __forceinline__ void nbr_cell_flat(const DevPtrs& P, int cur, int c) 
   const unsigned int crx = cell_centre_frac(q.cx, q.n0), cry = cell_centre_frac(q.cy, q.n1),
                      crz = cell_centre_frac(q.cz, q.n2);
   __syncthreads();  // the previous cell of this CTA is done with the shared arrays
-  copy_back<true, NT>(P, cur, q, rs);
+  copy_back<MIXED, NT>(P, cur, q);
   if (threadIdx.x < 32) stencil_warp(P, q, seg_s, seg_p, seg_len);
   for (int b = threadIdx.x; b < nb; b += NT) cnt[b] = 0;
   __syncthreads();
@@ -939,7 +794,10 @@ __device__ __forceinline__ void nbr_cell_flat(const DevPtrs& P, int cur, int c) 
   const float sx = rs.len_per_frac[0], sy = rs.len_per_frac[1], sz = rs.len_per_frac[2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kmax = P.kmax;
-  const float lcut = P.tab->list_cut_f + 1e-4f;
+  float lcut = P.tab->list_cut_f + 1e-4f;
+  // plain form: + the mirror's truncation (one unit per axis and pair) and the
+  // offsets' rounding (under 1e-6 of the cell size, itself under 2 list_cut)
+  if constexpr (!MIXED) lcut += 4e-6f * P.tab->list_cut_f + 4.f * fmaxf(sx, fmaxf(sy, sz));
   const float lc2 = lcut * lcut;
   const bool thin = q.n0 < 3 || q.n1 < 3 || q.n2 < 3;
   const float bx = sx * 4294967296.0f, by = sy * 4294967296.0f, bz = sz * 4294967296.0f;
@@ -1013,12 +871,12 @@ __device__ __forceinline__ void nbr_cell_flat(const DevPtrs& P, int cur, int c) 
   list_counts(P, q, cnt, NT);
 }
 
-template <int NT>
+template <bool MIXED, int NT>
 __global__ void __launch_bounds__(NT, 768 / NT) k_nbr_cells_flat(DevPtrs P, int cur) {
   pdl_wait();  // the reordered state
   if (!P.g->rebuild) return;
   list_build_begin(P);
-  for (int r = 0, c = list_cell(P, 0); c >= 0; c = list_cell(P, ++r)) nbr_cell_flat<NT>(P, cur, c);
+  for (int r = 0, c = list_cell(P, 0); c >= 0; c = list_cell(P, ++r)) nbr_cell_flat<MIXED, NT>(P, cur, c);
 }
 
 // ------------------------------------------------------------ the step
@@ -1882,6 +1740,101 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
   }
 }
 
+// Plain-form pair sums of the warp's 32 / G beads (bead i on lanes sub = 0 ..
+// G-1; inactive groups take part with an empty list).  The FP64 pipe bounds
+// this pass, and about half of a list's entries lie beyond rc.  The lanes
+// therefore first test kPairQueue entries in FP32 on the fractional mirror,
+// with a cut widened by the mirror's resolution and the FP32 rounding, and
+// queue what passes in shared memory; the FP64 distance, its exact test
+// against rc and the pair term then run on full groups of queued entries.
+// Every entry in FP64 took 78 FP64 instructions each and 362 us for an
+// 18,003-bead vesicle; with the list build in FP32 too, a loop step of it went
+// from 709 to 150 us.
+constexpr int kPairQueue = 128;
+template <int FL, int G>
+__device__ __forceinline__ void pair_sum_d(const DevPtrs& P, int cur, int i, int sub, bool active, const RepState& rs,
+                                           const double* sF, const double* sU, int nT, int* queue, double& fx,
+                                           double& fy, double& fz, double& ep, double& dU) {
+  const Tables& T = *P.tab;
+  const int lane = threadIdx.x & 31;
+  const unsigned int below = (1u << lane) - 1u;
+  const unsigned int mine = ((1u << G) - 1u) << (lane & ~(G - 1));
+  const int nn = active ? P.nnbr[i] : 0;
+  const int* nb = P.nbr + (size_t)i * P.kmax;
+  double4 me = make_double4(0.0, 0.0, 0.0, 0.0);
+  uint4 mu = make_uint4(0u, 0u, 0u, 0u);
+  if (active) {
+    me = P.d4[cur][i];
+    mu = P.m4[cur][i];
+  }
+  const int ti = __double_as_longlong(me.w) & 0xff;
+  const double* rowF = sF + 6 * ti * nT;
+  const double* rowU = sU + 6 * ti * nT;
+  const double rc2 = T.rc2;
+  const float s0 = rs.len_per_frac[0], s1 = rs.len_per_frac[1], s2 = rs.len_per_frac[2];
+  const float cut = T.rcf * (1.f + 4e-6f) + 4.f * fmaxf(s0, fmaxf(s1, s2));
+  const float cut2 = cut * cut;
+  const int h0 = __double2hiint(0.5 * rs.box[0]), h1 = __double2hiint(0.5 * rs.box[1]),
+            h2 = __double2hiint(0.5 * rs.box[2]);
+  float sq0 = 0.f, sq1 = 0.f, sq2 = 0.f;
+  if constexpr ((FL & F_DU) != 0) {
+    sq0 = rs.sq_f[0];
+    sq1 = rs.sq_f[1];
+    sq2 = rs.sq_f[2];
+  }
+  const int longest = __reduce_max_sync(0xffffffffu, nn);
+  for (int base = 0; base < longest; base += kPairQueue) {
+    const int end = min(kPairQueue, longest - base);
+    int queued = 0;
+#pragma unroll 4
+    for (int k0 = 0; k0 < end; k0 += G) {
+      const int k = base + k0 + sub;
+      bool near = false;
+      int j = 0;
+      if (k < nn) {
+        j = __ldg(nb + k);
+        const uint4 o = P.m4[cur][j];
+        const float dx = frac_delta(mu.x, o.x, s0), dy = frac_delta(mu.y, o.y, s1), dz = frac_delta(mu.z, o.z, s2);
+        const float r2 = dx * dx + dy * dy + dz * dz;
+        near = r2 < cut2;
+        if constexpr ((FL & F_DU) != 0) near = near || r2 + (sq0 * dx * dx + sq1 * dy * dy + sq2 * dz * dz) < cut2;
+      }
+      const unsigned int hits = __ballot_sync(0xffffffffu, near) & mine;
+      if (near) queue[queued + __popc(hits & below)] = j;
+      queued += __popc(hits);
+    }
+    __syncwarp();
+    for (int k = sub; k < queued; k += G) {
+      const int j = queue[k];
+      const double4 o = P.d4[cur][j];
+      const double dx = image64(me.x, o.x, rs.box[0], h0), dy = image64(me.y, o.y, rs.box[1], h1),
+                   dz = image64(me.z, o.z, rs.box[2], h2);
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      const int tj = __double_as_longlong(o.w) & 0xff;
+      double rinv;
+      if (r2 < rc2) {
+        if constexpr ((FL & F_ENERGY) == 0) {
+          const double mag = pair_mag64(rowF + 6 * tj, r2);
+          fx += dx * mag;
+          fy += dy * mag;
+          fz += dz * mag;
+        } else {
+          ep += 0.5 * pair_pot<double>(rowU + 6 * tj, root64(r2, rinv));
+        }
+      }
+      if constexpr ((FL & F_DU) != 0) {
+        const double nx = dx * rs.scale[0], ny = dy * rs.scale[1], nz = dz * rs.scale[2];
+        const double rn2 = nx * nx + ny * ny + nz * nz;
+        const double u0 = r2 < rc2 ? pair_pot<double>(rowU + 6 * tj, root64(r2, rinv)) : 0.0;
+        const double u1 = (rn2 < rc2 && (r2 < rc2 || ref_cells_adjacent(P, rs, i, j)))
+                              ? pair_pot<double>(rowU + 6 * tj, root64(rn2, rinv)) : 0.0;
+        dU += 0.5 * (u0 - u1);
+      }
+    }
+    __syncwarp();
+  }
+}
+
 template <bool MIXED, int FL, int G>
 __global__ void __launch_bounds__(kBlock) k_force(DevPtrs P, int cur) {
   pdl_trigger();
@@ -1907,57 +1860,16 @@ __global__ void __launch_bounds__(kBlock) k_force(DevPtrs P, int cur) {
   double dU = 0.0, ep = 0.0;
   long long qx = 0, qy = 0, qz = 0, dq = 0;
   double fx = 0, fy = 0, fz = 0;
-  if (active) {
-    const RepState& rs = P.rs[r];
-    const int nn = P.nnbr[i];
-    const int* nb = P.nbr + (size_t)i * P.kmax;
-    if constexpr (MIXED) {
+  const RepState& rs = P.rs[r];
+  if constexpr (MIXED) {
+    if (active) {
       float eacc = 0.f;
       pair_sum_q<FL, G>(P, cur, i, sub, rs, sF, sU, nT, qx, qy, qz, dq, eacc);
       ep = 0.5 * (double)eacc;
-    } else {
-      const double4 me = P.d4[cur][i];
-      const int ti = __double_as_longlong(me.w) & 0xff;
-      const double* rowF = sF + 6 * ti * nT;
-      const double* rowU = sU + 6 * ti * nT;
-      const double rc2 = T.rc2;
-      const double box[3] = {rs.box[0], rs.box[1], rs.box[2]};
-      for (int k = sub; k < nn; k += G) {
-        const int j = __ldg(nb + k);
-        const double4 o = P.d4[cur][j];
-        // minimum image applied to the neighbour first, as CellOpt shifts the
-        // neighbour cell's positions (cellOpt.h:810-840)
-        double ox = o.x, oy = o.y, oz = o.z;
-        if (me.x - ox > box[0] / 2.0) ox += box[0];
-        if (me.x - ox < -box[0] / 2.0) ox -= box[0];
-        if (me.y - oy > box[1] / 2.0) oy += box[1];
-        if (me.y - oy < -box[1] / 2.0) oy -= box[1];
-        if (me.z - oz > box[2] / 2.0) oz += box[2];
-        if (me.z - oz < -box[2] / 2.0) oz -= box[2];
-        const double dx = me.x - ox, dy = me.y - oy, dz = me.z - oz;
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        const int tj = __double_as_longlong(o.w) & 0xff;
-        if (r2 < rc2) {
-          const double rr = sqrt(r2);
-          if constexpr ((FL & F_ENERGY) == 0) {
-            const double mag = pair_mag<double>(rowF + 6 * tj, rr);
-            fx += dx * mag;
-            fy += dy * mag;
-            fz += dz * mag;
-          } else {
-            ep += 0.5 * pair_pot<double>(rowU + 6 * tj, rr);
-          }
-        }
-        if constexpr ((FL & F_DU) != 0) {
-          const double nx = dx * rs.scale[0], ny = dy * rs.scale[1], nz = dz * rs.scale[2];
-          const double rn2 = nx * nx + ny * ny + nz * nz;
-          const double u0 = r2 < rc2 ? pair_pot<double>(rowU + 6 * tj, sqrt(r2)) : 0.0;
-          const double u1 = (rn2 < rc2 && (r2 < rc2 || ref_cells_adjacent(P, rs, i, j)))
-                                ? pair_pot<double>(rowU + 6 * tj, sqrt(rn2)) : 0.0;
-          dU += 0.5 * (u0 - u1);
-        }
-      }
     }
+  } else {
+    __shared__ int queue[kBlock / G][kPairQueue];
+    pair_sum_d<FL, G>(P, cur, i, sub, active, rs, sF, sU, nT, queue[threadIdx.x / G], fx, fy, fz, ep, dU);
   }
   // group reduction (integer sums are exact in any order)
 #pragma unroll
@@ -2230,13 +2142,8 @@ __device__ __forceinline__ void integ_bead(const DevPtrs& P, int cur, int i, int
         const unsigned int fx = to_frac(x[0], rs.frac_per_len[0]), fy = to_frac(x[1], rs.frac_per_len[1]),
                            fz = to_frac(x[2], rs.frac_per_len[2]);
         vmax = displacement(P.ref[i], fx, fy, fz, rs);
-        if constexpr (MIXED) {
-          const uint4 me = P.m4[cur][i];
-          P.m4[cur ^ 1][i] = make_uint4(fx, fy, fz, me.w);
-        } else {
-          const double4 me = P.d4[cur][i];
-          P.d4[cur ^ 1][i] = make_double4(x[0], x[1], x[2], me.w);
-        }
+        P.m4[cur ^ 1][i] = make_uint4(fx, fy, fz, P.m4[cur][i].w);
+        if constexpr (!MIXED) P.d4[cur ^ 1][i] = make_double4(x[0], x[1], x[2], P.d4[cur][i].w);
       }
     }
   }
@@ -2401,13 +2308,8 @@ __global__ void __launch_bounds__(kBeadBlock) k_finish(DevPtrs P, int cur, int m
     const unsigned int fx = to_frac(x[0], rs.frac_per_len[0]), fy = to_frac(x[1], rs.frac_per_len[1]),
                        fz = to_frac(x[2], rs.frac_per_len[2]);
     vmax = displacement(P.ref[i], fx, fy, fz, rs);
-    if constexpr (MIXED) {
-      const uint4 me = P.m4[cur][i];
-      P.m4[cur ^ 1][i] = make_uint4(fx, fy, fz, me.w);
-    } else {
-      const double4 me = P.d4[cur][i];
-      P.d4[cur ^ 1][i] = make_double4(x[0], x[1], x[2], me.w);
-    }
+    P.m4[cur ^ 1][i] = make_uint4(fx, fy, fz, P.m4[cur][i].w);
+    if constexpr (!MIXED) P.d4[cur ^ 1][i] = make_double4(x[0], x[1], x[2], P.d4[cur][i].w);
   }
   vmax = warp_max(vmax);
   __shared__ float smax[kBeadBlock / 32];
@@ -2552,8 +2454,8 @@ __global__ void __launch_bounds__(kMaxSpheres) k_sphere(DevPtrs P, int cur, Step
         const unsigned int fx = to_frac(x[0], rs.frac_per_len[0]), fy = to_frac(x[1], rs.frac_per_len[1]),
                            fz = to_frac(x[2], rs.frac_per_len[2]);
         vmax = displacement(P.ref[j], fx, fy, fz, rs);
-        if constexpr (MIXED) P.m4[cur ^ 1][j] = make_uint4(fx, fy, fz, pos_s[s].w);
-        else P.d4[cur ^ 1][j] = make_double4(x[0], x[1], x[2], pos_s[s].w);
+        P.m4[cur ^ 1][j] = make_uint4(fx, fy, fz, P.m4[cur][j].w);
+        if constexpr (!MIXED) P.d4[cur ^ 1][j] = make_double4(x[0], x[1], x[2], pos_s[s].w);
       }
     }
   }
@@ -2620,11 +2522,9 @@ __global__ void __launch_bounds__(kBlock) k_mirror(DevPtrs P, int cur) {
   if (i >= P.n) return;
   const int r = rep_of(P, i);
   const RepState& rs = P.rs[r];
-  if constexpr (MIXED) {
-    const uint4 me = P.m4[cur][i];
-    P.m4[cur][i] = make_uint4(to_frac(P.x[i], rs.frac_per_len[0]), to_frac(P.y[i], rs.frac_per_len[1]),
-                              to_frac(P.z[i], rs.frac_per_len[2]), me.w);
-  } else {
+  P.m4[cur][i] = make_uint4(to_frac(P.x[i], rs.frac_per_len[0]), to_frac(P.y[i], rs.frac_per_len[1]),
+                            to_frac(P.z[i], rs.frac_per_len[2]), P.m4[cur][i].w);
+  if constexpr (!MIXED) {
     const double4 me = P.d4[cur][i];
     P.d4[cur][i] = make_double4(P.x[i], P.y[i], P.z[i], me.w);
   }
