@@ -1,12 +1,15 @@
-"""The FP64 pair passes (plain form and smd_pair_forces_static) against a
-direct FP64 sum over all pairs.
+"""The list build and the pair passes (both forms, and smd_pair_forces_static)
+against a direct FP64 sum over all pairs.
 
-Both passes queue the entries that an FP32 test keeps and evaluate those in
-FP64, so the sizes are the ones where that can go wrong: a single bead, group
+The FP64 passes queue the entries that an FP32 test keeps and evaluate those in
+FP64, and the list comes from matrix tiles of 16 beads by 8 candidates, so the
+sizes are the ones where that can go wrong: a single bead, group and tile
 remainders, boxes of exactly three cutoffs, thin list grids (minimum image per
-candidate), more neighbours than a queue holds, and beads on the faces 0 and L.
-A bead's force sums at most a few hundred terms of a few roundings each, so
-1e-12 of max |F| (the suite's plain-form tolerance) leaves a decade.
+candidate), cells of more than 32 beads, stencils of more than one chunk of
+1,024, more neighbours than a queue or a list buffer holds, cells wider than
+twice the list cut, and beads on the faces 0 and L.  A bead's force sums at most
+a few hundred terms of a few roundings each, so 1e-12 of max |F| (the suite's
+plain-form tolerance) leaves a decade; 1e-5 is the suite's for the mixed form.
 """
 import ctypes
 
@@ -20,7 +23,7 @@ pytestmark = pytest.mark.gpu
 RC = 2.0
 # beads, box
 CASES = [(1, (6.5, 6.5, 6.5)), (37, (6.0, 6.0, 6.0)), (613, (6.0, 17.3, 9.9)), (1500, (6.5, 6.5, 6.5)),
-         (2501, (31.0, 14.2, 9.1))]
+         (2501, (31.0, 14.2, 9.1)), (3000, (7.6, 7.7, 7.8)), (1901, (7.6, 7.6, 23.0))]
 
 
 def _system(n, box):
@@ -75,6 +78,12 @@ def test_fp64_pair_passes_against_all_pairs(built, n, box):
     assert np.abs(s.forces() - want).max() <= 1e-12 * scale
     assert abs(s.energy()[0]["pair"] - energy) <= 1e-12 * max(abs(energy), 1.0)
     s.close()
+    s = smd.System(m, precision=smd.MIXED)
+    for kern in range(3):
+        s.set_tuning(8, kern)
+        s.set_state(m.pos)  # builds the list with this kernel
+        assert np.abs(s.forces() - want).max() <= 1e-5 * scale
+    s.close()
     pos = torch.from_numpy(m.pos).cuda()
     typ = torch.from_numpy(m.type).cuda()
     fc = torch.from_numpy(m.fconst).cuda()
@@ -85,3 +94,15 @@ def test_fp64_pair_passes_against_all_pairs(built, n, box):
     assert rc == 0, smd.last_error()
     torch.cuda.synchronize()
     assert np.abs(out.cpu().numpy() - want).max() <= 1e-12 * scale
+
+
+@pytest.mark.parametrize("prec,tol", [(smd.PLAIN_FP64, 1e-12), (smd.MIXED, 1e-5)])
+def test_list_of_cells_wider_than_twice_the_cut(built, prec, tol):
+    """A box set far larger than the handle's cell grid was sized for."""
+    m = _system(700, (7.6, 7.6, 7.6))
+    s = smd.System(m, precision=prec)
+    m.box = np.array([30.0, 30.0, 30.0])
+    s.set_box(m.box)
+    want, _ = _direct(m)
+    assert np.abs(s.forces() - want).max() <= tol * np.abs(want).max()
+    s.close()
