@@ -195,11 +195,12 @@ int smd_autotune(smd_system* h, int force, int* lanes, int* list_kernel, float* 
  * 16; list_kernel 0, 1 or 2) and marks the handle tuned. */
 int smd_set_tuning(smd_system* h, int lanes, int list_kernel);
 
-/* Launch mode of smd_advance: on = 1 (default) runs each barostat period as
- * one CUDA graph whose list builds are conditional nodes; on = 0 launches the
- * same kernels one by one (profilers that cannot see kernel nodes inside
- * graphs with conditional nodes still see each kernel).  No reference
- * counterpart: the reference launches nothing. */
+/* Launch mode of smd_advance: on = 1 (default) runs a stretch of steps of a
+ * small or mid-size system as one persistent cooperative kernel, and each
+ * barostat period of any other as one CUDA graph whose list builds are
+ * conditional nodes; on = 0 launches the same work kernel by kernel (profilers
+ * that cannot see kernel nodes inside graphs with conditional nodes still see
+ * each kernel).  No reference counterpart: the reference launches nothing. */
 int smd_use_graphs(smd_system* h, int on);
 
 /* Waits for the handle's stream and reports any device-side error. */

@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_chain(DevPtrs P, int cur, const 
       const int p = ci & 0xfff, len = (ci >> 12) & 0xfff, set = (ci >> 24) & 0x1f;
       Vec3<double> e[4];
       bool valid[4];
-      chain_vectors<MIXED, double>(P, cur, i, p, len, box, e, valid);
+      chain_vectors<MIXED, double>(P, cur, i, p, len, box, rs, e, valid);
       // tangents: differences of w along the chain (file order is chain order)
       Vec3<Dd> ed[4];
       for (int k = 0; k < 4; ++k) {
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_hvp_out(DevPtrs P, int cur, cons
     const int p = ci & 0xfff, len = (ci >> 12) & 0xfff, set = (ci >> 24) & 0x1f;
     Vec3<double> e[4];
     bool valid[4];
-    chain_vectors<MIXED, double>(P, cur, i, p, len, box, e, valid);
+    chain_vectors<MIXED, double>(P, cur, i, p, len, box, rs, e, valid);
     Vec3<Dd> ed[4];
     for (int k = 0; k < 4; ++k) {
       const int a = o - 2 + k, b = o - 1 + k;

@@ -18,6 +18,7 @@
 #include "../../include/softmold_gb300.h"
 #include "mt19937.h"
 #include "smd_adjoint.cuh"
+#include "smd_run.cuh"
 
 namespace {
 
@@ -114,6 +115,15 @@ struct smd_system {
     int kernels = 0;  // kernel nodes outside the conditional bodies
   } graph[2];
   bool use_graphs = true;
+  // the persistent loop kernel (single systems without spheres or field terms,
+  // up to kRunMaxBeads): CTAs, beads and threads per CTA, lanes per bead
+  struct RunLoop {
+    int grid = 0;  // 0: not used
+    int beads = 0, threads = 0, lanes = 8;
+    size_t smem = 0;
+    int* cnt = nullptr;
+    RunSync* sync = nullptr;
+  } run;
   // launch configuration chosen by the autotuner (mixed form): lanes per bead
   // of the pair pass and the list-build kernel (0 flat/128, 1 flat/256,
   // 2 octant/256); every choice gives bitwise the same trajectory
@@ -416,6 +426,74 @@ bool is_trial_step(const smd_system* h, long long it) {
   return h->barostat && (it % h->resize_rate) == 0 && it != 0;
 }
 
+template <bool MIXED, int G>
+int launch_run(smd_system* h, RunArgs a) {
+  void* args[] = {&h->P, &a};
+  const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(&k_run<MIXED, G>), dim3(h->run.grid),
+                                                    dim3(h->run.threads), args, h->run.smem, h->stream);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    return fail(200 + (int)e, std::string("kernel launch: ") + cudaGetErrorString(e));
+  }
+  return check_launch(h);
+}
+
+// `steps` loop iterations (barostat trials included) in one persistent kernel.
+int advance_run(smd_system* h, int steps) {
+  const auto& r = h->run;
+  const RunArgs a{h->it, h->cur, steps, h->resize_rate, h->barostat ? 1 : 0, r.beads, r.cnt, r.sync};
+  int rc;
+  if (h->mixed) rc = r.lanes == 32 ? launch_run<true, 32>(h, a) : (r.lanes == 16 ? launch_run<true, 16>(h, a) : launch_run<true, 8>(h, a));
+  else rc = r.lanes == 32 ? launch_run<false, 32>(h, a) : (r.lanes == 16 ? launch_run<false, 16>(h, a) : launch_run<false, 8>(h, a));
+  if (rc) return rc;
+  for (int k = 0; k < steps; ++k)
+    if (is_trial_step(h, h->it + k)) h->trials_used++;
+  h->it += steps;
+  h->cur ^= steps & 1;
+  return 0;
+}
+
+// Sets up the persistent loop where the system fits it.
+template <bool MIXED, int G>
+int run_fits_device(smd_system* h, bool* fits) {
+  const void* f = reinterpret_cast<const void*>(&k_run<MIXED, G>);
+  int dev = 0, limit = 0, coop = 0, per_sm = 0;
+  SMD_CUDA(cudaGetDevice(&dev));
+  SMD_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  SMD_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+  cudaFuncAttributes at{};
+  SMD_CUDA(cudaFuncGetAttributes(&at, f));
+  *fits = false;
+  if (!coop || h->run.smem + at.sharedSizeBytes > (size_t)limit) return 0;
+  // the largest any handle may ask for, so that handles do not undo each other's setting
+  SMD_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, limit - (int)at.sharedSizeBytes));
+  SMD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, h->run.threads, h->run.smem));
+  *fits = (long long)per_sm * h->sms >= h->run.grid;
+  return 0;
+}
+int run_setup(smd_system* h) {
+  auto& r = h->run;
+  r.grid = 0;
+  if (h->n_rep != 1 || h->n_sph > 0 || h->has_fields || h->n > kRunMaxBeads || h->n_cells > kRunCells) return 0;
+  const int ctas = std::min(h->sms, 255);
+  r.beads = std::max(8, (h->n + ctas - 1) / ctas);
+  r.lanes = r.beads <= 24 ? 32 : (r.beads <= 48 ? 16 : 8);
+  r.threads = std::min(run_threads(r.lanes), std::max(256, (r.beads * r.lanes + r.beads + 63) / 32 * 32));
+  if (r.beads > r.threads) return 0;
+  r.smem = run_smem(r.beads, h->n_cells, h->mixed, r.threads, r.lanes);
+  const int grid = (h->n + r.beads - 1) / r.beads;
+  r.grid = grid;
+  bool fits = false;
+  int rc;
+  if (h->mixed) rc = r.lanes == 32 ? run_fits_device<true, 32>(h, &fits) : (r.lanes == 16 ? run_fits_device<true, 16>(h, &fits) : run_fits_device<true, 8>(h, &fits));
+  else rc = r.lanes == 32 ? run_fits_device<false, 32>(h, &fits) : (r.lanes == 16 ? run_fits_device<false, 16>(h, &fits) : run_fits_device<false, 8>(h, &fits));
+  r.grid = 0;
+  if (rc || !fits) return rc;
+  if ((rc = h->alloc(&r.cnt, 2 * (size_t)h->n_cells)) || (rc = h->alloc(&r.sync, 1))) return rc;
+  r.grid = grid;
+  return 0;
+}
+
 // Counts the barostat trials among the next `steps` iterations, draws their
 // two uniforms per replica from the MT19937 streams, and stages them.
 // Appends the decisions of the trials run from the staged buffer to the host
@@ -514,6 +592,7 @@ int read_error(smd_system* h) {
   SMD_CUDA(cudaStreamSynchronize(h->stream));
   h->graph_builds = g.graph_builds;
   if (g.n_occ > 0) h->occ_est = g.n_occ;
+  if (g.error & 8) return fail(11, "the persistent loop kernel gave up waiting for its CTAs (the handle's state is lost)");
   if (g.error & 2) return fail(8, "a Verlet-list cell holds more than 1024 beads (collapsed system)");
   if (g.error & 1) {
     char buf[256];
@@ -1029,6 +1108,7 @@ int smd_create_batch(const smd_system_desc* descs, int n_rep, int precision, smd
     SMD_CUDA(cudaMemcpy(P.rs, rs.data(), n_rep * sizeof(RepState), cudaMemcpyHostToDevice));
     SMD_CUDA(cudaMemcpy(tdev, &T, sizeof(Tables), cudaMemcpyHostToDevice));
   }
+  if ((rc = run_setup(h.get()))) return rc;
   // ---- size the Verlet list: count pass with zero capacity, then the build
   P.kmax = 0;
   if ((rc = force_rebuild(h.get()))) return rc;
@@ -1486,6 +1566,11 @@ int smd_advance(smd_system* h, int steps, int flags) {
     for (int s = 0; s < chunk; ++s) {
       // the last step of a stopping call runs alone (it stops after its second half-kick)
       const int left = chunk - s - ((stop_at_measure && done + chunk == steps) ? 1 : 0);
+      if (h->run.grid && left > 0 && h->use_graphs && !h->profile && !h->ext_noise_pending && !h->meas.tracking) {
+        if ((rc = advance_run(h, left))) return rc;
+        s += left - 1;
+        continue;
+      }
       if (graph_fits(h, h->it, left)) {
         auto& g = h->graph[h->cur];
         if (!g.exec && (rc = capture_period(h, h->cur))) return rc;

@@ -21,9 +21,16 @@ enum StepFlags {
   F_FORCES = 16,    // conservative forces only, written to P.force_out (file order)
   F_PAIRONLY = 32,  // with F_FORCES: non-bonded part only
   F_ENERGY = 64,    // energies only (pair, bonded, kinetic) into RepState
-  F_FIELDS = 128    // the system has external-field terms (their out-of-line
+  F_FIELDS = 128,   // the system has external-field terms (their out-of-line
                     // evaluation is compiled in only with this flag)
+  F_RUN = 256       // inside the persistent loop kernel, which writes the lists
+                    // it reads: no read-only loads of them
 };
+
+template <int FL>
+__device__ __forceinline__ int list_entry(const int* p) {
+  if constexpr ((FL & F_RUN) != 0) return *p; else return __ldg(p);
+}
 
 // ------------------------------------------------------------ last block
 // Runs once per launch after every block has passed its atomics.  The list
@@ -994,7 +1001,7 @@ __device__ __forceinline__ long long f2ll_rn(float y) {
 // fractional mirror (in FP64); PLAIN: FP64 with the bonded minimum image.
 template <bool MIXED, typename RT>
 __device__ __forceinline__ void chain_vectors(const DevPtrs& P, int cur, int i, int p, int len, const double box[3],
-                                              Vec3<RT> e[4], bool valid[4]) {
+                                              const RepState& rs, Vec3<RT> e[4], bool valid[4]) {
   const int o = P.orig[i];
   int idx[5];
   bool have[5];
@@ -1010,7 +1017,6 @@ __device__ __forceinline__ void chain_vectors(const DevPtrs& P, int cur, int i, 
     for (int k = 0; k < 5; ++k) m[k] = P.m4[cur][idx[k]];
     RT s0, s1, s2;
     if constexpr (std::is_same<RT, float>::value) {
-      const RepState& rs = P.rs[rep_of(P, i)];
       s0 = rs.len_per_frac[0];
       s1 = rs.len_per_frac[1];
       s2 = rs.len_per_frac[2];
@@ -1470,7 +1476,7 @@ __device__ __forceinline__ Vec3<typename std::conditional<MIXED, float, double>:
     const int p = ci & 0xfff, len = (ci >> 12) & 0xfff, set = (ci >> 24) & 0x1f;
     Vec3<R> er[4];
     bool valid[4];
-    chain_vectors<MIXED, R>(P, cur, i, p, len, box, er, valid);
+    chain_vectors<MIXED, R>(P, cur, i, p, len, box, rs, er, valid);
     const R* cf;
     if constexpr (MIXED) cf = T.chainF[set]; else cf = T.chainD[set];
     if (valid[1]) bond_term<R>(er[1], cf, (R)-1, fb);  // bond (p-1,p): second
@@ -1505,6 +1511,109 @@ __device__ __forceinline__ Vec3<typename std::conditional<MIXED, float, double>:
     }
   }
   return fb;
+}
+
+// Bonded energies (F_ENERGY) and size-change differences (F_DU) owned by bead
+// i: its CHAIN bond and bend as their first bead, then its BOND / BEND residue
+// and external-field terms.
+template <bool MIXED, int FL>
+__device__ __forceinline__ void bonded_sums(const DevPtrs& P, int cur, int i, int ci, const double box[3],
+                                            const RepState& rs, double& dU_bond, double& e_bond) {
+  const Tables& T = *P.tab;
+  using R = typename std::conditional<MIXED, float, double>::type;
+  if (ci < 0 && !(ci & 0x40000000)) {
+    const int p = ci & 0xfff, len = (ci >> 12) & 0xfff, set = (ci >> 24) & 0x1f;
+    // the chain's difference vectors in R (exact from the fractional
+    // mirror in the mixed form)
+    Vec3<R> er[4];
+    bool valid[4];
+    chain_vectors<MIXED, R>(P, cur, i, p, len, box, rs, er, valid);
+    // terms owned by the first bead of each bond / bend: energies in FP64;
+    // size-change differences in FP64 (plain) or factored FP32 (mixed)
+    if constexpr (MIXED && (FL & F_DU) != 0) {
+      const float* cf = T.chainF[set];
+      const float sq[3] = {rs.sq_f[0], rs.sq_f[1], rs.sq_f[2]};
+      float du = 0.f;
+      if (valid[2]) du += bond_dpot_f(er[2], sq, cf);
+      if (valid[2] && valid[3]) du += bend_dpot_f(er[2], er[3], sq, cf + 2);
+      dU_bond += (double)du;
+    }
+    if constexpr ((FL & F_ENERGY) != 0 || (!MIXED && (FL & F_DU) != 0)) {
+      Vec3<double> e[4];
+      if constexpr (MIXED) {
+        chain_vectors<MIXED, double>(P, cur, i, p, len, box, rs, e, valid);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) e[k] = Vec3<double>{er[k].x, er[k].y, er[k].z};
+      }
+      const double* cd = T.chainD[set];
+      if constexpr ((FL & F_ENERGY) != 0) {
+        if (valid[2]) e_bond += bond_pot(e[2], cd);
+        if (valid[2] && valid[3]) e_bond += bend_pot(e[2], e[3], cd + 2);
+      }
+      if constexpr (!MIXED && (FL & F_DU) != 0) {
+        const Vec3<double> s2{e[2].x * rs.scale[0], e[2].y * rs.scale[1], e[2].z * rs.scale[2]};
+        const Vec3<double> s3{e[3].x * rs.scale[0], e[3].y * rs.scale[1], e[3].z * rs.scale[2]};
+        if (valid[2]) dU_bond += bond_pot(e[2], cd) - bond_pot(s2, cd);
+        if (valid[2] && valid[3]) dU_bond += bend_pot(e[2], e[3], cd + 2) - bend_pot(s2, s3, cd + 2);
+      }
+    }
+  }
+  // ---- BOND / BEND residue terms of this bead: energies and differences
+  // (their forces are in bonded_force)
+  {
+    if (P.n_terms > 0) {
+      const int o = P.orig[i];
+      const int e1 = P.term_off[o + 1];
+      const float sq_f[3] = {rs.sq_f[0], rs.sq_f[1], rs.sq_f[2]};
+      for (int e = P.term_off[o]; e < e1; ++e) {
+        const int4 t = P.terms[e];
+        const int kind = term_kind(t.x), role = term_role(t.x), set = term_set(t.x);
+        if (kind > kTermBend) {  // external fields: energy only (no size-change term in the reference)
+          if constexpr ((FL & F_ENERGY) != 0 && (FL & F_FIELDS) != 0)
+            if (role == 0) e_bond += field_potential<MIXED>(P, cur, i, t, box);
+          continue;
+        }
+        const double* cd = T.termD[set];
+        if (kind == kTermBond) {  // bond (first, second): the bead's force is mag (x_self - x_other)
+          if constexpr ((FL & (F_DU | F_ENERGY)) != 0) {
+            if (role == 0) {  // energy terms owned by the first bead
+              if constexpr (MIXED && (FL & F_DU) != 0)
+                dU_bond += (double)bond_dpot_f(term_vec<MIXED, float>(P, cur, t.y, t.z, box, rs), sq_f,
+                                               T.termF[set]);
+              if constexpr ((FL & F_ENERGY) != 0 || (!MIXED && (FL & F_DU) != 0)) {
+                const Vec3<double> d = term_vec<MIXED, double>(P, cur, t.y, t.z, box, rs);
+                if constexpr ((FL & F_ENERGY) != 0) e_bond += bond_pot(d, cd);
+                if constexpr (!MIXED && (FL & F_DU) != 0) {
+                  const Vec3<double> sd{d.x * rs.scale[0], d.y * rs.scale[1], d.z * rs.scale[2]};
+                  dU_bond += bond_pot(d, cd) - bond_pot(sd, cd);
+                }
+              }
+            }
+          }
+        } else {  // bend (first, second, third): da = x1 - x2, db = x2 - x3
+          if constexpr ((FL & (F_DU | F_ENERGY)) != 0) {
+            if (role == 0) {
+              if constexpr (MIXED && (FL & F_DU) != 0)
+                dU_bond += (double)bend_dpot_f(term_vec<MIXED, float>(P, cur, t.y, t.z, box, rs),
+                                               term_vec<MIXED, float>(P, cur, t.z, t.w, box, rs), sq_f,
+                                               T.termF[set]);
+              if constexpr ((FL & F_ENERGY) != 0 || (!MIXED && (FL & F_DU) != 0)) {
+                const Vec3<double> da = term_vec<MIXED, double>(P, cur, t.y, t.z, box, rs);
+                const Vec3<double> db = term_vec<MIXED, double>(P, cur, t.z, t.w, box, rs);
+                if constexpr ((FL & F_ENERGY) != 0) e_bond += bend_pot(da, db, cd);
+                if constexpr (!MIXED && (FL & F_DU) != 0) {
+                  const Vec3<double> sa{da.x * rs.scale[0], da.y * rs.scale[1], da.z * rs.scale[2]};
+                  const Vec3<double> sb{db.x * rs.scale[0], db.y * rs.scale[1], db.z * rs.scale[2]};
+                  dU_bond += bend_pot(da, db, cd) - bend_pot(sa, sb, cd);
+                }
+              }
+            }
+          }
+        }
+      }
+    }
+  }
 }
 
 // Non-bonded pass: G lanes per bead walk the bead's Verlet-list entries
@@ -1661,7 +1770,7 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
     bool more = k + (kGather - 1) * G < nn;
     if (more) {
 #pragma unroll
-      for (int u = 0; u < kGather; ++u) jn[u] = __ldg(nb + k + u * G);
+      for (int u = 0; u < kGather; ++u) jn[u] = list_entry<FL>(nb + k + u * G);
     }
     for (; more; k += kGather * G) {
       uint4 og[kGather];
@@ -1674,7 +1783,7 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
       more = k + (2 * kGather - 1) * G < nn;
       if (more) {
 #pragma unroll
-        for (int u = 0; u < kGather; ++u) jn[u] = __ldg(nb + k + (kGather + u) * G);
+        for (int u = 0; u < kGather; ++u) jn[u] = list_entry<FL>(nb + k + (kGather + u) * G);
       }
       batch(og, jg);
     }
@@ -1684,7 +1793,7 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
       int jg[kGather];
 #pragma unroll
       for (int u = 0; u < kGather; ++u) {
-        jg[u] = __ldg(nb + k + u * G);
+        jg[u] = list_entry<FL>(nb + k + u * G);
         og[u] = P.m4[cur][jg[u]];
       }
       batch(og, jg);
@@ -1698,7 +1807,7 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
 #pragma unroll
     for (int u = 0; u < kGather - 1; ++u) {
       const bool ok = k + u * G < nn;
-      jg[u] = ok ? __ldg(nb + k + u * G) : -1;
+      jg[u] = ok ? list_entry<FL>(nb + k + u * G) : -1;
       og[u] = P.m4[cur][ok ? jg[u] : i];
     }
 #pragma unroll
@@ -1732,7 +1841,7 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
     // (ref_cells_adjacent); take the others' terms back out, bit for bit.
     if (entered) {
       for (int k2 = sub; k2 < nn; k2 += G) {
-        const int j = __ldg(nb + k2);
+        const int j = list_entry<FL>(nb + k2);
         const uint4 o = P.m4[cur][j];
         const float dx = frac_delta(me.x, o.x, s0), dy = frac_delta(me.y, o.y, s1), dz = frac_delta(me.z, o.z, s2);
         const float r2 = dist2(dx, dy, dz);
@@ -1762,7 +1871,7 @@ __device__ __forceinline__ void pair_sum_d(const DevPtrs& P, int cur, int i, int
   const Tables& T = *P.tab;
   const int lane = threadIdx.x & 31;
   const unsigned int below = (1u << lane) - 1u;
-  const unsigned int mine = ((1u << G) - 1u) << (lane & ~(G - 1));
+  const unsigned int mine = (0xffffffffu >> (32 - G)) << (lane & ~(G - 1));
   const int nn = active ? P.nnbr[i] : 0;
   const int* nb = P.nbr + (size_t)i * P.kmax;
   double4 me = make_double4(0.0, 0.0, 0.0, 0.0);
@@ -1796,7 +1905,7 @@ __device__ __forceinline__ void pair_sum_d(const DevPtrs& P, int cur, int i, int
       bool near = false;
       int j = 0;
       if (k < nn) {
-        j = __ldg(nb + k);
+        j = list_entry<FL>(nb + k);
         const uint4 o = P.m4[cur][j];
         const float dx = frac_delta(mu.x, o.x, s0), dy = frac_delta(mu.y, o.y, s1), dz = frac_delta(mu.z, o.z, s2);
         const float r2 = dx * dx + dy * dy + dz * dz;
@@ -1936,99 +2045,8 @@ __device__ __forceinline__ void integ_bead(const DevPtrs& P, int cur, int i, int
   // bonded forces: one function for every step variant, so stopped and
   // running steps round them alike
   if constexpr ((FL & (F_PAIRONLY | F_ENERGY)) == 0) fb = bonded_force<MIXED, (FL & F_FIELDS) != 0>(P, cur, i, ci, box, rs);
-  if ((FL & F_PAIRONLY) == 0 && (FL & (F_DU | F_ENERGY)) != 0 && ci < 0 && !(ci & 0x40000000)) {
-    const int p = ci & 0xfff, len = (ci >> 12) & 0xfff, set = (ci >> 24) & 0x1f;
-    // the chain's difference vectors in R (exact from the fractional
-    // mirror in the mixed form)
-    Vec3<R> er[4];
-    bool valid[4];
-    chain_vectors<MIXED, R>(P, cur, i, p, len, box, er, valid);
-    // terms owned by the first bead of each bond / bend: energies in FP64;
-    // size-change differences in FP64 (plain) or factored FP32 (mixed)
-    if constexpr (MIXED && (FL & F_DU) != 0) {
-      const float* cf = T.chainF[set];
-      const float sq[3] = {rs.sq_f[0], rs.sq_f[1], rs.sq_f[2]};
-      float du = 0.f;
-      if (valid[2]) du += bond_dpot_f(er[2], sq, cf);
-      if (valid[2] && valid[3]) du += bend_dpot_f(er[2], er[3], sq, cf + 2);
-      dU_bond += (double)du;
-    }
-    if constexpr ((FL & F_ENERGY) != 0 || (!MIXED && (FL & F_DU) != 0)) {
-      Vec3<double> e[4];
-      if constexpr (MIXED) {
-        chain_vectors<MIXED, double>(P, cur, i, p, len, box, e, valid);
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) e[k] = Vec3<double>{er[k].x, er[k].y, er[k].z};
-      }
-      const double* cd = T.chainD[set];
-      if constexpr ((FL & F_ENERGY) != 0) {
-        if (valid[2]) e_bond += bond_pot(e[2], cd);
-        if (valid[2] && valid[3]) e_bond += bend_pot(e[2], e[3], cd + 2);
-      }
-      if constexpr (!MIXED && (FL & F_DU) != 0) {
-        const Vec3<double> s2{e[2].x * rs.scale[0], e[2].y * rs.scale[1], e[2].z * rs.scale[2]};
-        const Vec3<double> s3{e[3].x * rs.scale[0], e[3].y * rs.scale[1], e[3].z * rs.scale[2]};
-        if (valid[2]) dU_bond += bond_pot(e[2], cd) - bond_pot(s2, cd);
-        if (valid[2] && valid[3]) dU_bond += bend_pot(e[2], e[3], cd + 2) - bend_pot(s2, s3, cd + 2);
-      }
-    }
-  }
-  // ---- BOND / BEND residue terms of this bead: energies and differences
-  // (their forces are in bonded_force)
-  if constexpr ((FL & F_PAIRONLY) == 0 && (FL & (F_DU | F_ENERGY)) != 0) {
-    if (P.n_terms > 0) {
-      const int o = P.orig[i];
-      const int e1 = P.term_off[o + 1];
-      const float sq_f[3] = {rs.sq_f[0], rs.sq_f[1], rs.sq_f[2]};
-      for (int e = P.term_off[o]; e < e1; ++e) {
-        const int4 t = P.terms[e];
-        const int kind = term_kind(t.x), role = term_role(t.x), set = term_set(t.x);
-        if (kind > kTermBend) {  // external fields: energy only (no size-change term in the reference)
-          if constexpr ((FL & F_ENERGY) != 0 && (FL & F_FIELDS) != 0)
-            if (role == 0) e_bond += field_potential<MIXED>(P, cur, i, t, box);
-          continue;
-        }
-        const double* cd = T.termD[set];
-        if (kind == kTermBond) {  // bond (first, second): the bead's force is mag (x_self - x_other)
-          if constexpr ((FL & (F_DU | F_ENERGY)) != 0) {
-            if (role == 0) {  // energy terms owned by the first bead
-              if constexpr (MIXED && (FL & F_DU) != 0)
-                dU_bond += (double)bond_dpot_f(term_vec<MIXED, float>(P, cur, t.y, t.z, box, rs), sq_f,
-                                               T.termF[set]);
-              if constexpr ((FL & F_ENERGY) != 0 || (!MIXED && (FL & F_DU) != 0)) {
-                const Vec3<double> d = term_vec<MIXED, double>(P, cur, t.y, t.z, box, rs);
-                if constexpr ((FL & F_ENERGY) != 0) e_bond += bond_pot(d, cd);
-                if constexpr (!MIXED && (FL & F_DU) != 0) {
-                  const Vec3<double> sd{d.x * rs.scale[0], d.y * rs.scale[1], d.z * rs.scale[2]};
-                  dU_bond += bond_pot(d, cd) - bond_pot(sd, cd);
-                }
-              }
-            }
-          }
-        } else {  // bend (first, second, third): da = x1 - x2, db = x2 - x3
-          if constexpr ((FL & (F_DU | F_ENERGY)) != 0) {
-            if (role == 0) {
-              if constexpr (MIXED && (FL & F_DU) != 0)
-                dU_bond += (double)bend_dpot_f(term_vec<MIXED, float>(P, cur, t.y, t.z, box, rs),
-                                               term_vec<MIXED, float>(P, cur, t.z, t.w, box, rs), sq_f,
-                                               T.termF[set]);
-              if constexpr ((FL & F_ENERGY) != 0 || (!MIXED && (FL & F_DU) != 0)) {
-                const Vec3<double> da = term_vec<MIXED, double>(P, cur, t.y, t.z, box, rs);
-                const Vec3<double> db = term_vec<MIXED, double>(P, cur, t.z, t.w, box, rs);
-                if constexpr ((FL & F_ENERGY) != 0) e_bond += bend_pot(da, db, cd);
-                if constexpr (!MIXED && (FL & F_DU) != 0) {
-                  const Vec3<double> sa{da.x * rs.scale[0], da.y * rs.scale[1], da.z * rs.scale[2]};
-                  const Vec3<double> sb{db.x * rs.scale[0], db.y * rs.scale[1], db.z * rs.scale[2]};
-                  dU_bond += bend_pot(da, db, cd) - bend_pot(sa, sb, cd);
-                }
-              }
-            }
-          }
-        }
-      }
-    }
-  }
+  if constexpr ((FL & F_PAIRONLY) == 0 && (FL & (F_DU | F_ENERGY)) != 0)
+    bonded_sums<MIXED, FL>(P, cur, i, ci, box, rs, dU_bond, e_bond);
   if constexpr ((FL & F_ENERGY) != 0) {
     const double vx = P.vx[i], vy = P.vy[i], vz = P.vz[i];
     e_kin = (vx * vx + vy * vy + vz * vz) / 2.0;
@@ -2198,31 +2216,52 @@ __global__ void __launch_bounds__(kBeadBlock) k_integ(DevPtrs P, int cur, StepEn
   }
 }
 
-// Barostat trial box of replica r (MD.cpp:593-611), drawn by k_ref_cells.
-__device__ __forceinline__ void trial_replica(const DevPtrs& P, int r) {
-  const int trial = P.g->trial_slot;
-  RepState& rs = P.rs[r];
+// Barostat trial box of a replica (MD.cpp:593-611) from its first draw, with
+// its size-change sums cleared.
+__device__ __forceinline__ void draw_trial(RepState& rs, const RepParams& rp, double u1) {
   rs.dU_pair = 0.0;
   rs.dU_bond = 0.0;
   rs.dUq_pair = 0;
   rs.dUq_bond = 0;
-  if (P.rp[r].dlxy == 0) {
+  if (rp.dlxy == 0) {
     const double one[3] = {1.0, 1.0, 1.0};
     set_scale(rs, one);
     return;
   }
-  const double u1 = P.trial_u[((size_t)trial * P.n_rep + r) * 2];
   double nb[3], s[3];
-  trial_box(rs.box, P.rp[r].dlxy, u1, nb, s);
+  trial_box(rs.box, rp.dlxy, u1, nb, s);
   for (int d = 0; d < 3; ++d) rs.trial_box[d] = nb[d];
   set_scale(rs, s);
-  rs.dU_pair = 0.0;
-  rs.dU_bond = 0.0;
-  rs.dUq_pair = 0;
-  rs.dUq_bond = 0;
+}
+__device__ __forceinline__ void trial_replica(const DevPtrs& P, int r) {  // drawn by k_ref_cells
+  const int trial = P.g->trial_slot;
+  draw_trial(P.rs[r], P.rp[r], P.trial_u[((size_t)trial * P.n_rep + r) * 2]);
 }
 
-// Metropolis decision (MD.cpp:677-720).
+// Metropolis decision of a replica (MD.cpp:677-720) from its second draw; on
+// acceptance the replica takes the trial box.  Returns the largest change of a
+// pair distance within rc + skin.
+__device__ __forceinline__ double decide_trial(RepState& rs, const RepParams& rp, const Tables& T, double u2) {
+  double dPot = rep_dU(rs);
+  if (rp.tension != 0) dPot += rp.tension * ((rs.trial_box[0] * rs.trial_box[1]) - (rs.box[0] * rs.box[1]));
+  rs.last_dU = dPot;
+  rs.n_trial++;
+  rs.accept = 0;
+  double shift = 0.0;
+  // MD.cpp's test D >= u2 || -dPot <= 0 with D = exp(dPot / kT); the
+  // exponential is needed only when the second clause fails
+  if (-dPot <= 0 || exp(dPot / rp.kT) >= u2) {
+    for (int d = 0; d < 3; ++d) {
+      shift = fmax(shift, fabs(rs.scale[d] - 1.0) * T.list_cut);
+      rs.box[d] = rs.trial_box[d];
+    }
+    derive_box(rs, rp.cell_cap, T.list_cut, T.rc);
+    rs.accept = 1;
+    rs.n_accept++;
+  }
+  return shift;
+}
+
 __global__ void k_mc(DevPtrs P) {
   const int trial = P.g->trial_slot;
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2231,28 +2270,9 @@ __global__ void k_mc(DevPtrs P) {
   const RepParams& rp = P.rp[r];
   rs.accept = 0;
   if (rp.dlxy == 0) return;
-  double dPot = rep_dU(rs);
-  if (rp.tension != 0) dPot += rp.tension * ((rs.trial_box[0] * rs.trial_box[1]) - (rs.box[0] * rs.box[1]));
-  const double u2 = P.trial_u[((size_t)trial * P.n_rep + r) * 2 + 1];
-  rs.last_dU = dPot;
-  rs.n_trial++;
-  // MD.cpp's test D >= u2 || -dPot <= 0 with D = exp(dPot / kT); the
-  // exponential is needed only when the second clause fails
-  if (-dPot <= 0 || exp(dPot / rp.kT) >= u2) {
-    double shift = 0.0;  // pair distances within rc + skin change by at most this
-    for (int d = 0; d < 3; ++d) {
-      shift = fmax(shift, fabs(rs.scale[d] - 1.0) * P.tab->list_cut);
-      rs.box[d] = rs.trial_box[d];
-    }
-    derive_box(rs, rp.cell_cap, P.tab->list_cut, P.tab->rc);
-    rs.accept = 1;
-    rs.n_accept++;
-    P.accept_log[(size_t)trial * P.n_rep + r] = 1;
-    atomicMax((unsigned long long*)&P.g->mc_shift, (unsigned long long)__double_as_longlong(shift));
-  } else {
-    rs.accept = 0;
-    P.accept_log[(size_t)trial * P.n_rep + r] = 0;
-  }
+  const double shift = decide_trial(rs, rp, *P.tab, P.trial_u[((size_t)trial * P.n_rep + r) * 2 + 1]);
+  P.accept_log[(size_t)trial * P.n_rep + r] = rs.accept;
+  if (rs.accept) atomicMax((unsigned long long*)&P.g->mc_shift, (unsigned long long)__double_as_longlong(shift));
 }
 
 // Completes a stopped step: optional restart half-kick, optional box rescale

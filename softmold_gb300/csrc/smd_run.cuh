@@ -1,0 +1,686 @@
+// The MD loop of a small or mid-size system as one persistent kernel.
+//
+// Kernel by kernel, a loop step of a few thousand beads is all latency: two
+// step kernels and, every second step, four list kernels of 5-25 us each that
+// keep at most a tenth of the chip's warps busy (1,176 beads: 35 us per step,
+// 15,000 beads: 41 us; here 17 and 32).  Here every CTA owns a contiguous range of the
+// cell-sorted beads and keeps their positions, velocities and bookkeeping in
+// shared memory; only the position mirror goes through global memory.  A step
+// is one grid barrier: each CTA forms its beads' pair sums (and beside them
+// the bonded forces and the noise), integrates them, writes the next mirror
+// and arrives.  A list rebuild adds one barrier (between the reordering and
+// the stencil scans), a barostat trial one (its summed energy difference).
+// Every barrier waits with a limit.
+//
+// The arithmetic of a step is that of k_force, k_integ, k_mc and k_finish, and
+// the mixed form's sums are exact in any order, so a mixed run has the same
+// bits here and there.
+#pragma once
+
+#include "smd_kernels.cuh"
+
+namespace smd {
+
+// threads per CTA at most: 80 registers per thread, or 64 where many beads want more warps
+__host__ __device__ constexpr int run_threads(int lanes) { return lanes == 8 ? 1024 : 768; }
+// Above this a step is throughput, and the separate kernels' occupancy wins
+// (15,000 beads: 32 us per step here, 41 us kernel by kernel).
+constexpr int kRunMaxBeads = 20000;
+constexpr int kRunCells = 20480;    // largest list-cell grid (its starts are kept in shared memory)
+constexpr int kRunSpinLimit = 1 << 22;  // polls of a barrier: some seconds
+
+// Grid-wide words of the persistent loop (zero between launches).
+struct RunSync {
+  // arrivals in the low 40 bits, then three 8-bit counts (by step modulo 3) of
+  // the CTAs with a bead beyond the list's margin: they ride on the arrival,
+  // so the barrier itself tells whether the list must be rebuilt
+  unsigned long long arrive;
+  unsigned int left;             // CTAs that are done with the kernel
+  unsigned int pad;
+  long long dq_pair[2], dq_bond[2];  // trial sums, alternating
+  double du_pair[2], du_bond[2];
+};
+
+struct RunArgs {
+  long long it;   // loop step of the first iteration
+  int cur;        // current mirror
+  int steps;      // iterations to run
+  int rate;       // barostat period
+  int barostat;
+  int beads;      // beads per CTA
+  int* cnt;       // 2 x n_cells_total cell counts, zero between launches
+  RunSync* sync;
+};
+
+// Shared memory per CTA beyond the static part.
+__host__ __device__ constexpr size_t run_align(size_t b) { return (b + 15) & ~(size_t)15; }
+__host__ __device__ constexpr size_t run_smem(int beads, int cells, bool mixed, int threads, int lanes) {
+  return run_align(sizeof(int) * ((size_t)cells + 1)) + run_align(sizeof(double) * 6 * (size_t)beads) +  // starts, x v
+         run_align(sizeof(double) * 3 * (size_t)beads) + run_align(sizeof(double) * 3 * (size_t)beads) +  // sums, bonded
+         run_align(sizeof(uint4) * (size_t)beads) + run_align(sizeof(int) * 4 * (size_t)beads) +
+         (mixed ? 0 : run_align(sizeof(int) * (size_t)kPairQueue * (threads / lanes)));
+}
+
+// Both bounds of the periodic wrap decided on the bits, in the integer pipe:
+// doubles order like signed integers when one of them is positive, and x < 0
+// is a set sign bit other than -0.
+__device__ __forceinline__ double wrap64(double x, double box) {
+  if (__double_as_longlong(x) > __double_as_longlong(box)) x -= box;
+  if ((unsigned long long)__double_as_longlong(x) > 0x8000000000000000ull) x += box;
+  return x;
+}
+
+// Appends to the lists of bead a (and of b, in the same cell; b < 0: none) the
+// beads [s, s + len) of the cell order within the list cut.  Distances come
+// from the exact fractional differences, whose wrap is the minimum image, so
+// thin grids need no other path; with five cells on every axis b's follow from
+// a's and the offset between the two (no candidate of the stencil is then near
+// half the box from a and in range of b).  ca, cb: the list lengths in shared
+// memory (several warps append to one bead's list).  One warp.
+template <bool OFFSET>
+__device__ __forceinline__ void run_scan(const uint4* m, int s, int len, const uint4& ma, const uint4& mb, int ia,
+                                         int ib, float x0, float x1, float x2, float lc2, int* oa, int* ob, int* ca,
+                                         int* cb, int kmax) {
+  const int lane = threadIdx.x & 31;
+  const unsigned int below = (1u << lane) - 1u;
+  float ex = 0.f, ey = 0.f, ez = 0.f;
+  if constexpr (OFFSET) {
+    ex = frac_delta(mb.x, ma.x, x0);
+    ey = frac_delta(mb.y, ma.y, x1);
+    ez = frac_delta(mb.z, ma.z, x2);
+  }
+  uint4 next = m[s + min(lane, len - 1)];
+  for (int k0 = 0; k0 < len; k0 += 32) {
+    const uint4 o = next;
+    const int k = k0 + lane, j = s + k;
+    if (k0 + 32 < len) next = m[s + min(k + 32, len - 1)];
+    const float ax = frac_delta(ma.x, o.x, x0), ay = frac_delta(ma.y, o.y, x1), az = frac_delta(ma.z, o.z, x2);
+    float bx, by, bz;
+    if constexpr (OFFSET) {
+      bx = ax + ex;
+      by = ay + ey;
+      bz = az + ez;
+    } else {
+      bx = frac_delta(mb.x, o.x, x0);
+      by = frac_delta(mb.y, o.y, x1);
+      bz = frac_delta(mb.z, o.z, x2);
+    }
+    const bool ha = (ax * ax + ay * ay + az * az < lc2) & (j != ia) & (k < len);
+    const bool hb = (bx * bx + by * by + bz * bz < lc2) & (j != ib) & (k < len) & (ib >= 0);
+    const unsigned int va = __ballot_sync(0xffffffffu, ha), vb = __ballot_sync(0xffffffffu, hb);
+    int at = 0;  // lane 0 claims for bead a, lane 1 for bead b
+    if (lane < 2) at = atomicAdd(lane == 0 ? ca : cb, __popc(lane == 0 ? va : vb));
+    const int pa = __shfl_sync(0xffffffffu, at, 0) + __popc(va & below);
+    const int pb = __shfl_sync(0xffffffffu, at, 1) + __popc(vb & below);
+    if (ha && pa < kmax) oa[pa] = j;
+    if (hb && pb < kmax) ob[pb] = j;
+  }
+}
+
+// Stencil rows t0 .. t1 - 1 (dy, dz) for bead a and, in the same cell, bead b.
+__device__ __forceinline__ void run_scan_rows(const DevPtrs& P, const uint4* m, const RepState& rs, const int* starts,
+                                              int t0, int t1, int ia, int ib, const uint4& ma, const uint4& mb,
+                                              int* ca, int* cb, float lc2) {
+  const int n0 = rs.ncell[0], n1 = rs.ncell[1], n2 = rs.ncell[2];
+  const int cx = __umulhi(ma.x, (unsigned)n0), cy = __umulhi(ma.y, (unsigned)n1), cz = __umulhi(ma.z, (unsigned)n2);
+  const float x0 = rs.len_per_frac[0], x1 = rs.len_per_frac[1], x2 = rs.len_per_frac[2];
+  const bool offset = n0 >= 5 && n1 >= 5 && n2 >= 5;
+  const int kmax = P.kmax;
+  int* oa = P.nbr + (size_t)ia * kmax;
+  int* ob = P.nbr + (size_t)(ib < 0 ? ia : ib) * kmax;
+  int xa = cx - 1, xb = cx + 1;
+  if (n0 < 3) {
+    xa = 0;
+    xb = n0 - 1;
+  }
+  for (int t = t0; t < t1; ++t) {
+    const int oz = t >= 6 ? 1 : (t >= 3 ? 0 : -1), oy = t - 3 * (oz + 1) - 1;
+    // axes with fewer than 3 cells take every cell once
+    if ((oy < 0 && n1 < 3) || (oy > 0 && n1 < 2) || (oz < 0 && n2 < 3) || (oz > 0 && n2 < 2)) continue;
+    int yy = cy + oy, zz = cz + oz;
+    yy += yy < 0 ? n1 : (yy >= n1 ? -n1 : 0);
+    zz += zz < 0 ? n2 : (zz >= n2 ? -n2 : 0);
+    const int row = n0 * (yy + n1 * zz);
+    // cells xa .. xb, or two ranges where they wrap
+    const bool wraps = xa < 0 || xb >= n0;
+    int s = starts[row + (xa < 0 ? n0 - 1 : xa)], len = starts[row + (wraps ? n0 : xb + 1)] - s;
+    for (int half = 0;; ++half) {
+      if (len > 0) {
+        if (offset) run_scan<true>(m, s, len, ma, mb, ia, ib, x0, x1, x2, lc2, oa, ob, ca, cb, kmax);
+        else run_scan<false>(m, s, len, ma, mb, ia, ib, x0, x1, x2, lc2, oa, ob, ca, cb, kmax);
+      }
+      if (!wraps || half) break;
+      s = starts[row];
+      len = starts[row + (xa < 0 ? xb + 1 : 1)] - s;
+    }
+  }
+}
+
+template <bool MIXED, int G>
+__global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A) {
+  using R = typename std::conditional<MIXED, float, double>::type;
+  using Sum = typename std::conditional<MIXED, long long, double>::type;
+  extern __shared__ uint4 run_dyn[];
+  __shared__ RepState rs;
+  __shared__ R sF[6 * kMaxTypes * kMaxTypes], sU[6 * kMaxTypes * kMaxTypes];
+  __shared__ int wsum[run_threads(G) / 32];
+  __shared__ float smax[run_threads(G) / 32];
+  __shared__ long long sdq[2];
+  __shared__ double sdu[2];
+  __shared__ double slack, shift_s;
+  __shared__ int rebuild, slot, abort_s;
+  __shared__ unsigned long long seen;
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  const int b0 = blockIdx.x * A.beads, nb = min(A.beads, P.n - b0);
+  const int ncell = P.n_cells_total;
+  // dynamic shared memory (run_smem)
+  unsigned char* at = reinterpret_cast<unsigned char*>(run_dyn);
+  int* starts = reinterpret_cast<int*>(at);
+  at += run_align(sizeof(int) * ((size_t)ncell + 1));
+  double* st = reinterpret_cast<double*>(at);  // x, y, z, vx, vy, vz of the CTA's beads
+  at += run_align(sizeof(double) * 6 * (size_t)A.beads);
+  Sum* fsum = reinterpret_cast<Sum*>(at);
+  at += run_align(sizeof(double) * 3 * (size_t)A.beads);
+  R* fbond = reinterpret_cast<R*>(at);  // mixed: bonded force + noise in FP32; plain: bonded force
+  at += run_align(sizeof(double) * 3 * (size_t)A.beads);
+  uint4* ref = reinterpret_cast<uint4*>(at);
+  at += run_align(sizeof(uint4) * (size_t)A.beads);
+  int* orig = reinterpret_cast<int*>(at);
+  int* cinfo = orig + A.beads;
+  int* key = cinfo + A.beads;
+  int* cnt = key + A.beads;
+  at += run_align(sizeof(int) * 4 * (size_t)A.beads);
+  int* queue = reinterpret_cast<int*>(at);
+  const Tables& T = *P.tab;
+  const RepParams& rp = P.rp[0];
+  const int nT = T.nT;
+  const int NB = A.beads;
+
+  // ---- entry
+  for (int k = tid; k < (int)(sizeof(RepState) / 4); k += nt)
+    reinterpret_cast<int*>(&rs)[k] = reinterpret_cast<const int*>(P.rs)[k];
+  for (int k = tid; k < 6 * nT * nT; k += nt) {
+    if constexpr (MIXED) {
+      sF[k] = T.fF[k];
+      sU[k] = T.fU[k];
+    } else {
+      sF[k] = T.dF[k];
+      sU[k] = T.dU[k];
+    }
+  }
+  if (*(volatile int*)&P.g->error & 8) return;  // an earlier launch gave up: its words are not clean
+  if (tid == 0) {
+    slack = P.g->slack;
+    slot = P.g->trial_slot;
+    rebuild = P.g->rebuild;
+    abort_s = 0;
+  }
+  if (tid < nb) {
+    const int i = b0 + tid;
+    st[tid] = P.x[i];
+    st[NB + tid] = P.y[i];
+    st[2 * NB + tid] = P.z[i];
+    st[3 * NB + tid] = P.vx[i];
+    st[4 * NB + tid] = P.vy[i];
+    st[5 * NB + tid] = P.vz[i];
+    ref[tid] = P.ref[i];
+    orig[tid] = P.orig[i];
+    cinfo[tid] = P.cinfo[i];
+  }
+  __syncthreads();
+  const double gamma = rp.gamma, dt = rp.dt, h = dt * 0.5;
+  long long it = A.it;
+  int cur = A.cur;
+  unsigned long long waited = 0;  // barriers so far
+
+  // Arrives with inc and waits for every CTA; false when the limit ran out.
+  auto barrier = [&](unsigned long long inc) -> bool {
+    __syncthreads();
+    ++waited;
+    if (tid == 0) {
+      const unsigned long long target = waited * gridDim.x;
+      // release: the CTA's writes (ordered before by the block barrier) are
+      // visible to whoever sees the arrival; the acquire below is its other end
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&A.sync->arrive), "l"(inc) : "memory");
+      unsigned long long v = 0;
+      int polls = 0;
+      for (;;) {
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&A.sync->arrive) : "memory");
+        if ((v & ((1ull << 40) - 1)) >= target) break;
+        if (++polls > kRunSpinLimit) {
+          atomicOr(&P.g->error, 8);
+          abort_s = 1;
+          break;
+        }
+      }
+      seen = v;
+    }
+    __syncthreads();
+    return abort_s == 0;
+  };
+  auto trial_at = [&](long long step) { return A.barostat && step % A.rate == 0 && step != 0; };
+  // list cell of own bead t on the current grid
+  auto cell_of = [&](const uint4& m) {
+    const int n0 = rs.ncell[0], n1 = rs.ncell[1], n2 = rs.ncell[2];
+    return (int)__umulhi(m.x, (unsigned)n0) +
+           n0 * ((int)__umulhi(m.y, (unsigned)n1) + n1 * (int)__umulhi(m.z, (unsigned)n2));
+  };
+  // counts own bead t's cell (every lane of the warp calls it)
+  auto count_cell = [&](bool on, int c, int* counts) {
+    const unsigned int lanes = __ballot_sync(0xffffffffu, on);
+    if (!on) return;
+    const unsigned int same = __match_any_sync(lanes, c);
+    if (lane == __ffs(same) - 1) atomicAdd(&counts[c], __popc(same));
+  };
+  // own bead t's cell on the reference's grid (the size-change passes)
+  auto ref_key = [&](const double x[3]) {
+    unsigned long long k = 0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      k |= (unsigned long long)(ref_cell_coord(x[d], rs.ref_cs[d], rs.ref_inv_cs[d], rs.refn[d]) & 0x1fffff) << (21 * d);
+    return k;
+  };
+  // the trial of a barostat step: every CTA draws it into its own copy
+  auto draw = [&]() {
+    if (tid == 0) draw_trial(rs, rp, P.trial_u[(size_t)slot * 2]);
+  };
+  bool trial = trial_at(it);
+  {
+    const bool stale = rebuild != 0;
+    if (trial) draw();
+    if (stale && tid < ((nb + 31) & ~31)) {
+      const bool on = tid < nb;
+      const int c = on ? cell_of(P.m4[cur][b0 + tid]) : 0;
+      if (on) key[tid] = c;
+      count_cell(on, c, A.cnt + ncell);
+    }
+    if (trial && !stale && tid < nb) {
+      const double x[3] = {st[tid], st[NB + tid], st[2 * NB + tid]};
+      P.refcell[b0 + tid] = ref_key(x);
+    }
+    if ((stale || trial) && !barrier(1)) return;
+  }
+
+  int trials = 0;
+  for (int s = 0; s < A.steps; ++s) {
+    const bool last = s + 1 == A.steps;
+    if (rebuild) {
+      // ---- exclusive scan of the cell counts, by every CTA for itself
+      const int* counts = A.cnt + (size_t)((s + 1) & 1) * ncell;
+      {
+        constexpr int kBatch = 4;
+        int most = 0;
+        for (int c = tid; c < ncell; c += kBatch * nt) {  // loads issued together
+          int v[kBatch];
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u) v[u] = c + u * nt < ncell ? __ldcg(counts + c + u * nt) : 0;
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u)
+            if (c + u * nt < ncell) {
+              starts[c + u * nt] = v[u];
+              most = max(most, v[u]);
+            }
+        }
+        if (most > kNbrMaxCell) atomicOr(&P.g->error, 2);
+        __syncthreads();
+        // each thread sums an odd number of consecutive counts (no bank conflicts)
+        const int per = ((ncell + nt - 1) / nt) | 1, c0 = min(tid * per, ncell), c1 = min(c0 + per, ncell);
+        int sum = 0;
+        for (int c = c0; c < c1; ++c) sum += starts[c];
+        int x = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, x, o);
+          if (lane >= o) x += y;
+        }
+        if (lane == 31) wsum[warp] = x;
+        __syncthreads();
+        int before = 0;
+        for (int w = 0; w < warp; ++w) before += wsum[w];
+        int ex = before + x - sum;
+        for (int c = c0; c < c1; ++c) {
+          const int v = starts[c];
+          starts[c] = ex;
+          ex += v;
+        }
+        if (tid == nt - 1) starts[ncell] = P.n;
+      }
+      __syncthreads();
+      // ---- scatter to the new order (cell_count: the cells' fill)
+      if (tid < ((nb + 31) & ~31)) {
+        const bool on = tid < nb;
+        const unsigned int lanes = __ballot_sync(0xffffffffu, on);
+        if (on) {
+          const int c = key[tid];
+          const unsigned int same = __match_any_sync(lanes, c);
+          const int leader = __ffs(same) - 1;
+          int base = 0;
+          if (lane == leader) base = atomicAdd(&P.cell_count[c], __popc(same));
+          base = __shfl_sync(same, base, leader);
+          const int nw_i = starts[c] + base + __popc(same & ((1u << lane) - 1u));
+          P.tx[nw_i] = st[tid];
+          P.ty[nw_i] = st[NB + tid];
+          P.tz[nw_i] = st[2 * NB + tid];
+          P.tvx[nw_i] = st[3 * NB + tid];
+          P.tvy[nw_i] = st[4 * NB + tid];
+          P.tvz[nw_i] = st[5 * NB + tid];
+          const int o = orig[tid];
+          P.torig[nw_i] = o;
+          P.tcinfo[nw_i] = cinfo[tid];
+          P.inv[o] = nw_i;
+          P.m4[cur ^ 1][nw_i] = P.m4[cur][b0 + tid];
+          if constexpr (!MIXED) P.d4[cur ^ 1][nw_i] = P.d4[cur][b0 + tid];
+          if (trial) {
+            const double x[3] = {st[tid], st[NB + tid], st[2 * NB + tid]};
+            P.refcell[nw_i] = ref_key(x);
+          }
+        }
+      }
+      if (!barrier(1)) return;
+      cur ^= 1;
+      if (tid < nb) {
+        const int i = b0 + tid;
+        st[tid] = __ldcg(P.tx + i);
+        st[NB + tid] = __ldcg(P.ty + i);
+        st[2 * NB + tid] = __ldcg(P.tz + i);
+        st[3 * NB + tid] = __ldcg(P.tvx + i);
+        st[4 * NB + tid] = __ldcg(P.tvy + i);
+        st[5 * NB + tid] = __ldcg(P.tvz + i);
+        const int o = __ldcg(P.torig + i);
+        orig[tid] = o;
+        P.orig[i] = o;
+        cinfo[tid] = __ldcg(P.tcinfo + i);
+        ref[tid] = P.m4[cur][i];
+        cnt[tid] = 0;
+      }
+      if (tid == 0) {
+        slack = 0.0;
+        if (blockIdx.x == 0) P.g->n_rebuilds++;
+      }
+      __syncthreads();
+      // ---- lists: a row of the stencil for two neighbouring beads per warp
+      {
+        const float lcut = MIXED ? T.list_cut_f + 1e-4f
+                                 : T.list_cut_f * (1.f + 4e-6f) + 1e-4f +
+                                       4.f * fmaxf(rs.len_per_frac[0], fmaxf(rs.len_per_frac[1], rs.len_per_frac[2]));
+        const float lc2 = lcut * lcut;
+        const uint4* m = P.m4[cur];
+        // tasks: two neighbouring beads by three stencil rows, or by one where
+        // that leaves warps idle
+        const int pairs = (nb + 1) >> 1, rows = pairs * 3 >= nw ? 3 : 1, parts = 9 / rows;
+        for (int task = warp; task < pairs * parts; task += nw) {
+          const int p = rows == 3 ? task / 3 : task / 9, t0 = (task - p * parts) * rows;
+          const int a = 2 * p, b = a + 1 < nb ? a + 1 : a;
+          const uint4 ma = ref[a], mb = ref[b];
+          const int i = b0 + a;
+          if (b != a && cell_of(ma) == cell_of(mb)) {
+            run_scan_rows(P, m, rs, starts, t0, t0 + rows, i, i + 1, ma, mb, cnt + a, cnt + b, lc2);
+          } else {
+            for (int q = a; q <= b; ++q)
+              run_scan_rows(P, m, rs, starts, t0, t0 + rows, b0 + q, -1, ref[q], ref[q], cnt + q, cnt + q, lc2);
+          }
+        }
+      }
+      __syncthreads();
+      if (tid < nb) {
+        const int count = cnt[tid];
+        P.nnbr[b0 + tid] = min(count, P.kmax);
+        if (count > *(volatile int*)&P.g->max_nbr) atomicMax(&P.g->max_nbr, count);
+        if (count > P.kmax) {
+          atomicOr(&P.g->error, 1);
+          atomicMax(&P.g->need_nbr, count);
+        }
+      }
+      for (int c = blockIdx.x * nt + tid; c < ncell; c += gridDim.x * nt) P.cell_count[c] = 0;
+      __syncthreads();
+    }
+    // the counts of the step before this one: read above at the latest
+    for (int c = blockIdx.x * nt + tid; c < ncell; c += gridDim.x * nt) A.cnt[(size_t)((s + 1) & 1) * ncell + c] = 0;
+    if (tid == 0) {
+      sdq[0] = sdq[1] = 0;
+      sdu[0] = sdu[1] = 0.0;
+    }
+    if (trial) __syncthreads();
+
+    // ---- forces: warps take the bonded terms and the noise, then the pair sums
+    const int bond_tasks = (nb + 31) >> 5, pair_tasks = (nb * G + 31) >> 5;
+    for (int task = warp; task < bond_tasks + pair_tasks; task += nw) {
+      if (task < bond_tasks) {
+        const int b = task * 32 + lane;
+        double dU = 0.0, unused = 0.0;
+        if (b < nb) {
+          const int ci = cinfo[b];
+          const double box[3] = {rs.box[0], rs.box[1], rs.box[2]};
+          const Vec3<R> f = bonded_force<MIXED, false>(P, cur, b0 + b, ci, box, rs);
+          if (trial) bonded_sums<MIXED, F_DU>(P, cur, b0 + b, ci, box, rs, dU, unused);
+          if constexpr (MIXED) {
+            float nf[3];
+            langevin_noise_f(rp.seed, orig[b] - rp.bead_begin, it, 0, rp.sig31f, nf);
+            fbond[3 * b] = f.x + nf[0];
+            fbond[3 * b + 1] = f.y + nf[1];
+            fbond[3 * b + 2] = f.z + nf[2];
+          } else {
+            fbond[3 * b] = f.x;
+            fbond[3 * b + 1] = f.y;
+            fbond[3 * b + 2] = f.z;
+          }
+        }
+        if (trial) {
+          if constexpr (MIXED) {
+            long long q = __double2ll_rn(dU * 4294967296.0);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+            if (lane == 0) atomicAdd((unsigned long long*)&sdq[1], (unsigned long long)q);
+          } else {
+            dU = warp_sum(dU);
+            if (lane == 0) atomicAdd(&sdu[1], dU);
+          }
+        }
+      } else {
+        const int g = (task - bond_tasks) * 32 + lane;
+        const int b = g / G, sub = g % G;
+        const bool active = b < nb;
+        const int i = b0 + (active ? b : 0);
+        if constexpr (MIXED) {
+          long long qx = 0, qy = 0, qz = 0, dq = 0;
+          float unused = 0.f;
+          if (active) {
+            if (trial)
+              pair_sum_q<F_DU | F_RUN, G>(P, cur, i, sub, rs, sF, sU, nT, qx, qy, qz, dq, unused);
+            else
+              pair_sum_q<F_RUN, G>(P, cur, i, sub, rs, sF, sU, nT, qx, qy, qz, dq, unused);
+          }
+#pragma unroll
+          for (int o = G / 2; o > 0; o >>= 1) {
+            qx += __shfl_xor_sync(0xffffffffu, qx, o);
+            qy += __shfl_xor_sync(0xffffffffu, qy, o);
+            qz += __shfl_xor_sync(0xffffffffu, qz, o);
+          }
+          if (active && sub == 0) {
+            fsum[3 * b] = qx;
+            fsum[3 * b + 1] = qy;
+            fsum[3 * b + 2] = qz;
+          }
+          if (trial) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) dq += __shfl_xor_sync(0xffffffffu, dq, o);
+            if (lane == 0) atomicAdd((unsigned long long*)&sdq[0], (unsigned long long)dq);
+          }
+        } else {
+          double fx = 0, fy = 0, fz = 0, ep = 0, dU = 0;
+          int* q = queue + (size_t)(tid / G) * kPairQueue;
+          if (trial)
+            pair_sum_d<F_DU | F_RUN, G>(P, cur, i, sub, active, rs, sF, sU, nT, q, fx, fy, fz, ep, dU);
+          else
+            pair_sum_d<F_RUN, G>(P, cur, i, sub, active, rs, sF, sU, nT, q, fx, fy, fz, ep, dU);
+#pragma unroll
+          for (int o = G / 2; o > 0; o >>= 1) {
+            fx += __shfl_xor_sync(0xffffffffu, fx, o);
+            fy += __shfl_xor_sync(0xffffffffu, fy, o);
+            fz += __shfl_xor_sync(0xffffffffu, fz, o);
+          }
+          if (active && sub == 0) {
+            fsum[3 * b] = fx;
+            fsum[3 * b + 1] = fy;
+            fsum[3 * b + 2] = fz;
+          }
+          if (trial) {
+            dU = warp_sum(dU);
+            if (lane == 0) atomicAdd(&sdu[0], dU);
+          }
+        }
+      }
+    }
+    __syncthreads();
+
+    // ---- acceleration of own bead tid
+    double a[3] = {0, 0, 0}, x[3] = {0, 0, 0}, v[3] = {0, 0, 0};
+    int ti = 0;
+    unsigned int w = 0;
+    if (tid < nb) {
+      w = P.m4[cur][b0 + tid].w;
+      ti = w & 0xff;
+      for (int d = 0; d < 3; ++d) {
+        x[d] = st[d * NB + tid];
+        v[d] = st[(3 + d) * NB + tid];
+      }
+      if constexpr (MIXED) {
+        for (int d = 0; d < 3; ++d)
+          a[d] = fma(-gamma, v[d], fma((double)fsum[3 * tid + d], T.inv_fscale, (double)fbond[3 * tid + d]));
+      } else {
+        double noise[3];
+        langevin_noise(rp.seed, orig[tid] - rp.bead_begin, it, 0, rp.sig31, noise);
+        for (int d = 0; d < 3; ++d) a[d] = fma(-gamma, v[d], fsum[3 * tid + d] + fbond[3 * tid + d]) + noise[d];
+      }
+      if (ti != 0)
+        for (int d = 0; d < 3; ++d) v[d] = fma(a[d], h, v[d]);  // second half-kick
+    }
+    bool scaled = false;
+    if (trial) {
+      // ---- the trial's energy difference over the grid, and the decision by every CTA
+      const int par = trials & 1;
+      if (tid == 0) {
+        if constexpr (MIXED) {
+          atomicAdd((unsigned long long*)&A.sync->dq_pair[par], (unsigned long long)sdq[0]);
+          atomicAdd((unsigned long long*)&A.sync->dq_bond[par], (unsigned long long)sdq[1]);
+        } else {
+          atomicAdd(&A.sync->du_pair[par], sdu[0]);
+          atomicAdd(&A.sync->du_bond[par], sdu[1]);
+        }
+        if (blockIdx.x == 0) {  // the previous trial's sums: every CTA has read them
+          A.sync->dq_pair[par ^ 1] = A.sync->dq_bond[par ^ 1] = 0;
+          A.sync->du_pair[par ^ 1] = A.sync->du_bond[par ^ 1] = 0.0;
+        }
+      }
+      if (!barrier(1)) return;
+      if (tid == 0) {
+        rs.dUq_pair = __ldcg(&A.sync->dq_pair[par]);
+        rs.dUq_bond = __ldcg(&A.sync->dq_bond[par]);
+        rs.dU_pair = __ldcg(&A.sync->du_pair[par]);
+        rs.dU_bond = __ldcg(&A.sync->du_bond[par]);
+        rs.accept = 0;
+        shift_s = 0.0;
+        if (rp.dlxy != 0) {
+          shift_s = decide_trial(rs, rp, T, P.trial_u[(size_t)slot * 2 + 1]);
+          if (blockIdx.x == 0) P.accept_log[slot] = rs.accept;
+        }
+        slack += shift_s;
+        ++slot;
+      }
+      __syncthreads();
+      scaled = rs.accept != 0;
+      ++trials;
+    }
+    // ---- first half-kick and drift of the next step, its mirror and cell count
+    const bool next_trial = trial_at(it + 1);
+    float vmax = 0.f;
+    int c = 0;
+    if (tid < nb) {
+      const int i = b0 + tid;
+      if (scaled)
+        for (int d = 0; d < 3; ++d) x[d] *= rs.scale[d];
+      if (ti != 0) {
+        for (int d = 0; d < 3; ++d) {
+          v[d] = fma(a[d], h, v[d]);
+          x[d] = wrap64(fma(v[d], dt, x[d]), rs.box[d]);
+          st[(3 + d) * NB + tid] = v[d];
+        }
+      }
+      for (int d = 0; d < 3; ++d) st[d * NB + tid] = x[d];
+      const uint4 mn = make_uint4(to_frac(x[0], rs.frac_per_len[0]), to_frac(x[1], rs.frac_per_len[1]),
+                                  to_frac(x[2], rs.frac_per_len[2]), w);
+      vmax = displacement(ref[tid], mn.x, mn.y, mn.z, rs);
+      P.m4[cur ^ 1][i] = mn;
+      if constexpr (!MIXED) P.d4[cur ^ 1][i] = make_double4(x[0], x[1], x[2], P.d4[cur][i].w);
+      c = cell_of(mn);
+      key[tid] = c;
+      if (next_trial && !last) P.refcell[i] = ref_key(x);
+    }
+    if (!last && tid < ((nb + 31) & ~31)) count_cell(tid < nb, c, A.cnt + (size_t)(s & 1) * ncell);
+    vmax = warp_max(vmax);
+    if (lane == 0) smax[warp] = vmax;
+    __syncthreads();
+    // ---- arrive: a bead beyond the margin (half the skin less the slack) asks for a rebuild
+    unsigned long long inc = 1;
+    if (tid == 0) {
+      float bm = 0.f;
+      for (int k = 0; k < nw; ++k) bm = fmaxf(bm, smax[k]);
+      if ((double)bm + slack > P.half_skin) inc += 1ull << (40 + 8 * (s % 3));
+      if (last && bm > 0.f) atomicMax(&P.g->dmax_bits, __float_as_uint(bm));
+      // CTA 0 clears the field of two steps ago (the next step's), which every CTA has read
+      if (blockIdx.x == 0 && s >= 2) inc -= ((seen >> (40 + 8 * ((s + 1) % 3))) & 0xffull) << (40 + 8 * ((s + 1) % 3));
+    }
+    if (!barrier(inc)) return;
+    if (tid == 0) {
+      rebuild = ((seen >> (40 + 8 * (s % 3))) & 0xffull) != 0;
+    }
+    cur ^= 1;
+    ++it;
+    trial = next_trial;
+    if (trial && !last) draw();
+    __syncthreads();
+  }
+
+  // ---- exit: the CTA's beads back to global memory, the mirror where the host expects it
+  const int want = A.cur ^ (A.steps & 1);
+  if (tid < nb) {
+    const int i = b0 + tid;
+    P.x[i] = st[tid];
+    P.y[i] = st[NB + tid];
+    P.z[i] = st[2 * NB + tid];
+    P.vx[i] = st[3 * NB + tid];
+    P.vy[i] = st[4 * NB + tid];
+    P.vz[i] = st[5 * NB + tid];
+    P.ref[i] = ref[tid];
+    P.cinfo[i] = cinfo[tid];
+    if (cur != want) {
+      P.m4[want][i] = P.m4[cur][i];
+      if constexpr (!MIXED) P.d4[want][i] = P.d4[cur][i];
+    }
+  }
+  if (blockIdx.x == 0) {
+    for (int k = tid; k < (int)(sizeof(RepState) / 4); k += nt)
+      reinterpret_cast<int*>(P.rs)[k] = reinterpret_cast<const int*>(&rs)[k];
+    if (tid == 0) {
+      P.g->slack = slack;
+      P.g->trial_slot = slot;
+      P.g->rebuild = rebuild;
+      P.g->it = it;
+      P.g->last_disp = __uint_as_float(atomicExch(&P.g->dmax_bits, 0u));
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    if (atomicAdd(&A.sync->left, 1u) == gridDim.x - 1) {  // every CTA has passed its last barrier
+      A.sync->arrive = 0;
+      A.sync->left = 0;
+      for (int k = 0; k < 2; ++k) {
+        A.sync->dq_pair[k] = A.sync->dq_bond[k] = 0;
+        A.sync->du_pair[k] = A.sync->du_bond[k] = 0.0;
+      }
+    }
+  }
+}
+
+}  // namespace smd
