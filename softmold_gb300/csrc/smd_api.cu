@@ -474,7 +474,7 @@ int run_fits_device(smd_system* h, bool* fits) {
 int run_setup(smd_system* h) {
   auto& r = h->run;
   r.grid = 0;
-  if (h->n_rep != 1 || h->n_sph > 0 || h->has_fields || h->n > kRunMaxBeads || h->n_cells > kRunCells) return 0;
+  if (h->n_rep != 1 || h->n_sph > 0 || h->n_terms > 0 || h->n > kRunMaxBeads || h->n_cells > kRunCells) return 0;
   const int ctas = std::min(h->sms, 255);
   r.beads = std::max(8, (h->n + ctas - 1) / ctas);
   r.lanes = r.beads <= 24 ? 32 : (r.beads <= 48 ? 16 : 8);
@@ -489,7 +489,7 @@ int run_setup(smd_system* h) {
   else rc = r.lanes == 32 ? run_fits_device<false, 32>(h, &fits) : (r.lanes == 16 ? run_fits_device<false, 16>(h, &fits) : run_fits_device<false, 8>(h, &fits));
   r.grid = 0;
   if (rc || !fits) return rc;
-  if ((rc = h->alloc(&r.cnt, 2 * (size_t)h->n_cells)) || (rc = h->alloc(&r.sync, 1))) return rc;
+  if ((rc = h->alloc(&r.cnt, 2 * (size_t)run_cells(h->n_cells))) || (rc = h->alloc(&r.sync, 1))) return rc;
   r.grid = grid;
   return 0;
 }

@@ -21,17 +21,21 @@ enum StepFlags {
   F_FORCES = 16,    // conservative forces only, written to P.force_out (file order)
   F_PAIRONLY = 32,  // with F_FORCES: non-bonded part only
   F_ENERGY = 64,    // energies only (pair, bonded, kinetic) into RepState
-  F_FIELDS = 128,   // the system has external-field terms (their out-of-line
+  F_FIELDS = 128    // the system has external-field terms (their out-of-line
                     // evaluation is compiled in only with this flag)
-  F_RUN = 256       // inside the persistent loop kernel, which writes the lists
-                    // it reads: no read-only loads of them
 };
 
-template <int FL>
-__device__ __forceinline__ int list_entry(const int* p) {
-  if constexpr ((FL & F_RUN) != 0) return *p; else return __ldg(p);
-}
-
+// A bead's list and the mirror it indexes.  NC: through read-only loads (not
+// in the persistent loop, which writes the lists it reads).
+template <bool NC>
+struct BeadList {
+  const int* list;
+  const uint4* mirror;
+  __device__ __forceinline__ int entry(int k) const {
+    if constexpr (NC) return __ldg(list + k); else return list[k];
+  }
+  __device__ __forceinline__ uint4 pos(int j) const { return mirror[j]; }
+};
 // ------------------------------------------------------------ last block
 // Runs once per launch after every block has passed its atomics.  The list
 // stays valid while every bead is within half the skin of its build position
@@ -1678,19 +1682,26 @@ __device__ __forceinline__ bool ref_cells_adjacent(const DevPtrs& P, const RepSt
   return adj;
 }
 
+// Place of constant k of the force table in its packed order: of a row's six,
+// the edges C0 and C3 first, then C1 C2 and C4 C5.
+__device__ __forceinline__ int pack_force_row(int k) {
+  const int row = k / 6 * 6, q = k - row;
+  return row + (q == 3 ? 1 : (q == 1 || q == 2 ? q + 1 : q));
+}
+
 // Mixed-form pair sums of bead i over its Verlet list, lane `sub` of its G
 // lanes: each pair force rounded to fixed point and summed in int32 per lane
 // (flushed to int64 every 32 terms), with F_DU the size-change difference
-// (fixed point) and with F_ENERGY the pair energy.  sF, sU: the FP32 tables
-// in shared memory.
-template <int FL, int G>
-__device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int sub, const RepState& rs,
-                                           const float* sF, const float* sU, int nT, long long& qx, long long& qy,
-                                           long long& qz, long long& dq, float& eacc) {
+// (fixed point) and with F_ENERGY the pair energy.  The list has nn entries.
+// sF, sU: the FP32 tables in shared memory, sF packed (pack_force_row): a pair's row is two 8-byte loads, its two
+// segment edges and then the segment's two constants.  (Four 4-byte loads
+// took a third of the pass's L1 wavefronts, which bound it.)
+template <int FL, int G, typename List>
+__device__ __forceinline__ void pair_sum_q(const DevPtrs& P, const List& list, int nn, int i, int sub, const RepState& rs,
+                                           const float* sF, const float* sU, int nT, long long& qx,
+                                           long long& qy, long long& qz, long long& dq, float& eacc) {
   const Tables& T = *P.tab;
-  const int nn = P.nnbr[i];
-  const int* nb = P.nbr + (size_t)i * P.kmax;
-  const uint4 me = P.m4[cur][i];
+  const uint4 me = list.pos(i);
   const int ti = me.w & 0xff;
   const float s0 = rs.len_per_frac[0], s1 = rs.len_per_frac[1], s2 = rs.len_per_frac[2];
   float sq0 = 0.f, sq1 = 0.f, sq2 = 0.f;
@@ -1707,11 +1718,13 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
   // below 2^26 in fixed point, so 32 of them cannot overflow
   int ax = 0, ay = 0, az = 0;
   auto pair_force_q = [&](float dx, float dy, float dz, float r2, int tj) {
-    const float* c = rowF + 6 * tj;
+    const float2* c = reinterpret_cast<const float2*>(rowF + 6 * tj);
     const float rinv = rsqrtf(r2), r = r2 * rinv;
-    const int ci = (r >= c[0]) ? 3 : 0;
-    const float m = c[ci] - r;
-    float mag = ((c[ci + 1] - c[ci + 2] * m) * m) * rinv * fs;
+    const float2 edge = c[0];
+    const bool outer = r >= edge.x;
+    const float m = (outer ? edge.y : edge.x) - r;
+    const float2 seg = c[outer ? 2 : 1];
+    float mag = ((seg.x - seg.y * m) * m) * rinv * fs;
     mag = (r2 < rc2) ? mag : 0.f;
     ax += __float2int_rn(dx * mag);
     ay += __float2int_rn(dy * mag);
@@ -1770,7 +1783,7 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
     bool more = k + (kGather - 1) * G < nn;
     if (more) {
 #pragma unroll
-      for (int u = 0; u < kGather; ++u) jn[u] = list_entry<FL>(nb + k + u * G);
+      for (int u = 0; u < kGather; ++u) jn[u] = list.entry(k + u * G);
     }
     for (; more; k += kGather * G) {
       uint4 og[kGather];
@@ -1778,12 +1791,12 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
 #pragma unroll
       for (int u = 0; u < kGather; ++u) {
         jg[u] = jn[u];
-        og[u] = P.m4[cur][jg[u]];
+        og[u] = list.pos(jg[u]);
       }
       more = k + (2 * kGather - 1) * G < nn;
       if (more) {
 #pragma unroll
-        for (int u = 0; u < kGather; ++u) jn[u] = list_entry<FL>(nb + k + (kGather + u) * G);
+        for (int u = 0; u < kGather; ++u) jn[u] = list.entry(k + (kGather + u) * G);
       }
       batch(og, jg);
     }
@@ -1793,8 +1806,8 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
       int jg[kGather];
 #pragma unroll
       for (int u = 0; u < kGather; ++u) {
-        jg[u] = list_entry<FL>(nb + k + u * G);
-        og[u] = P.m4[cur][jg[u]];
+        jg[u] = list.entry(k + u * G);
+        og[u] = list.pos(jg[u]);
       }
       batch(og, jg);
     }
@@ -1807,8 +1820,8 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
 #pragma unroll
     for (int u = 0; u < kGather - 1; ++u) {
       const bool ok = k + u * G < nn;
-      jg[u] = ok ? list_entry<FL>(nb + k + u * G) : -1;
-      og[u] = P.m4[cur][ok ? jg[u] : i];
+      jg[u] = ok ? list.entry(k + u * G) : -1;
+      og[u] = list.pos(ok ? jg[u] : i);
     }
 #pragma unroll
     for (int u = 0; u < kGather - 1; ++u) {
@@ -1841,8 +1854,8 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
     // (ref_cells_adjacent); take the others' terms back out, bit for bit.
     if (entered) {
       for (int k2 = sub; k2 < nn; k2 += G) {
-        const int j = list_entry<FL>(nb + k2);
-        const uint4 o = P.m4[cur][j];
+        const int j = list.entry(k2);
+        const uint4 o = list.pos(j);
         const float dx = frac_delta(me.x, o.x, s0), dy = frac_delta(me.y, o.y, s1), dz = frac_delta(me.z, o.z, s2);
         const float r2 = dist2(dx, dy, dz);
         const float q = dscale(dx, dy, dz);
@@ -1854,7 +1867,7 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
 }
 
 // Plain-form pair sums of the warp's 32 / G beads (bead i on lanes sub = 0 ..
-// G-1; inactive groups take part with an empty list).  The FP64 pipe bounds
+// G-1; inactive groups take part with an empty list, nn = 0).  The FP64 pipe bounds
 // this pass, and about half of a list's entries lie beyond rc.  The lanes
 // therefore first test kPairQueue entries in FP32 on the fractional mirror,
 // with a cut widened by the mirror's resolution and the FP32 rounding, and
@@ -1864,22 +1877,16 @@ __device__ __forceinline__ void pair_sum_q(const DevPtrs& P, int cur, int i, int
 // 18,003-bead vesicle; with the list build in FP32 too, a loop step of it went
 // from 709 to 150 us.
 constexpr int kPairQueue = 128;
-template <int FL, int G>
-__device__ __forceinline__ void pair_sum_d(const DevPtrs& P, int cur, int i, int sub, bool active, const RepState& rs,
-                                           const double* sF, const double* sU, int nT, int* queue, double& fx,
-                                           double& fy, double& fz, double& ep, double& dU) {
+template <int FL, int G, typename List>
+__device__ __forceinline__ void pair_sum_d(const DevPtrs& P, int cur, const List& list, int nn, int i, int sub,
+                                           const RepState& rs, const double* sF, const double* sU, int nT,
+                                           int* queue, double& fx, double& fy, double& fz, double& ep, double& dU) {
   const Tables& T = *P.tab;
   const int lane = threadIdx.x & 31;
   const unsigned int below = (1u << lane) - 1u;
   const unsigned int mine = (0xffffffffu >> (32 - G)) << (lane & ~(G - 1));
-  const int nn = active ? P.nnbr[i] : 0;
-  const int* nb = P.nbr + (size_t)i * P.kmax;
-  double4 me = make_double4(0.0, 0.0, 0.0, 0.0);
-  uint4 mu = make_uint4(0u, 0u, 0u, 0u);
-  if (active) {
-    me = P.d4[cur][i];
-    mu = P.m4[cur][i];
-  }
+  const double4 me = P.d4[cur][i];
+  const uint4 mu = list.pos(i);
   const int ti = __double_as_longlong(me.w) & 0xff;
   const double* rowF = sF + 6 * ti * nT;
   const double* rowU = sU + 6 * ti * nT;
@@ -1905,8 +1912,8 @@ __device__ __forceinline__ void pair_sum_d(const DevPtrs& P, int cur, int i, int
       bool near = false;
       int j = 0;
       if (k < nn) {
-        j = list_entry<FL>(nb + k);
-        const uint4 o = P.m4[cur][j];
+        j = list.entry(k);
+        const uint4 o = list.pos(j);
         const float dx = frac_delta(mu.x, o.x, s0), dy = frac_delta(mu.y, o.y, s1), dz = frac_delta(mu.z, o.z, s2);
         const float r2 = dx * dx + dy * dy + dz * dz;
         near = r2 < cut2;
@@ -1948,17 +1955,18 @@ __device__ __forceinline__ void pair_sum_d(const DevPtrs& P, int cur, int i, int
   }
 }
 
+// (The mixed size-change pass is held to four CTAs per SM.)
 template <bool MIXED, int FL, int G>
-__global__ void __launch_bounds__(kBlock) k_force(DevPtrs P, int cur) {
+__global__ void __launch_bounds__(kBlock, (MIXED && (FL & F_DU) != 0) ? 4 : 0) k_force(DevPtrs P, int cur) {
   pdl_trigger();
   using R = typename std::conditional<MIXED, float, double>::type;
-  __shared__ R sF[6 * kMaxTypes * kMaxTypes];
+  __shared__ __align__(8) R sF[6 * kMaxTypes * kMaxTypes];
   __shared__ R sU[6 * kMaxTypes * kMaxTypes];
   const Tables& T = *P.tab;
   const int nT = T.nT;
   for (int k = threadIdx.x; k < 6 * nT * nT; k += kBlock) {
     if constexpr (MIXED) {
-      sF[k] = T.fF[k];
+      sF[pack_force_row(k)] = T.fF[k];
       sU[k] = T.fU[k];
     } else {
       sF[k] = T.dF[k];
@@ -1977,12 +1985,16 @@ __global__ void __launch_bounds__(kBlock) k_force(DevPtrs P, int cur) {
   if constexpr (MIXED) {
     if (active) {
       float eacc = 0.f;
-      pair_sum_q<FL, G>(P, cur, i, sub, rs, sF, sU, nT, qx, qy, qz, dq, eacc);
+      const BeadList<true> list{P.nbr + (size_t)i * P.kmax, P.m4[cur]};
+      pair_sum_q<FL, G>(P, list, P.nnbr[i], i, sub, rs, sF, sU, nT, qx, qy, qz, dq, eacc);
       ep = 0.5 * (double)eacc;
     }
   } else {
     __shared__ int queue[kBlock / G][kPairQueue];
-    pair_sum_d<FL, G>(P, cur, i, sub, active, rs, sF, sU, nT, queue[threadIdx.x / G], fx, fy, fz, ep, dU);
+    const int ii = active ? i : 0;
+    const BeadList<true> list{P.nbr + (size_t)ii * P.kmax, P.m4[cur]};
+    pair_sum_d<FL, G>(P, cur, list, active ? P.nnbr[i] : 0, ii, sub, rs, sF, sU, nT, queue[threadIdx.x / G], fx, fy,
+                      fz, ep, dU);
   }
   // group reduction (integer sums are exact in any order)
 #pragma unroll

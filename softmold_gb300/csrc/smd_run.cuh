@@ -3,7 +3,7 @@
 // Kernel by kernel, a loop step of a few thousand beads is all latency: two
 // step kernels and, every second step, four list kernels of 5-25 us each that
 // keep at most a tenth of the chip's warps busy (1,176 beads: 35 us per step,
-// 15,000 beads: 41 us; here 17 and 32).  Here every CTA owns a contiguous range of the
+// 15,000 beads: 41 us; here 15 and 25).  Here every CTA owns a contiguous range of the
 // cell-sorted beads and keeps their positions, velocities and bookkeeping in
 // shared memory; only the position mirror goes through global memory.  A step
 // is one grid barrier: each CTA forms its beads' pair sums (and beside them
@@ -24,7 +24,7 @@ namespace smd {
 // threads per CTA at most: 80 registers per thread, or 64 where many beads want more warps
 __host__ __device__ constexpr int run_threads(int lanes) { return lanes == 8 ? 1024 : 768; }
 // Above this a step is throughput, and the separate kernels' occupancy wins
-// (15,000 beads: 32 us per step here, 41 us kernel by kernel).
+// (15,000 beads: 25 us per step here, 41 us kernel by kernel).
 constexpr int kRunMaxBeads = 20000;
 constexpr int kRunCells = 20480;    // largest list-cell grid (its starts are kept in shared memory)
 constexpr int kRunSpinLimit = 1 << 22;  // polls of a barrier: some seconds
@@ -48,14 +48,15 @@ struct RunArgs {
   int rate;       // barostat period
   int barostat;
   int beads;      // beads per CTA
-  int* cnt;       // 2 x n_cells_total cell counts, zero between launches
+  int* cnt;       // 2 x run_cells(n_cells_total) cell counts, zero between launches
   RunSync* sync;
 };
 
 // Shared memory per CTA beyond the static part.
 __host__ __device__ constexpr size_t run_align(size_t b) { return (b + 15) & ~(size_t)15; }
+__host__ __device__ constexpr int run_cells(int cells) { return (cells + 3) & ~3; }
 __host__ __device__ constexpr size_t run_smem(int beads, int cells, bool mixed, int threads, int lanes) {
-  return run_align(sizeof(int) * ((size_t)cells + 1)) + run_align(sizeof(double) * 6 * (size_t)beads) +  // starts, x v
+  return run_align(sizeof(unsigned short) * ((size_t)run_cells(cells) + 1)) + run_align(sizeof(double) * 6 * (size_t)beads) +  // starts, x v
          run_align(sizeof(double) * 3 * (size_t)beads) + run_align(sizeof(double) * 3 * (size_t)beads) +  // sums, bonded
          run_align(sizeof(uint4) * (size_t)beads) + run_align(sizeof(int) * 4 * (size_t)beads) +
          (mixed ? 0 : run_align(sizeof(int) * (size_t)kPairQueue * (threads / lanes)));
@@ -70,88 +71,109 @@ __device__ __forceinline__ double wrap64(double x, double box) {
   return x;
 }
 
-// Appends to the lists of bead a (and of b, in the same cell; b < 0: none) the
-// beads [s, s + len) of the cell order within the list cut.  Distances come
-// from the exact fractional differences, whose wrap is the minimum image, so
-// thin grids need no other path; with five cells on every axis b's follow from
-// a's and the offset between the two (no candidate of the stencil is then near
-// half the box from a and in range of b).  ca, cb: the list lengths in shared
-// memory (several warps append to one bead's list).  One warp.
-template <bool OFFSET>
-__device__ __forceinline__ void run_scan(const uint4* m, int s, int len, const uint4& ma, const uint4& mb, int ia,
-                                         int ib, float x0, float x1, float x2, float lc2, int* oa, int* ob, int* ca,
-                                         int* cb, int kmax) {
+// The stencil of cell (cx, cy, cz) as contiguous bead ranges with prefix sums,
+// formed by one warp: lane l < 18 takes half of row l / 2 (dy, dz), whose
+// cells cx - 1 .. cx + 1 are one range unless it wraps in x; axes with fewer
+// than 3 cells take every cell once.  seg: first beads [0, 18), first slots
+// [18, 37).  Returns the number of slots.
+__device__ __forceinline__ int run_stencil(const RepState& rs, const unsigned short* starts, int cx, int cy, int cz,
+                                           int* seg) {
   const int lane = threadIdx.x & 31;
-  const unsigned int below = (1u << lane) - 1u;
-  float ex = 0.f, ey = 0.f, ez = 0.f;
-  if constexpr (OFFSET) {
-    ex = frac_delta(mb.x, ma.x, x0);
-    ey = frac_delta(mb.y, ma.y, x1);
-    ez = frac_delta(mb.z, ma.z, x2);
-  }
-  uint4 next = m[s + min(lane, len - 1)];
-  for (int k0 = 0; k0 < len; k0 += 32) {
-    const uint4 o = next;
-    const int k = k0 + lane, j = s + k;
-    if (k0 + 32 < len) next = m[s + min(k + 32, len - 1)];
-    const float ax = frac_delta(ma.x, o.x, x0), ay = frac_delta(ma.y, o.y, x1), az = frac_delta(ma.z, o.z, x2);
-    float bx, by, bz;
-    if constexpr (OFFSET) {
-      bx = ax + ex;
-      by = ay + ey;
-      bz = az + ez;
-    } else {
-      bx = frac_delta(mb.x, o.x, x0);
-      by = frac_delta(mb.y, o.y, x1);
-      bz = frac_delta(mb.z, o.z, x2);
+  const int n0 = rs.ncell[0], n1 = rs.ncell[1], n2 = rs.ncell[2];
+  int start = 0, len = 0;
+  if (lane < 18) {
+    const int t = lane >> 1, half = lane & 1, oy = t % 3 - 1, oz = t / 3 - 1;
+    if (!((oy < 0 && n1 < 3) || (oy > 0 && n1 < 2) || (oz < 0 && n2 < 3) || (oz > 0 && n2 < 2))) {
+      int yy = cy + oy, zz = cz + oz;
+      yy += yy < 0 ? n1 : (yy >= n1 ? -n1 : 0);
+      zz += zz < 0 ? n2 : (zz >= n2 ? -n2 : 0);
+      const int row = n0 * (yy + n1 * zz);
+      int u0 = n0 < 3 ? 0 : cx - 1, u1 = n0 < 3 ? n0 - 1 : cx + 1;
+      if (u0 < 0) {
+        u0 = half ? 0 : n0 - 1;
+        u1 = half ? u1 : n0 - 1;
+      } else if (u1 >= n0) {
+        u0 = half ? 0 : u0;
+        u1 = half ? 0 : n0 - 1;
+      } else if (half) {
+        u1 = u0 - 1;
+      }
+      if (u1 >= u0) {
+        start = starts[row + u0];
+        len = starts[row + u1 + 1] - start;
+      }
     }
-    const bool ha = (ax * ax + ay * ay + az * az < lc2) & (j != ia) & (k < len);
-    const bool hb = (bx * bx + by * by + bz * bz < lc2) & (j != ib) & (k < len) & (ib >= 0);
-    const unsigned int va = __ballot_sync(0xffffffffu, ha), vb = __ballot_sync(0xffffffffu, hb);
-    int at = 0;  // lane 0 claims for bead a, lane 1 for bead b
-    if (lane < 2) at = atomicAdd(lane == 0 ? ca : cb, __popc(lane == 0 ? va : vb));
-    const int pa = __shfl_sync(0xffffffffu, at, 0) + __popc(va & below);
-    const int pb = __shfl_sync(0xffffffffu, at, 1) + __popc(vb & below);
-    if (ha && pa < kmax) oa[pa] = j;
-    if (hb && pb < kmax) ob[pb] = j;
   }
+  int incl = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const unsigned int full = __ballot_sync(0xffffffffu, len > 0);
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  __syncwarp();
+  if (len > 0) {
+    const int k = __popc(full & ((1u << lane) - 1u));
+    seg[k] = start;
+    seg[18 + k] = incl - len;
+  }
+  if (lane == 0) seg[18 + __popc(full)] = total;
+  __syncwarp();
+  return total;
 }
 
-// Stencil rows t0 .. t1 - 1 (dy, dz) for bead a and, in the same cell, bead b.
-__device__ __forceinline__ void run_scan_rows(const DevPtrs& P, const uint4* m, const RepState& rs, const int* starts,
-                                              int t0, int t1, int ia, int ib, const uint4& ma, const uint4& mb,
-                                              int* ca, int* cb, float lc2) {
-  const int n0 = rs.ncell[0], n1 = rs.ncell[1], n2 = rs.ncell[2];
-  const int cx = __umulhi(ma.x, (unsigned)n0), cy = __umulhi(ma.y, (unsigned)n1), cz = __umulhi(ma.z, (unsigned)n2);
-  const float x0 = rs.len_per_frac[0], x1 = rs.len_per_frac[1], x2 = rs.len_per_frac[2];
-  const bool offset = n0 >= 5 && n1 >= 5 && n2 >= 5;
-  const int kmax = P.kmax;
-  int* oa = P.nbr + (size_t)ia * kmax;
-  int* ob = P.nbr + (size_t)(ib < 0 ? ia : ib) * kmax;
-  int xa = cx - 1, xb = cx + 1;
-  if (n0 < 3) {
-    xa = 0;
-    xb = n0 - 1;
-  }
-  for (int t = t0; t < t1; ++t) {
-    const int oz = t >= 6 ? 1 : (t >= 3 ? 0 : -1), oy = t - 3 * (oz + 1) - 1;
-    // axes with fewer than 3 cells take every cell once
-    if ((oy < 0 && n1 < 3) || (oy > 0 && n1 < 2) || (oz < 0 && n2 < 3) || (oz > 0 && n2 < 2)) continue;
-    int yy = cy + oy, zz = cz + oz;
-    yy += yy < 0 ? n1 : (yy >= n1 ? -n1 : 0);
-    zz += zz < 0 ? n2 : (zz >= n2 ? -n2 : 0);
-    const int row = n0 * (yy + n1 * zz);
-    // cells xa .. xb, or two ranges where they wrap
-    const bool wraps = xa < 0 || xb >= n0;
-    int s = starts[row + (xa < 0 ? n0 - 1 : xa)], len = starts[row + (wraps ? n0 : xb + 1)] - s;
-    for (int half = 0;; ++half) {
-      if (len > 0) {
-        if (offset) run_scan<true>(m, s, len, ma, mb, ia, ib, x0, x1, x2, lc2, oa, ob, ca, cb, kmax);
-        else run_scan<false>(m, s, len, ma, mb, ia, ib, x0, x1, x2, lc2, oa, ob, ca, cb, kmax);
+// Lists of bead a and (PAIR) of b in the same cell from the stencil's M slots,
+// by one warp.  Distances come from the exact fractional differences, whose
+// wrap is the minimum image, so thin grids need no other path; with OFFSET
+// (five cells on every axis) b's follow from a's and the offset between the
+// two: no candidate of the stencil is then near half the box from a and in
+// range of b.
+template <bool PAIR, bool OFFSET>
+__device__ __forceinline__ void run_scan(const uint4* m, const int* seg, int M, uint4 ma, uint4 mb, int ia, float x0,
+                                         float x1, float x2, float lc2, int* oa, int kmax, int& ca, int& cb) {
+  const int lane = threadIdx.x & 31;
+  const unsigned int below = (1u << lane) - 1u;
+  const float ex = frac_delta(mb.x, ma.x, x0), ey = frac_delta(mb.y, ma.y, x1), ez = frac_delta(mb.z, ma.z, x2);
+  int* ob = oa + kmax;
+  int t = 0;  // segment of this lane's next slot (slots only increase)
+  auto slot_bead = [&](int g) {
+    while (seg[18 + t + 1] <= g) ++t;
+    return seg[t] + (g - seg[18 + t]);
+  };
+  ca = cb = 0;
+  int j = slot_bead(min(lane, M - 1));
+  uint4 o = m[j];
+  for (int k0 = 0; k0 < M; k0 += 32) {
+    const int jc = j;
+    const uint4 c = o;
+    const bool on = k0 + lane < M;
+    if (k0 + 32 < M) {  // the next round's candidate, a round ahead
+      j = slot_bead(min(k0 + 32 + lane, M - 1));
+      o = m[j];
+    }
+    const float ax = frac_delta(ma.x, c.x, x0), ay = frac_delta(ma.y, c.y, x1), az = frac_delta(ma.z, c.z, x2);
+    const bool ha = on & (jc != ia) & (ax * ax + ay * ay + az * az < lc2);
+    const unsigned int va = __ballot_sync(0xffffffffu, ha);
+    const int pa = ca + __popc(va & below);
+    if (ha && pa < kmax) oa[pa] = jc;
+    ca += __popc(va);
+    if constexpr (PAIR) {
+      float bx, by, bz;
+      if constexpr (OFFSET) {
+        bx = ax + ex;
+        by = ay + ey;
+        bz = az + ez;
+      } else {
+        bx = frac_delta(mb.x, c.x, x0);
+        by = frac_delta(mb.y, c.y, x1);
+        bz = frac_delta(mb.z, c.z, x2);
       }
-      if (!wraps || half) break;
-      s = starts[row];
-      len = starts[row + (xa < 0 ? xb + 1 : 1)] - s;
+      const bool hb = on & (jc != ia + 1) & (bx * bx + by * by + bz * bz < lc2);
+      const unsigned int vb = __ballot_sync(0xffffffffu, hb);
+      const int pb = cb + __popc(vb & below);
+      if (hb && pb < kmax) ob[pb] = jc;
+      cb += __popc(vb);
     }
   }
 }
@@ -162,8 +184,9 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
   using Sum = typename std::conditional<MIXED, long long, double>::type;
   extern __shared__ uint4 run_dyn[];
   __shared__ RepState rs;
-  __shared__ R sF[6 * kMaxTypes * kMaxTypes], sU[6 * kMaxTypes * kMaxTypes];
+  __shared__ __align__(8) R sF[6 * kMaxTypes * kMaxTypes], sU[6 * kMaxTypes * kMaxTypes];
   __shared__ int wsum[run_threads(G) / 32];
+  __shared__ int segs[run_threads(G) / 32][38];
   __shared__ float smax[run_threads(G) / 32];
   __shared__ long long sdq[2];
   __shared__ double sdu[2];
@@ -172,11 +195,12 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
   __shared__ unsigned long long seen;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
   const int b0 = blockIdx.x * A.beads, nb = min(A.beads, P.n - b0);
-  const int ncell = P.n_cells_total;
+  const int ncell = P.n_cells_total, ncell4 = run_cells(ncell);
   // dynamic shared memory (run_smem)
   unsigned char* at = reinterpret_cast<unsigned char*>(run_dyn);
-  int* starts = reinterpret_cast<int*>(at);
-  at += run_align(sizeof(int) * ((size_t)ncell + 1));
+  static_assert(kRunMaxBeads < 65536, "16-bit cell starts");
+  unsigned short* starts = reinterpret_cast<unsigned short*>(at);
+  at += run_align(sizeof(unsigned short) * ((size_t)ncell4 + 1));
   double* st = reinterpret_cast<double*>(at);  // x, y, z, vx, vy, vz of the CTA's beads
   at += run_align(sizeof(double) * 6 * (size_t)A.beads);
   Sum* fsum = reinterpret_cast<Sum*>(at);
@@ -201,7 +225,7 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
     reinterpret_cast<int*>(&rs)[k] = reinterpret_cast<const int*>(P.rs)[k];
   for (int k = tid; k < 6 * nT * nT; k += nt) {
     if constexpr (MIXED) {
-      sF[k] = T.fF[k];
+      sF[pack_force_row(k)] = T.fF[k];
       sU[k] = T.fU[k];
     } else {
       sF[k] = T.dF[k];
@@ -258,19 +282,12 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
     __syncthreads();
     return abort_s == 0;
   };
-  auto trial_at = [&](long long step) { return A.barostat && step % A.rate == 0 && step != 0; };
+  int phase = (int)(((it % A.rate) + A.rate) % A.rate);  // of the barostat period
   // list cell of own bead t on the current grid
   auto cell_of = [&](const uint4& m) {
     const int n0 = rs.ncell[0], n1 = rs.ncell[1], n2 = rs.ncell[2];
     return (int)__umulhi(m.x, (unsigned)n0) +
            n0 * ((int)__umulhi(m.y, (unsigned)n1) + n1 * (int)__umulhi(m.z, (unsigned)n2));
-  };
-  // counts own bead t's cell (every lane of the warp calls it)
-  auto count_cell = [&](bool on, int c, int* counts) {
-    const unsigned int lanes = __ballot_sync(0xffffffffu, on);
-    if (!on) return;
-    const unsigned int same = __match_any_sync(lanes, c);
-    if (lane == __ffs(same) - 1) atomicAdd(&counts[c], __popc(same));
   };
   // own bead t's cell on the reference's grid (the size-change passes)
   auto ref_key = [&](const double x[3]) {
@@ -281,18 +298,38 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
     return k;
   };
   // the trial of a barostat step: every CTA draws it into its own copy
+  // exclusive sum of v over the block's threads, and the total (scratch: 32
+  // words; the caller synchronises before it is used again)
+  auto block_scan = [&](int v, int* scratch, int& total) {
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) scratch[warp] = x;
+    __syncthreads();
+    int t = lane < nw ? scratch[lane] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += y;
+    }
+    total = __shfl_sync(0xffffffffu, t, 31);
+    const int before = __shfl_sync(0xffffffffu, t, warp > 0 ? warp - 1 : 0);
+    return (warp > 0 ? before : 0) + x - v;
+  };
   auto draw = [&]() {
     if (tid == 0) draw_trial(rs, rp, P.trial_u[(size_t)slot * 2]);
   };
-  bool trial = trial_at(it);
+  bool trial = A.barostat && phase == 0 && it != 0;
   {
     const bool stale = rebuild != 0;
     if (trial) draw();
-    if (stale && tid < ((nb + 31) & ~31)) {
-      const bool on = tid < nb;
-      const int c = on ? cell_of(P.m4[cur][b0 + tid]) : 0;
-      if (on) key[tid] = c;
-      count_cell(on, c, A.cnt + ncell);
+    if (stale && tid < nb) {
+      const int c = cell_of(P.m4[cur][b0 + tid]);
+      key[tid] = c;
+      atomicAdd(A.cnt + ncell4 + c, 1);
     }
     if (trial && !stale && tid < nb) {
       const double x[3] = {st[tid], st[NB + tid], st[2 * NB + tid]};
@@ -306,74 +343,61 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
     const bool last = s + 1 == A.steps;
     if (rebuild) {
       // ---- exclusive scan of the cell counts, by every CTA for itself
-      const int* counts = A.cnt + (size_t)((s + 1) & 1) * ncell;
       {
-        constexpr int kBatch = 4;
-        int most = 0;
-        for (int c = tid; c < ncell; c += kBatch * nt) {  // loads issued together
-          int v[kBatch];
+        const int4* counts = reinterpret_cast<const int4*>(A.cnt + (size_t)((s + 1) & 1) * ncell4);
+        constexpr int kQuads = 4;  // 16 consecutive counts per thread and pass, loaded together
+        int carry = 0, most = 0;
+        for (int q0 = 0; q0 < ncell4 / 4; q0 += kQuads * nt) {
+          int4 v[kQuads];
+          int sum = 0;
 #pragma unroll
-          for (int u = 0; u < kBatch; ++u) v[u] = c + u * nt < ncell ? __ldcg(counts + c + u * nt) : 0;
+          for (int u = 0; u < kQuads; ++u) {
+            const int q = q0 + kQuads * tid + u;
+            v[u] = q < ncell4 / 4 ? __ldcg(counts + q) : make_int4(0, 0, 0, 0);
+          }
 #pragma unroll
-          for (int u = 0; u < kBatch; ++u)
-            if (c + u * nt < ncell) {
-              starts[c + u * nt] = v[u];
-              most = max(most, v[u]);
-            }
+          for (int u = 0; u < kQuads; ++u) {
+            sum += v[u].x + v[u].y + v[u].z + v[u].w;
+            most = max(max(most, max(v[u].x, v[u].y)), max(v[u].z, v[u].w));
+          }
+          int total;
+          int ex = carry + block_scan(sum, wsum, total);
+#pragma unroll
+          for (int u = 0; u < kQuads; ++u) {
+            const int q = q0 + kQuads * tid + u;
+            ushort4 f;
+            f.x = (unsigned short)ex;
+            f.y = (unsigned short)(ex += v[u].x);
+            f.z = (unsigned short)(ex += v[u].y);
+            f.w = (unsigned short)(ex += v[u].z);
+            ex += v[u].w;
+            if (q < ncell4 / 4) reinterpret_cast<ushort4*>(starts)[q] = f;
+          }
+          carry += total;
+          __syncthreads();  // wsum is used again
         }
         if (most > kNbrMaxCell) atomicOr(&P.g->error, 2);
-        __syncthreads();
-        // each thread sums an odd number of consecutive counts (no bank conflicts)
-        const int per = ((ncell + nt - 1) / nt) | 1, c0 = min(tid * per, ncell), c1 = min(c0 + per, ncell);
-        int sum = 0;
-        for (int c = c0; c < c1; ++c) sum += starts[c];
-        int x = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, x, o);
-          if (lane >= o) x += y;
-        }
-        if (lane == 31) wsum[warp] = x;
-        __syncthreads();
-        int before = 0;
-        for (int w = 0; w < warp; ++w) before += wsum[w];
-        int ex = before + x - sum;
-        for (int c = c0; c < c1; ++c) {
-          const int v = starts[c];
-          starts[c] = ex;
-          ex += v;
-        }
-        if (tid == nt - 1) starts[ncell] = P.n;
+        if (tid == 0) starts[ncell4] = (unsigned short)P.n;
       }
       __syncthreads();
       // ---- scatter to the new order (cell_count: the cells' fill)
-      if (tid < ((nb + 31) & ~31)) {
-        const bool on = tid < nb;
-        const unsigned int lanes = __ballot_sync(0xffffffffu, on);
-        if (on) {
-          const int c = key[tid];
-          const unsigned int same = __match_any_sync(lanes, c);
-          const int leader = __ffs(same) - 1;
-          int base = 0;
-          if (lane == leader) base = atomicAdd(&P.cell_count[c], __popc(same));
-          base = __shfl_sync(same, base, leader);
-          const int nw_i = starts[c] + base + __popc(same & ((1u << lane) - 1u));
-          P.tx[nw_i] = st[tid];
-          P.ty[nw_i] = st[NB + tid];
-          P.tz[nw_i] = st[2 * NB + tid];
-          P.tvx[nw_i] = st[3 * NB + tid];
-          P.tvy[nw_i] = st[4 * NB + tid];
-          P.tvz[nw_i] = st[5 * NB + tid];
-          const int o = orig[tid];
-          P.torig[nw_i] = o;
-          P.tcinfo[nw_i] = cinfo[tid];
-          P.inv[o] = nw_i;
-          P.m4[cur ^ 1][nw_i] = P.m4[cur][b0 + tid];
-          if constexpr (!MIXED) P.d4[cur ^ 1][nw_i] = P.d4[cur][b0 + tid];
-          if (trial) {
-            const double x[3] = {st[tid], st[NB + tid], st[2 * NB + tid]};
-            P.refcell[nw_i] = ref_key(x);
-          }
+      if (tid < nb) {
+        const int c = key[tid], nw_i = starts[c] + atomicAdd(&P.cell_count[c], 1);
+        P.tx[nw_i] = st[tid];
+        P.ty[nw_i] = st[NB + tid];
+        P.tz[nw_i] = st[2 * NB + tid];
+        P.tvx[nw_i] = st[3 * NB + tid];
+        P.tvy[nw_i] = st[4 * NB + tid];
+        P.tvz[nw_i] = st[5 * NB + tid];
+        const int o = orig[tid];
+        P.torig[nw_i] = o;
+        P.tcinfo[nw_i] = cinfo[tid];
+        P.inv[o] = nw_i;
+        P.m4[cur ^ 1][nw_i] = P.m4[cur][b0 + tid];
+        if constexpr (!MIXED) P.d4[cur ^ 1][nw_i] = P.d4[cur][b0 + tid];
+        if (trial) {
+          const double x[3] = {st[tid], st[NB + tid], st[2 * NB + tid]};
+          P.refcell[nw_i] = ref_key(x);
         }
       }
       if (!barrier(1)) return;
@@ -391,34 +415,48 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
         P.orig[i] = o;
         cinfo[tid] = __ldcg(P.tcinfo + i);
         ref[tid] = P.m4[cur][i];
-        cnt[tid] = 0;
       }
       if (tid == 0) {
         slack = 0.0;
         if (blockIdx.x == 0) P.g->n_rebuilds++;
       }
       __syncthreads();
-      // ---- lists: a row of the stencil for two neighbouring beads per warp
+      // ---- lists: a warp takes two neighbouring beads at a time, or one where that leaves warps idle
+      if (tid < nb) key[tid] = cell_of(ref[tid]);
+      __syncthreads();
       {
         const float lcut = MIXED ? T.list_cut_f + 1e-4f
                                  : T.list_cut_f * (1.f + 4e-6f) + 1e-4f +
                                        4.f * fmaxf(rs.len_per_frac[0], fmaxf(rs.len_per_frac[1], rs.len_per_frac[2]));
         const float lc2 = lcut * lcut;
+        const float x0 = rs.len_per_frac[0], x1 = rs.len_per_frac[1], x2 = rs.len_per_frac[2];
+        const bool offset = rs.ncell[0] >= 5 && rs.ncell[1] >= 5 && rs.ncell[2] >= 5;
         const uint4* m = P.m4[cur];
-        // tasks: two neighbouring beads by three stencil rows, or by one where
-        // that leaves warps idle
-        const int pairs = (nb + 1) >> 1, rows = pairs * 3 >= nw ? 3 : 1, parts = 9 / rows;
-        for (int task = warp; task < pairs * parts; task += nw) {
-          const int p = rows == 3 ? task / 3 : task / 9, t0 = (task - p * parts) * rows;
-          const int a = 2 * p, b = a + 1 < nb ? a + 1 : a;
-          const uint4 ma = ref[a], mb = ref[b];
-          const int i = b0 + a;
-          if (b != a && cell_of(ma) == cell_of(mb)) {
-            run_scan_rows(P, m, rs, starts, t0, t0 + rows, i, i + 1, ma, mb, cnt + a, cnt + b, lc2);
-          } else {
-            for (int q = a; q <= b; ++q)
-              run_scan_rows(P, m, rs, starts, t0, t0 + rows, b0 + q, -1, ref[q], ref[q], cnt + q, cnt + q, lc2);
+        const int kmax = P.kmax;
+        int* seg = segs[warp];
+        const int each = nb > nw ? 2 * ((nb + 2 * nw - 1) / (2 * nw)) : 1, end = min((warp + 1) * each, nb);
+        int last_cell = -1, M = 0;
+        for (int q = warp * each; q < end;) {
+          const uint4 ma = ref[q];
+          const int c = key[q];
+          if (c != last_cell) {  // neighbouring beads mostly share it
+            const int n0 = rs.ncell[0], n1 = rs.ncell[1], row = c / n0;
+            M = run_stencil(rs, starts, c - row * n0, row % n1, row / n1, seg);
+            last_cell = c;
           }
+          const bool pair = q + 1 < end && key[q + 1] == c;
+          const uint4 mb = ref[pair ? q + 1 : q];
+          const int i = b0 + q;
+          int* out = P.nbr + (size_t)i * kmax;
+          int ca, cb;
+          if (pair && offset) run_scan<true, true>(m, seg, M, ma, mb, i, x0, x1, x2, lc2, out, kmax, ca, cb);
+          else if (pair) run_scan<true, false>(m, seg, M, ma, mb, i, x0, x1, x2, lc2, out, kmax, ca, cb);
+          else run_scan<false, false>(m, seg, M, ma, mb, i, x0, x1, x2, lc2, out, kmax, ca, cb);
+          if (lane == 0) {
+            cnt[q] = ca;
+            if (pair) cnt[q + 1] = cb;
+          }
+          q += pair ? 2 : 1;
         }
       }
       __syncthreads();
@@ -435,7 +473,7 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
       __syncthreads();
     }
     // the counts of the step before this one: read above at the latest
-    for (int c = blockIdx.x * nt + tid; c < ncell; c += gridDim.x * nt) A.cnt[(size_t)((s + 1) & 1) * ncell + c] = 0;
+    for (int c = blockIdx.x * nt + tid; c < ncell; c += gridDim.x * nt) A.cnt[(size_t)((s + 1) & 1) * ncell4 + c] = 0;
     if (tid == 0) {
       sdq[0] = sdq[1] = 0;
       sdu[0] = sdu[1] = 0.0;
@@ -485,10 +523,10 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
           long long qx = 0, qy = 0, qz = 0, dq = 0;
           float unused = 0.f;
           if (active) {
-            if (trial)
-              pair_sum_q<F_DU | F_RUN, G>(P, cur, i, sub, rs, sF, sU, nT, qx, qy, qz, dq, unused);
-            else
-              pair_sum_q<F_RUN, G>(P, cur, i, sub, rs, sF, sU, nT, qx, qy, qz, dq, unused);
+            const BeadList<false> list{P.nbr + (size_t)i * P.kmax, P.m4[cur]};
+            const int nn = P.nnbr[i];
+            if (trial) pair_sum_q<F_DU, G>(P, list, nn, i, sub, rs, sF, sU, nT, qx, qy, qz, dq, unused);
+            else pair_sum_q<0, G>(P, list, nn, i, sub, rs, sF, sU, nT, qx, qy, qz, dq, unused);
           }
 #pragma unroll
           for (int o = G / 2; o > 0; o >>= 1) {
@@ -509,10 +547,10 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
         } else {
           double fx = 0, fy = 0, fz = 0, ep = 0, dU = 0;
           int* q = queue + (size_t)(tid / G) * kPairQueue;
-          if (trial)
-            pair_sum_d<F_DU | F_RUN, G>(P, cur, i, sub, active, rs, sF, sU, nT, q, fx, fy, fz, ep, dU);
-          else
-            pair_sum_d<F_RUN, G>(P, cur, i, sub, active, rs, sF, sU, nT, q, fx, fy, fz, ep, dU);
+          const BeadList<false> list{P.nbr + (size_t)i * P.kmax, P.m4[cur]};
+          const int nn = active ? P.nnbr[i] : 0;
+          if (trial) pair_sum_d<F_DU, G>(P, cur, list, nn, i, sub, rs, sF, sU, nT, q, fx, fy, fz, ep, dU);
+          else pair_sum_d<0, G>(P, cur, list, nn, i, sub, rs, sF, sU, nT, q, fx, fy, fz, ep, dU);
 #pragma unroll
           for (int o = G / 2; o > 0; o >>= 1) {
             fx += __shfl_xor_sync(0xffffffffu, fx, o);
@@ -538,7 +576,7 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
     int ti = 0;
     unsigned int w = 0;
     if (tid < nb) {
-      w = P.m4[cur][b0 + tid].w;
+      w = ref[tid].w;
       ti = w & 0xff;
       for (int d = 0; d < 3; ++d) {
         x[d] = st[d * NB + tid];
@@ -592,9 +630,9 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
       ++trials;
     }
     // ---- first half-kick and drift of the next step, its mirror and cell count
-    const bool next_trial = trial_at(it + 1);
+    phase = phase + 1 == A.rate ? 0 : phase + 1;
+    const bool next_trial = A.barostat && phase == 0 && it + 1 != 0;
     float vmax = 0.f;
-    int c = 0;
     if (tid < nb) {
       const int i = b0 + tid;
       if (scaled)
@@ -611,22 +649,21 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
                                   to_frac(x[2], rs.frac_per_len[2]), w);
       vmax = displacement(ref[tid], mn.x, mn.y, mn.z, rs);
       P.m4[cur ^ 1][i] = mn;
-      if constexpr (!MIXED) P.d4[cur ^ 1][i] = make_double4(x[0], x[1], x[2], P.d4[cur][i].w);
-      c = cell_of(mn);
+      if constexpr (!MIXED) P.d4[cur ^ 1][i] = make_double4(x[0], x[1], x[2], __longlong_as_double((long long)w));
+      const int c = cell_of(mn);
       key[tid] = c;
+      if (!last) atomicAdd(A.cnt + (size_t)(s & 1) * ncell4 + c, 1);
       if (next_trial && !last) P.refcell[i] = ref_key(x);
     }
-    if (!last && tid < ((nb + 31) & ~31)) count_cell(tid < nb, c, A.cnt + (size_t)(s & 1) * ncell);
     vmax = warp_max(vmax);
     if (lane == 0) smax[warp] = vmax;
     __syncthreads();
     // ---- arrive: a bead beyond the margin (half the skin less the slack) asks for a rebuild
     unsigned long long inc = 1;
-    if (tid == 0) {
-      float bm = 0.f;
-      for (int k = 0; k < nw; ++k) bm = fmaxf(bm, smax[k]);
+    if (warp == 0) {
+      const float bm = warp_max(lane < nw ? smax[lane] : 0.f);
       if ((double)bm + slack > P.half_skin) inc += 1ull << (40 + 8 * (s % 3));
-      if (last && bm > 0.f) atomicMax(&P.g->dmax_bits, __float_as_uint(bm));
+      if (last && lane == 0 && bm > 0.f) atomicMax(&P.g->dmax_bits, __float_as_uint(bm));
       // CTA 0 clears the field of two steps ago (the next step's), which every CTA has read
       if (blockIdx.x == 0 && s >= 2) inc -= ((seen >> (40 + 8 * ((s + 1) % 3))) & 0xffull) << (40 + 8 * ((s + 1) % 3));
     }
