@@ -19,34 +19,120 @@
 // constants 1 and 3 (include/MD.h:384-431, 683-789), so their derivatives
 // are the same kernels evaluated with derivative rows or unit constants.
 //
-// MIXED: pair terms in FP32 from the exact fractional mirror, every sum and
-// the adjoint state in FP64.  PLAIN: FP64 throughout.  The CHAIN terms are
-// FP64 in both, their K w from forward-mode dual numbers through the force
-// formulas.
+// MIXED: pair terms in FP32 from the exact fractional mirror, summed as pairs
+// of FP32 (TwoSum), the adjoint state in FP64.  PLAIN: FP64 throughout.  The
+// CHAIN terms are FP64 in both, their K w the directional derivative of the
+// force formulas, written out.
 #pragma once
 
 #include "smd_kernels.cuh"
 
 namespace smd {
 
-// ------------------------------------------------------------ dual numbers
-struct Dd {  // value and directional derivative
-  double v, t;
+// A sum of FP32 terms held as an unevaluated pair hi + lo (Knuth's TwoSum: the
+// rounding error of each addition, exact, is added to lo).  Its error, some
+// 2^-45 of the terms' magnitude, is far below the terms' own FP32 rounding, and
+// its seven FP32 instructions cost a tenth of an FP64 conversion and addition.
+struct Sum2 {
+  float hi = 0.f, lo = 0.f;
+  __device__ __forceinline__ void add(float x) {
+    const float s = __fadd_rn(hi, x);
+    const float b = __fsub_rn(s, hi);
+    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
+    hi = s;
+  }
+  __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
-__device__ __forceinline__ Dd operator+(Dd a, Dd b) { return {a.v + b.v, a.t + b.t}; }
-__device__ __forceinline__ Dd operator-(Dd a, Dd b) { return {a.v - b.v, a.t - b.t}; }
-__device__ __forceinline__ Dd operator-(Dd a) { return {-a.v, -a.t}; }
-__device__ __forceinline__ Dd operator*(Dd a, Dd b) { return {a.v * b.v, a.t * b.v + a.v * b.t}; }
-__device__ __forceinline__ Dd operator/(Dd a, Dd b) {
-  const double q = a.v / b.v;
-  return {q, (a.t - q * b.t) / b.v};
+struct Sum1 {  // the plain form's sums
+  double v = 0.0;
+  __device__ __forceinline__ void add(double x) { v += x; }
+  __device__ __forceinline__ double value() const { return v; }
+};
+
+// CHAIN terms of one bead in FP64, with unit force constants (the forces are
+// linear in them): bonds and bends summed apart, each with its directional
+// derivative along the beads' w, and the energies the bead owns.  For a bond
+// d with tangent t, r = |d|:
+//   f = -(1 - l/r) d,   f' = -(1 - l/r) t - (l/r^3)(d . t) d;
+// for a bend of unit vectors a, b (lengths p, q), c = a . b, m = c0 - c:
+//   g1 = (m/p)(b - a c) on the first bead, g2 = (m/q)(a - b c) off the third,
+//   the second taking g2 - g1, with a' = (t_a - a (a . t_a)) / p and so on.
+// One reciprocal root per vector serves everything: the same terms by dual
+// numbers through sqrt and divisions took 1,280 FP64 instructions per warp and
+// 95 us at 15,000 beads, these 260 and 24 us.
+struct ChainDual {
+  double fb[3] = {0, 0, 0}, tb[3] = {0, 0, 0};  // bonds: force, derivative
+  double fn[3] = {0, 0, 0}, tn[3] = {0, 0, 0};  // bends
+  double ub = 0.0, un = 0.0;                    // energies
+};
+__device__ __forceinline__ double dot3(const double a[3], const double b[3]) {
+  return fma(a[2], b[2], fma(a[1], b[1], a[0] * b[0]));
 }
-__device__ __forceinline__ Dd& operator+=(Dd& a, Dd b) { return a = a + b; }
-__device__ __forceinline__ Dd& operator-=(Dd& a, Dd b) { return a = a - b; }
-__device__ __forceinline__ Dd& operator/=(Dd& a, Dd b) { return a = a / b; }
-__device__ __forceinline__ Dd sqrt(Dd a) {
-  const double s = ::sqrt(a.v);
-  return {s, a.t / (2.0 * s)};
+// e[k] = x(p-2+k) - x(p-1+k) and t[k] the same difference of w, k = 0 .. 3.
+// sums: 1 with the forces themselves and energies, 0 derivatives only.
+template <bool SUMS>
+__device__ __forceinline__ void chain_dual(const Vec3<double> e[4], const double t[4][3], const bool valid[4],
+                                           const double* cd, ChainDual& c) {
+  double u[4][3], ri[4];  // unit vectors and reciprocal lengths
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    u[k][0] = u[k][1] = u[k][2] = ri[k] = 0.0;
+    if (!valid[k]) continue;
+    const double d[3] = {e[k].x, e[k].y, e[k].z};
+    const double r2 = dot3(d, d);
+    ri[k] = rsqrt(r2);
+    for (int a = 0; a < 3; ++a) u[k][a] = d[a] * ri[k];
+    if (k == 1 || k == 2) {  // bonds (p-1, p) as second, (p, p+1) as first
+      const double sg = k == 1 ? -1.0 : 1.0;
+      const double l = cd[0], lr = l * ri[k], A = sg * (lr - 1.0);
+      const double B = sg * lr * dot3(u[k], t[k]);  // (l/r)(u . t)
+      for (int a = 0; a < 3; ++a) {
+        if constexpr (SUMS) c.fb[a] = fma(A, d[a], c.fb[a]);
+        c.tb[a] += fma(A, t[k][a], -B * u[k][a]);
+      }
+      if constexpr (SUMS) {
+        if (k == 2) {
+          const double x = fma(r2, ri[k], -l);
+          c.ub = 0.5 * x * x;
+        }
+      }
+    }
+  }
+  // bends (e[k], e[k+1]): the bead is the third, second, first for k = 0, 1, 2;
+  // one turn per bend the bead has (one for three-bead chains, whichever it is)
+  unsigned int todo = (valid[0] && valid[1] ? 1u : 0u) | (valid[1] && valid[2] ? 2u : 0u) | (valid[2] && valid[3] ? 4u : 0u);
+  while (todo) {
+    const int k = __ffs(todo) - 1;
+    todo &= todo - 1;
+    double a[3], b[3], ta[3], tb[3];
+    for (int x = 0; x < 3; ++x) {
+      a[x] = k == 0 ? u[0][x] : (k == 1 ? u[1][x] : u[2][x]);
+      b[x] = k == 0 ? u[1][x] : (k == 1 ? u[2][x] : u[3][x]);
+      ta[x] = k == 0 ? t[0][x] : (k == 1 ? t[1][x] : t[2][x]);
+      tb[x] = k == 0 ? t[1][x] : (k == 1 ? t[2][x] : t[3][x]);
+    }
+    const double ia = k == 0 ? ri[0] : (k == 1 ? ri[1] : ri[2]), ib = k == 0 ? ri[1] : (k == 1 ? ri[2] : ri[3]);
+    const double cs = dot3(a, b), m = cd[2] - cs;
+    const double pa = dot3(a, ta), pb = dot3(b, tb);  // rates of the lengths
+    double da[3], db[3];
+    for (int x = 0; x < 3; ++x) {
+      da[x] = fma(-a[x], pa, ta[x]) * ia;
+      db[x] = fma(-b[x], pb, tb[x]) * ib;
+    }
+    const double dc = dot3(da, b) + dot3(a, db);
+    const double ma = m * ia, mb = m * ib;
+    const double na = fma(-ma, pa, -dc) * ia, nb = fma(-mb, pb, -dc) * ib;  // rates of m/p, m/q
+    const double s1 = k == 0 ? 0.0 : (k == 1 ? -1.0 : 1.0), s2 = k == 0 ? -1.0 : (k == 1 ? 1.0 : 0.0);
+    for (int x = 0; x < 3; ++x) {
+      const double va = fma(-a[x], cs, b[x]), vb = fma(-b[x], cs, a[x]);
+      const double wa = fma(-a[x], dc, fma(-da[x], cs, db[x])), wb = fma(-b[x], dc, fma(-db[x], cs, da[x]));
+      if constexpr (SUMS) c.fn[x] = fma(s1 * ma, va, fma(s2 * mb, vb, c.fn[x]));
+      c.tn[x] = fma(s1, fma(ma, wa, na * va), fma(s2, fma(mb, wb, nb * vb), c.tn[x]));
+    }
+    if constexpr (SUMS) {
+      if (k == 2) c.un = 0.5 * m * m;
+    }
+  }
 }
 
 // Device accumulators of one adjoint run.
@@ -118,7 +204,8 @@ __global__ void __launch_bounds__(kBlock) k_adj_wsort(DevPtrs P, const double* w
 
 // Pair part of step n: for bead i the non-bonded force F_i, (K w)_i, and the
 // replica sums of U, dU/dUmin and w_i . dF_i/dUmin.  G lanes per bead walk
-// the Verlet list as k_force does; every sum is FP64.
+// the Verlet list as k_force does.  The mixed form's sums are Sum2: 39 us per
+// pass at 15,000 beads against 92 with each term converted and added in FP64.
 template <bool MIXED, int G>
 __global__ void __launch_bounds__(kBlock) k_adj_pair(DevPtrs P, int cur, const AdjTables* AT,
                                                      const typename std::conditional<MIXED, float4, double4>::type* ws,
@@ -128,7 +215,8 @@ __global__ void __launch_bounds__(kBlock) k_adj_pair(DevPtrs P, int cur, const A
   const int t = blockIdx.x * kBlock + threadIdx.x;
   const int i = t / G, sub = t % G;
   const bool active = i < P.n;
-  double F[3] = {0, 0, 0}, K[3] = {0, 0, 0}, u = 0, ut = 0, wft = 0;
+  using Sum = typename std::conditional<MIXED, Sum2, Sum1>::type;
+  Sum sF[3], sK[3], su, sut, swft;
   if (active) {
     const RepState& rs = P.rs[rep_of(P, i)];
     const int nn = P.nnbr[i];
@@ -199,21 +287,26 @@ __global__ void __launch_bounds__(kBlock) k_adj_pair(DevPtrs P, int cur, const A
       const auto wj = ws[j];
       const R ex = (R)wi.x - (R)wj.x, ey = (R)wi.y - (R)wj.y, ez = (R)wi.z - (R)wj.z;
       const R dd = q * (dx * ex + dy * ey + dz * ez);
-      F[0] += (double)(g * dx);
-      F[1] += (double)(g * dy);
-      F[2] += (double)(g * dz);
-      K[0] += (double)(g * ex + dd * dx);
-      K[1] += (double)(g * ey + dd * dy);
-      K[2] += (double)(g * ez + dd * dz);
-      u += 0.5 * (double)pair_pot<R>(rowU + 6 * tj, rr);
+      sF[0].add(g * dx);
+      sF[1].add(g * dy);
+      sF[2].add(g * dz);
+      sK[0].add(g * ex + dd * dx);
+      sK[1].add(g * ey + dd * dy);
+      sK[2].add(g * ez + dd * dz);
+      su.add((R)0.5 * pair_pot<R>(rowU + 6 * tj, rr));
       const R* ct = rowFt + 6 * tj;
       if (ct[1] != (R)0 || ct[4] != (R)0) {
         const R mt = ct[ci] - rr;
         const R gt = ((ct[ci + 1] - ct[ci + 2] * mt) * mt) / rr;
-        wft += (double)(gt * (dx * (R)wi.x + dy * (R)wi.y + dz * (R)wi.z));
-        ut += 0.5 * (double)pair_pot<R>(rowUt + 6 * tj, rr);
+        swft.add(gt * (dx * (R)wi.x + dy * (R)wi.y + dz * (R)wi.z));
+        sut.add((R)0.5 * pair_pot<R>(rowUt + 6 * tj, rr));
       }
     }
+  }
+  double F[3], K[3];
+  for (int d = 0; d < 3; ++d) {
+    F[d] = sF[d].value();
+    K[d] = sK[d].value();
   }
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) {
@@ -229,12 +322,20 @@ __global__ void __launch_bounds__(kBlock) k_adj_pair(DevPtrs P, int cur, const A
     }
   }
   // replica sums (single-system handles): J and the Umin component
-  const double gJ = invT * u, g0 = dt * wft + invT * ut;
+  const double gJ = invT * su.value(), g0 = dt * swft.value() + invT * sut.value();
   const double sJ = warp_sum(gJ), s0 = warp_sum(g0);
   if ((threadIdx.x & 31) == 0) {
     if (sJ != 0.0) atomicAdd(&acc->J, sJ);
     if (s0 != 0.0) atomicAdd(&acc->grad[0], s0);
   }
+}
+
+// Differences of w along the chain of file-order bead o (file order is chain
+// order), 0 where a vector does not exist.
+__device__ __forceinline__ void chain_tangents(const double* w, int o, const bool valid[4], double t[4][3]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    for (int d = 0; d < 3; ++d) t[k][d] = valid[k] ? w[3 * (o - 2 + k) + d] - w[3 * (o - 1 + k) + d] : 0.0;
 }
 
 // CHAIN part of step n and the adjoint update of every bead (file order):
@@ -264,45 +365,18 @@ __global__ void __launch_bounds__(kBlock) k_adj_chain(DevPtrs P, int cur, const 
       Vec3<double> e[4];
       bool valid[4];
       chain_vectors<MIXED, double>(P, cur, i, p, len, box, rs, e, valid);
-      // tangents: differences of w along the chain (file order is chain order)
-      Vec3<Dd> ed[4];
-      for (int k = 0; k < 4; ++k) {
-        const int a = o - 2 + k, b = o - 1 + k;
-        double t[3] = {0, 0, 0};
-        if (valid[k])
-          for (int d = 0; d < 3; ++d) t[d] = w[3 * a + d] - w[3 * b + d];
-        ed[k] = Vec3<Dd>{{e[k].x, t[0]}, {e[k].y, t[1]}, {e[k].z, t[2]}};
-      }
+      double t[4][3];
+      chain_tangents(w, o, valid, t);
       const double* cd = T.chainD[set];
-      const Dd cb[2] = {{cd[0], 0.0}, {cd[1], 0.0}};
-      const Dd cn[2] = {{cd[2], 0.0}, {cd[3], 0.0}};
-      Vec3<Dd> fbond{{0, 0}, {0, 0}, {0, 0}}, fbend{{0, 0}, {0, 0}, {0, 0}};
-      if (valid[1]) bond_term<Dd>(ed[1], cb, Dd{-1.0, 0.0}, fbond);
-      if (valid[2]) bond_term<Dd>(ed[2], cb, Dd{1.0, 0.0}, fbond);
-      if (valid[0] && valid[1]) bend_term<Dd>(ed[0], ed[1], cn, 2, fbend);
-      if (valid[1] && valid[2]) bend_term<Dd>(ed[1], ed[2], cn, 1, fbend);
-      if (valid[2] && valid[3]) bend_term<Dd>(ed[2], ed[3], cn, 0, fbend);
-      F[0] += fbond.x.v + fbend.x.v;
-      F[1] += fbond.y.v + fbend.y.v;
-      F[2] += fbond.z.v + fbend.z.v;
-      K[0] += fbond.x.t + fbend.x.t;
-      K[1] += fbond.y.t + fbend.y.t;
-      K[2] += fbond.z.t + fbend.z.t;
-      // dF/dk with unit constants (the forces are linear in k)
-      const double ub[2] = {cd[0], 1.0}, un[2] = {cd[2], 1.0};
-      Vec3<double> f1{0, 0, 0}, f2{0, 0, 0};
-      if (valid[1]) bond_term<double>(e[1], ub, -1.0, f1);
-      if (valid[2]) bond_term<double>(e[2], ub, 1.0, f1);
-      if (valid[0] && valid[1]) bend_term<double>(e[0], e[1], un, 2, f2);
-      if (valid[1] && valid[2]) bend_term<double>(e[1], e[2], un, 1, f2);
-      if (valid[2] && valid[3]) bend_term<double>(e[2], e[3], un, 0, f2);
-      // energies owned by the first bead of each bond / bend
-      double ub_u = 0.0, un_u = 0.0;
-      if (valid[2]) ub_u = bond_pot(e[2], ub);
-      if (valid[2] && valid[3]) un_u = bend_pot(e[2], e[3], un);
-      gJ = invT * (cd[1] * ub_u + cd[3] * un_u);
-      g1 = dt * (wi[0] * f1.x + wi[1] * f1.y + wi[2] * f1.z) + invT * ub_u;
-      g2 = dt * (wi[0] * f2.x + wi[1] * f2.y + wi[2] * f2.z) + invT * un_u;
+      ChainDual c;
+      chain_dual<true>(e, t, valid, cd, c);
+      for (int d = 0; d < 3; ++d) {
+        F[d] += fma(cd[1], c.fb[d], cd[3] * c.fn[d]);
+        K[d] += fma(cd[1], c.tb[d], cd[3] * c.tn[d]);
+      }
+      gJ = invT * (cd[1] * c.ub + cd[3] * c.un);
+      g1 = dt * dot3(wi, c.fb) + invT * c.ub;
+      g2 = dt * dot3(wi, c.fn) + invT * c.un;
     }
     const double damp = 1.0 - rp.gamma * dt;
     for (int d = 0; d < 3; ++d) {
@@ -342,26 +416,12 @@ __global__ void __launch_bounds__(kBlock) k_adj_hvp_out(DevPtrs P, int cur, cons
     Vec3<double> e[4];
     bool valid[4];
     chain_vectors<MIXED, double>(P, cur, i, p, len, box, rs, e, valid);
-    Vec3<Dd> ed[4];
-    for (int k = 0; k < 4; ++k) {
-      const int a = o - 2 + k, b = o - 1 + k;
-      double t[3] = {0, 0, 0};
-      if (valid[k])
-        for (int d = 0; d < 3; ++d) t[d] = w[3 * a + d] - w[3 * b + d];
-      ed[k] = Vec3<Dd>{{e[k].x, t[0]}, {e[k].y, t[1]}, {e[k].z, t[2]}};
-    }
+    double t[4][3];
+    chain_tangents(w, o, valid, t);
     const double* cd = T.chainD[set];
-    const Dd cb[2] = {{cd[0], 0.0}, {cd[1], 0.0}};
-    const Dd cn[2] = {{cd[2], 0.0}, {cd[3], 0.0}};
-    Vec3<Dd> f{{0, 0}, {0, 0}, {0, 0}};
-    if (valid[1]) bond_term<Dd>(ed[1], cb, Dd{-1.0, 0.0}, f);
-    if (valid[2]) bond_term<Dd>(ed[2], cb, Dd{1.0, 0.0}, f);
-    if (valid[0] && valid[1]) bend_term<Dd>(ed[0], ed[1], cn, 2, f);
-    if (valid[1] && valid[2]) bend_term<Dd>(ed[1], ed[2], cn, 1, f);
-    if (valid[2] && valid[3]) bend_term<Dd>(ed[2], ed[3], cn, 0, f);
-    K[0] += f.x.t;
-    K[1] += f.y.t;
-    K[2] += f.z.t;
+    ChainDual c;
+    chain_dual<false>(e, t, valid, cd, c);
+    for (int d = 0; d < 3; ++d) K[d] += fma(cd[1], c.tb[d], cd[3] * c.tn[d]);
   }
   for (int d = 0; d < 3; ++d) out[3 * o + d] = K[d];
 }
