@@ -1,9 +1,12 @@
-// The MD loop of a small or mid-size system as one persistent kernel.
+// The MD loop of a system of up to 65,000 beads as one persistent kernel.
 //
 // Kernel by kernel, a loop step of a few thousand beads is all latency: two
 // step kernels and, every second step, four list kernels of 5-25 us each that
-// keep at most a tenth of the chip's warps busy (1,176 beads: 35 us per step,
-// 15,000 beads: 41 us; here 15 and 25).  Here every CTA owns a contiguous range of the
+// keep at most a tenth of the chip's warps busy.  At tens of thousands the
+// launches' starts and tails, the reordered state's way through memory and one
+// list cell per CTA still cost a quarter of a step.  us per step, kernel by
+// kernel and here: 1,176 beads 35 and 14, 15,000 41 and 23, 24,000 54 and 31,
+// 33,000 64 and 37, 60,000 83 and 63.  Here every CTA owns a contiguous range of the
 // cell-sorted beads and keeps their positions, velocities and bookkeeping in
 // shared memory; only the position mirror goes through global memory.  A step
 // is one grid barrier: each CTA forms its beads' pair sums (and beside them
@@ -23,10 +26,10 @@ namespace smd {
 
 // threads per CTA at most: 80 registers per thread, or 64 where many beads want more warps
 __host__ __device__ constexpr int run_threads(int lanes) { return lanes == 8 ? 1024 : 768; }
-// Above this a step is throughput, and the separate kernels' occupancy wins
-// (15,000 beads: 25 us per step here, 41 us kernel by kernel).
-constexpr int kRunMaxBeads = 20000;
-constexpr int kRunCells = 20480;    // largest list-cell grid (its starts are kept in shared memory)
+// What 16-bit cell starts can count.  It still gains a quarter there (63,654
+// beads: 84 us per step kernel by kernel, 67 here).
+constexpr int kRunMaxBeads = 65000;
+constexpr int kRunCells = 81920;    // largest list-cell grid (its starts, 160 KB, are kept in shared memory)
 constexpr int kRunSpinLimit = 1 << 22;  // polls of a barrier: some seconds
 
 // Grid-wide words of the persistent loop (zero between launches).
@@ -74,8 +77,9 @@ __device__ __forceinline__ double wrap64(double x, double box) {
 // The stencil of cell (cx, cy, cz) as contiguous bead ranges with prefix sums,
 // formed by one warp: lane l < 18 takes half of row l / 2 (dy, dz), whose
 // cells cx - 1 .. cx + 1 are one range unless it wraps in x; axes with fewer
-// than 3 cells take every cell once.  seg: first beads [0, 18), first slots
-// [18, 37).  Returns the number of slots.
+// than 3 cells take every cell once.  seg: first bead less first slot [0, 18),
+// the slot after the last [18, 36), none after the last segment's.  Returns the
+// number of slots.
 __device__ __forceinline__ int run_stencil(const RepState& rs, const unsigned short* starts, int cx, int cy, int cz,
                                            int* seg) {
   const int lane = threadIdx.x & 31;
@@ -115,67 +119,137 @@ __device__ __forceinline__ int run_stencil(const RepState& rs, const unsigned sh
   __syncwarp();
   if (len > 0) {
     const int k = __popc(full & ((1u << lane) - 1u));
-    seg[k] = start;
-    seg[18 + k] = incl - len;
+    seg[k] = start - (incl - len);
+    seg[18 + k] = incl == total ? 0x7fffffff : incl;
   }
-  if (lane == 0) seg[18 + __popc(full)] = total;
   __syncwarp();
   return total;
 }
 
+// The beads of a stencil's slots, 32 at a time.  The segment of the first slot
+// is the warp's; lanes behind a boundary take the next one, so a round costs a
+// few uniform instructions per boundary it crosses instead of a search per lane.
+struct SlotWalk {
+  const int* seg;
+  int t = 0, off, end;
+  __device__ __forceinline__ explicit SlotWalk(const int* s) : seg(s), off(s[0]), end(s[18]) {}
+  // bead of slot min(k0 + lane, M - 1); k0 advances by 32 from call to call
+  __device__ __forceinline__ int round(int k0, int lane, int M) {
+    const int g = min(k0 + lane, M - 1);
+    while (end <= k0) {  // (only where the last round ended with the segment)
+      ++t;
+      off = seg[t];
+      end = seg[18 + t];
+    }
+    int o = off;
+    while (end < k0 + 32) {
+      ++t;
+      off = seg[t];
+      o = g >= end ? off : o;
+      end = seg[18 + t];
+    }
+    return o + g;
+  }
+};
+
+// Appends j to the list at out for the lanes with r2 < lim and d != self, in
+// lane order: a ballot, two counts and a predicated store (a branch around the
+// store costs three instructions more).
+__device__ __forceinline__ void keep_hits(float r2, float lim, int d, int self, unsigned int below, int j, int* out,
+                                          int kmax, int& count) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t.reg .b32 h, b;\n\t.reg .b64 a;\n\t"
+      "setp.lt.f32 p, %1, %2;\n\t"
+      "setp.ne.and.s32 p, %3, %4, p;\n\t"
+      "vote.sync.ballot.b32 h, p, 0xffffffff;\n\t"
+      "and.b32 b, h, %5;\n\t"
+      "popc.b32 b, b;\n\t"
+      "add.s32 b, b, %0;\n\t"
+      "setp.lt.and.s32 p, b, %6, p;\n\t"
+      "mad.wide.s32 a, b, 4, %7;\n\t"
+      "@p st.global.u32 [a], %8;\n\t"
+      "popc.b32 h, h;\n\t"
+      "add.s32 %0, %0, h;\n\t"
+      "}"
+      : "+r"(count)
+      : "f"(r2), "f"(lim), "r"(d), "r"(self), "r"(below), "r"(kmax), "l"(__cvta_generic_to_global(out)), "r"(j)
+      : "memory");
+}
+
 // Lists of bead a and (PAIR) of b in the same cell from the stencil's M slots,
 // by one warp.  Distances come from the exact fractional differences, whose
-// wrap is the minimum image, so thin grids need no other path; with OFFSET
-// (five cells on every axis) b's follow from a's and the offset between the
-// two: no candidate of the stencil is then near half the box from a and in
-// range of b.
-template <bool PAIR, bool OFFSET>
+// wrap is the minimum image, so thin grids need no other path.
+template <bool PAIR>
 __device__ __forceinline__ void run_scan(const uint4* m, const int* seg, int M, uint4 ma, uint4 mb, int ia, float x0,
                                          float x1, float x2, float lc2, int* oa, int kmax, int& ca, int& cb) {
   const int lane = threadIdx.x & 31;
   const unsigned int below = (1u << lane) - 1u;
-  const float ex = frac_delta(mb.x, ma.x, x0), ey = frac_delta(mb.y, ma.y, x1), ez = frac_delta(mb.z, ma.z, x2);
-  int* ob = oa + kmax;
-  int t = 0;  // segment of this lane's next slot (slots only increase)
-  auto slot_bead = [&](int g) {
-    while (seg[18 + t + 1] <= g) ++t;
-    return seg[t] + (g - seg[18 + t]);
-  };
   ca = cb = 0;
-  int j = slot_bead(min(lane, M - 1));
+  SlotWalk walk(seg);
+  int j = walk.round(0, lane, M);
   uint4 o = m[j];
   for (int k0 = 0; k0 < M; k0 += 32) {
     const int jc = j;
     const uint4 c = o;
-    const bool on = k0 + lane < M;
+    const float lim = k0 + lane < M ? lc2 : -1.f;
     if (k0 + 32 < M) {  // the next round's candidate, a round ahead
-      j = slot_bead(min(k0 + 32 + lane, M - 1));
+      j = walk.round(k0 + 32, lane, M);
       o = m[j];
     }
     const float ax = frac_delta(ma.x, c.x, x0), ay = frac_delta(ma.y, c.y, x1), az = frac_delta(ma.z, c.z, x2);
-    const bool ha = on & (jc != ia) & (ax * ax + ay * ay + az * az < lc2);
-    const unsigned int va = __ballot_sync(0xffffffffu, ha);
-    const int pa = ca + __popc(va & below);
-    if (ha && pa < kmax) oa[pa] = jc;
-    ca += __popc(va);
+    keep_hits(ax * ax + ay * ay + az * az, lim, jc - ia, 0, below, jc, oa, kmax, ca);
     if constexpr (PAIR) {
-      float bx, by, bz;
-      if constexpr (OFFSET) {
-        bx = ax + ex;
-        by = ay + ey;
-        bz = az + ez;
-      } else {
-        bx = frac_delta(mb.x, c.x, x0);
-        by = frac_delta(mb.y, c.y, x1);
-        bz = frac_delta(mb.z, c.z, x2);
-      }
-      const bool hb = on & (jc != ia + 1) & (bx * bx + by * by + bz * bz < lc2);
-      const unsigned int vb = __ballot_sync(0xffffffffu, hb);
-      const int pb = cb + __popc(vb & below);
-      if (hb && pb < kmax) ob[pb] = jc;
-      cb += __popc(vb);
+      const float bx = frac_delta(mb.x, c.x, x0), by = frac_delta(mb.y, c.y, x1), bz = frac_delta(mb.z, c.z, x2);
+      keep_hits(bx * bx + by * by + bz * bz, lim, jc - ia, 1, below, jc, oa + kmax, kmax, cb);
     }
   }
+}
+
+// Lists of n <= Q neighbouring beads of one cell, from bead ia on, by one warp
+// (grids of five cells on every axis: no candidate of the stencil is then near
+// half the box from the first bead and in range of another).  With c a
+// candidate's and x a bead's offset from the first of them, |c - x|^2 < L^2 is
+// |c|^2 - 2 x . c < L^2 - |x|^2: three FMAs and a comparison per bead, and one
+// load and conversion of a candidate for all: 104,000 cycles per build at 395
+// beads per CTA against 150,000 in pairs with six operations per distance.
+template <int Q>
+__device__ __forceinline__ void run_scan_group(const uint4* m, const int* seg, int M, const uint4* own, int n, int ia,
+                                               float x0, float x1, float x2, float lc2, int* out, int kmax, int* cnt) {
+  const int lane = threadIdx.x & 31;
+  const unsigned int below = (1u << lane) - 1u;
+  const uint4 ma = own[0];
+  float fx[Q], fy[Q], fz[Q], lim[Q];
+  int count[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const uint4 mq = own[q < n ? q : 0];
+    const float x = frac_delta(mq.x, ma.x, x0), y = frac_delta(mq.y, ma.y, x1), z = frac_delta(mq.z, ma.z, x2);
+    fx[q] = -2.f * x;
+    fy[q] = -2.f * y;
+    fz[q] = -2.f * z;
+    lim[q] = q < n ? lc2 - (x * x + y * y + z * z) : -1e30f;  // past the last bead: no hit
+    count[q] = 0;
+  }
+  SlotWalk walk(seg);
+  int j = walk.round(0, lane, M);
+  uint4 o = m[j];
+  for (int k0 = 0; k0 < M; k0 += 32) {
+    const int jc = j;
+    const float cx = frac_delta(o.x, ma.x, x0), cy = frac_delta(o.y, ma.y, x1), cz = frac_delta(o.z, ma.z, x2);
+    const float cc = k0 + lane < M ? cx * cx + cy * cy + cz * cz : 1e30f;
+    if (k0 + 32 < M) {  // the next round's candidate, a round ahead
+      j = walk.round(k0 + 32, lane, M);
+      o = m[j];
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      keep_hits(fmaf(fz[q], cz, fmaf(fy[q], cy, fmaf(fx[q], cx, cc))), lim[q], jc - ia, q, below, jc, out + q * kmax,
+                kmax, count[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if (lane == q && q < n) cnt[q] = count[q];
 }
 
 template <bool MIXED, int G>
@@ -186,7 +260,7 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
   __shared__ RepState rs;
   __shared__ __align__(8) R sF[6 * kMaxTypes * kMaxTypes], sU[6 * kMaxTypes * kMaxTypes];
   __shared__ int wsum[run_threads(G) / 32];
-  __shared__ int segs[run_threads(G) / 32][38];
+  __shared__ int segs[run_threads(G) / 32][36];
   __shared__ float smax[run_threads(G) / 32];
   __shared__ long long sdq[2];
   __shared__ double sdu[2];
@@ -425,8 +499,10 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
       if (tid < nb) key[tid] = cell_of(ref[tid]);
       __syncthreads();
       {
-        const float lcut = MIXED ? T.list_cut_f + 1e-4f
-                                 : T.list_cut_f * (1.f + 4e-6f) + 1e-4f +
+        // 1e-5 of the cut: more than the rounding of run_scan_group's squares (offsets
+        // stay within 4.2 cuts); plain form: + the mirror's resolution
+        const float lcut = MIXED ? T.list_cut_f * (1.f + 1e-5f) + 1e-4f
+                                 : T.list_cut_f * (1.f + 1e-5f) + 1e-4f +
                                        4.f * fmaxf(rs.len_per_frac[0], fmaxf(rs.len_per_frac[1], rs.len_per_frac[2]));
         const float lc2 = lcut * lcut;
         const float x0 = rs.len_per_frac[0], x1 = rs.len_per_frac[1], x2 = rs.len_per_frac[2];
@@ -445,13 +521,19 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
             last_cell = c;
           }
           const bool pair = q + 1 < end && key[q + 1] == c;
-          const uint4 mb = ref[pair ? q + 1 : q];
           const int i = b0 + q;
           int* out = P.nbr + (size_t)i * kmax;
+          if (pair && offset) {  // up to four beads at once (the order is by cell)
+            const int n = q + 2 < end && key[q + 2] == c ? (q + 3 < end && key[q + 3] == c ? 4 : 3) : 2;
+            if (n > 2) run_scan_group<4>(m, seg, M, ref + q, n, i, x0, x1, x2, lc2, out, kmax, cnt + q);
+            else run_scan_group<2>(m, seg, M, ref + q, n, i, x0, x1, x2, lc2, out, kmax, cnt + q);
+            q += n;
+            continue;
+          }
+          const uint4 mb = ref[pair ? q + 1 : q];
           int ca, cb;
-          if (pair && offset) run_scan<true, true>(m, seg, M, ma, mb, i, x0, x1, x2, lc2, out, kmax, ca, cb);
-          else if (pair) run_scan<true, false>(m, seg, M, ma, mb, i, x0, x1, x2, lc2, out, kmax, ca, cb);
-          else run_scan<false, false>(m, seg, M, ma, mb, i, x0, x1, x2, lc2, out, kmax, ca, cb);
+          if (pair) run_scan<true>(m, seg, M, ma, mb, i, x0, x1, x2, lc2, out, kmax, ca, cb);
+          else run_scan<false>(m, seg, M, ma, mb, i, x0, x1, x2, lc2, out, kmax, ca, cb);
           if (lane == 0) {
             cnt[q] = ca;
             if (pair) cnt[q + 1] = cb;

@@ -39,7 +39,7 @@ def _run(m, persistent, precision, cuts):
 
 
 CASES = [("bilayer", 150), ("bilayer", 401), ("bilayer", 1300), ("bilayer", 2601), ("bilayer", 9000), ("thin", 700),
-         ("vesicle", 300), ("vesicle", 4999)]
+         ("vesicle", 300), ("vesicle", 4999), ("vesicle", 13001), ("bilayer", 21650)]
 
 
 @pytest.mark.parametrize("shape,lipids", CASES)
@@ -52,8 +52,7 @@ def test_mixed_loop_bitwise(built, tmp_path, shape, lipids):
         assert np.array_equal(x, y)
     assert a[3] == b[3] and a[4] == b[4] > 0
     assert np.array_equal(a[5], b[5])  # the list and state it leaves serve the other calls
-    if len(m.type) <= 20000:  # larger systems run as graphs
-        assert a[6] < b[6] / 10
+    assert a[6] < b[6] / 10
 
 
 @pytest.mark.parametrize("shape,lipids", [("bilayer", 150), ("bilayer", 1300), ("thin", 700), ("vesicle", 2999)])
