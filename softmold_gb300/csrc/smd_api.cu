@@ -115,14 +115,15 @@ struct smd_system {
     int kernels = 0;  // kernel nodes outside the conditional bodies
   } graph[2];
   bool use_graphs = true;
-  // the persistent loop kernel (single systems without spheres or field terms,
-  // up to kRunMaxBeads): CTAs, beads and threads per CTA, lanes per bead
+  // the persistent loop kernel (no spheres, no BOND / BEND or field terms, up to
+  // kRunMaxBeads per replica): CTAs, beads and threads per CTA, lanes per bead
   struct RunLoop {
     int grid = 0;  // 0: not used
     int beads = 0, threads = 0, lanes = 8;
     size_t smem = 0;
     int* cnt = nullptr;
     RunSync* sync = nullptr;
+    RunPlace* place = nullptr;
   } run;
   // launch configuration chosen by the autotuner (mixed form): lanes per bead
   // of the pair pass and the list-build kernel (0 flat/128, 1 flat/256,
@@ -441,7 +442,7 @@ int launch_run(smd_system* h, RunArgs a) {
 // `steps` loop iterations (barostat trials included) in one persistent kernel.
 int advance_run(smd_system* h, int steps) {
   const auto& r = h->run;
-  const RunArgs a{h->it, h->cur, steps, h->resize_rate, h->barostat ? 1 : 0, r.beads, r.cnt, r.sync};
+  const RunArgs a{h->it, h->cur, steps, h->resize_rate, h->barostat ? 1 : 0, r.beads, r.cnt, r.sync, r.place};
   int rc;
   if (h->mixed) rc = r.lanes == 32 ? launch_run<true, 32>(h, a) : (r.lanes == 16 ? launch_run<true, 16>(h, a) : launch_run<true, 8>(h, a));
   else rc = r.lanes == 32 ? launch_run<false, 32>(h, a) : (r.lanes == 16 ? launch_run<false, 16>(h, a) : launch_run<false, 8>(h, a));
@@ -474,14 +475,44 @@ int run_fits_device(smd_system* h, bool* fits) {
 int run_setup(smd_system* h) {
   auto& r = h->run;
   r.grid = 0;
-  if (h->n_rep != 1 || h->n_sph > 0 || h->n_terms > 0 || h->n > kRunMaxBeads || h->n_cells > kRunCells) return 0;
-  const int ctas = std::min(h->sms, 255);
-  r.beads = std::max(8, (h->n + ctas - 1) / ctas);
+  if (h->n_rep > h->sms || h->n_sph > 0 || h->n_terms > 0) return 0;
+  int cells = 0, most = 0;  // of the largest replica
+  for (int k = 0; k < h->n_rep; ++k) {
+    cells = std::max(cells, h->rp[k].cell_cap);
+    most = std::max(most, h->rp[k].bead_end - h->rp[k].bead_begin);
+  }
+  if (most > kRunMaxBeads || cells > kRunCells) return 0;
+  // the fewest beads per CTA that leave every replica CTAs of its own (at most
+  // 255 each: the barrier counts them in 8 bits)
+  auto ctas_at = [&](int beads, int* largest) {
+    long long sum = 0;
+    for (int k = 0; k < h->n_rep; ++k) {
+      const int c = (h->rp[k].bead_end - h->rp[k].bead_begin + beads - 1) / beads;
+      *largest = std::max(*largest, c);
+      sum += c;
+    }
+    return sum;
+  };
+  int lo = 8, hi = std::max(8, most);
+  while (lo < hi) {
+    const int mid = (lo + hi) / 2;
+    int largest = 0;
+    const long long sum = ctas_at(mid, &largest);
+    if (sum <= h->sms && largest <= 255) hi = mid; else lo = mid + 1;
+  }
+  r.beads = lo;
   r.lanes = r.beads <= 24 ? 32 : (r.beads <= 48 ? 16 : 8);
   r.threads = std::min(run_threads(r.lanes), std::max(256, (r.beads * r.lanes + r.beads + 63) / 32 * 32));
   if (r.beads > r.threads) return 0;
-  r.smem = run_smem(r.beads, h->n_cells, h->mixed, r.threads, r.lanes);
-  const int grid = (h->n + r.beads - 1) / r.beads;
+  r.smem = run_smem(r.beads, cells, h->mixed, r.threads, r.lanes);
+  std::vector<RunPlace> place;
+  int cnt = 0;
+  for (int k = 0; k < h->n_rep; ++k) {
+    const int c = (h->rp[k].bead_end - h->rp[k].bead_begin + r.beads - 1) / r.beads;
+    for (int i = 0; i < c; ++i) place.push_back(RunPlace{k, i, c, cnt});
+    cnt += 2 * run_cells(h->rp[k].cell_cap);
+  }
+  const int grid = (int)place.size();
   r.grid = grid;
   bool fits = false;
   int rc;
@@ -489,7 +520,11 @@ int run_setup(smd_system* h) {
   else rc = r.lanes == 32 ? run_fits_device<false, 32>(h, &fits) : (r.lanes == 16 ? run_fits_device<false, 16>(h, &fits) : run_fits_device<false, 8>(h, &fits));
   r.grid = 0;
   if (rc || !fits) return rc;
-  if ((rc = h->alloc(&r.cnt, 2 * (size_t)run_cells(h->n_cells))) || (rc = h->alloc(&r.sync, 1))) return rc;
+  if ((rc = h->alloc(&r.cnt, (size_t)cnt)) || (rc = h->alloc(&r.sync, (size_t)h->n_rep)) ||
+      (rc = h->alloc(&r.place, place.size())))
+    return rc;
+  SMD_CUDA(cudaMemcpyAsync(r.place, place.data(), place.size() * sizeof(RunPlace), cudaMemcpyHostToDevice, h->stream));
+  SMD_CUDA(cudaStreamSynchronize(h->stream));
   r.grid = grid;
   return 0;
 }

@@ -1,4 +1,5 @@
-// The MD loop of a system of up to 65,000 beads as one persistent kernel.
+// The MD loop as one persistent kernel, for systems and batches whose replicas
+// have up to 65,000 beads each.
 //
 // Kernel by kernel, a loop step of a few thousand beads is all latency: two
 // step kernels and, every second step, four list kernels of 5-25 us each that
@@ -13,7 +14,9 @@
 // the bonded forces and the noise), integrates them, writes the next mirror
 // and arrives.  A list rebuild adds one barrier (between the reordering and
 // the stencil scans), a barostat trial one (its summed energy difference).
-// Every barrier waits with a limit.
+// Every barrier waits with a limit.  The CTAs of a batch are dealt out to its
+// replicas, which wait for nobody else: each has its own barrier, its own list
+// rebuilds and its own trials.
 //
 // The arithmetic of a step is that of k_force, k_integ, k_mc and k_finish, and
 // the mixed form's sums are exact in any order, so a mixed run has the same
@@ -32,14 +35,21 @@ constexpr int kRunMaxBeads = 65000;
 constexpr int kRunCells = 81920;    // largest list-cell grid (its starts, 160 KB, are kept in shared memory)
 constexpr int kRunSpinLimit = 1 << 22;  // polls of a barrier: some seconds
 
-// Grid-wide words of the persistent loop (zero between launches).
+// A CTA's place: its replica, its number among the replica's CTAs, and where
+// the replica's cell counts begin.
+struct RunPlace {
+  int rep, index, ctas, cnt;
+};
+
+// Words shared by a replica's CTAs in the persistent loop (zero between launches).
 struct RunSync {
   // arrivals in the low 40 bits, then three 8-bit counts (by step modulo 3) of
   // the CTAs with a bead beyond the list's margin: they ride on the arrival,
   // so the barrier itself tells whether the list must be rebuilt
   unsigned long long arrive;
-  unsigned int left;             // CTAs that are done with the kernel
-  unsigned int pad;
+  unsigned int left;             // CTAs of the grid that are done with the kernel (first replica's)
+  int rebuild, rebuilds;         // the replica's list state at the end, for the last of them
+  double slack;
   long long dq_pair[2], dq_bond[2];  // trial sums, alternating
   double du_pair[2], du_bond[2];
 };
@@ -51,8 +61,9 @@ struct RunArgs {
   int rate;       // barostat period
   int barostat;
   int beads;      // beads per CTA
-  int* cnt;       // 2 x run_cells(n_cells_total) cell counts, zero between launches
-  RunSync* sync;
+  int* cnt;       // 2 x run_cells(cells) cell counts per replica, zero between launches
+  RunSync* sync;  // per replica
+  const RunPlace* place;  // per CTA
 };
 
 // Shared memory per CTA beyond the static part.
@@ -80,8 +91,8 @@ __device__ __forceinline__ double wrap64(double x, double box) {
 // than 3 cells take every cell once.  seg: first bead less first slot [0, 18),
 // the slot after the last [18, 36), none after the last segment's.  Returns the
 // number of slots.
-__device__ __forceinline__ int run_stencil(const RepState& rs, const unsigned short* starts, int cx, int cy, int cz,
-                                           int* seg) {
+__device__ __forceinline__ int run_stencil(const RepState& rs, const unsigned short* starts, int first, int cx,
+                                           int cy, int cz, int* seg) {
   const int lane = threadIdx.x & 31;
   const int n0 = rs.ncell[0], n1 = rs.ncell[1], n2 = rs.ncell[2];
   int start = 0, len = 0;
@@ -103,8 +114,8 @@ __device__ __forceinline__ int run_stencil(const RepState& rs, const unsigned sh
         u1 = u0 - 1;
       }
       if (u1 >= u0) {
-        start = starts[row + u0];
-        len = starts[row + u1 + 1] - start;
+        start = first + starts[row + u0];
+        len = starts[row + u1 + 1] - starts[row + u0];
       }
     }
   }
@@ -268,8 +279,16 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
   __shared__ int rebuild, slot, abort_s;
   __shared__ unsigned long long seen;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  const int b0 = blockIdx.x * A.beads, nb = min(A.beads, P.n - b0);
-  const int ncell = P.n_cells_total, ncell4 = run_cells(ncell);
+  // kept in shared memory, as what follows from it: registers are short here
+  __shared__ RunPlace me;
+  __shared__ RepParams rp;
+  if (tid == 0) {
+    me = A.place[blockIdx.x];
+    rp = P.rp[me.rep];
+  }
+  __syncthreads();
+  const int b0 = rp.bead_begin + me.index * A.beads, nb = min(A.beads, rp.bead_end - b0);
+  const int ncell = rp.cell_cap, ncell4 = run_cells(ncell);
   // dynamic shared memory (run_smem)
   unsigned char* at = reinterpret_cast<unsigned char*>(run_dyn);
   static_assert(kRunMaxBeads < 65536, "16-bit cell starts");
@@ -290,13 +309,12 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
   at += run_align(sizeof(int) * 4 * (size_t)A.beads);
   int* queue = reinterpret_cast<int*>(at);
   const Tables& T = *P.tab;
-  const RepParams& rp = P.rp[0];
   const int nT = T.nT;
   const int NB = A.beads;
 
   // ---- entry
   for (int k = tid; k < (int)(sizeof(RepState) / 4); k += nt)
-    reinterpret_cast<int*>(&rs)[k] = reinterpret_cast<const int*>(P.rs)[k];
+    reinterpret_cast<int*>(&rs)[k] = reinterpret_cast<const int*>(P.rs + me.rep)[k];
   for (int k = tid; k < 6 * nT * nT; k += nt) {
     if constexpr (MIXED) {
       sF[pack_force_row(k)] = T.fF[k];
@@ -336,14 +354,14 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
     __syncthreads();
     ++waited;
     if (tid == 0) {
-      const unsigned long long target = waited * gridDim.x;
+      const unsigned long long target = waited * me.ctas;
       // release: the CTA's writes (ordered before by the block barrier) are
       // visible to whoever sees the arrival; the acquire below is its other end
-      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&A.sync->arrive), "l"(inc) : "memory");
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&A.sync[me.rep].arrive), "l"(inc) : "memory");
       unsigned long long v = 0;
       int polls = 0;
       for (;;) {
-        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&A.sync->arrive) : "memory");
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&A.sync[me.rep].arrive) : "memory");
         if ((v & ((1ull << 40) - 1)) >= target) break;
         if (++polls > kRunSpinLimit) {
           atomicOr(&P.g->error, 8);
@@ -394,7 +412,7 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
     return (warp > 0 ? before : 0) + x - v;
   };
   auto draw = [&]() {
-    if (tid == 0) draw_trial(rs, rp, P.trial_u[(size_t)slot * 2]);
+    if (tid == 0) draw_trial(rs, rp, P.trial_u[((size_t)slot * P.n_rep + me.rep) * 2]);
   };
   bool trial = A.barostat && phase == 0 && it != 0;
   {
@@ -403,7 +421,7 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
     if (stale && tid < nb) {
       const int c = cell_of(P.m4[cur][b0 + tid]);
       key[tid] = c;
-      atomicAdd(A.cnt + ncell4 + c, 1);
+      atomicAdd(A.cnt + me.cnt + ncell4 + c, 1);
     }
     if (trial && !stale && tid < nb) {
       const double x[3] = {st[tid], st[NB + tid], st[2 * NB + tid]};
@@ -412,13 +430,13 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
     if ((stale || trial) && !barrier(1)) return;
   }
 
-  int trials = 0;
+  int trials = 0, rebuilds = 0;
   for (int s = 0; s < A.steps; ++s) {
     const bool last = s + 1 == A.steps;
     if (rebuild) {
       // ---- exclusive scan of the cell counts, by every CTA for itself
       {
-        const int4* counts = reinterpret_cast<const int4*>(A.cnt + (size_t)((s + 1) & 1) * ncell4);
+        const int4* counts = reinterpret_cast<const int4*>(A.cnt + me.cnt + (size_t)((s + 1) & 1) * ncell4);
         constexpr int kQuads = 4;  // 16 consecutive counts per thread and pass, loaded together
         int carry = 0, most = 0;
         for (int q0 = 0; q0 < ncell4 / 4; q0 += kQuads * nt) {
@@ -451,12 +469,12 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
           __syncthreads();  // wsum is used again
         }
         if (most > kNbrMaxCell) atomicOr(&P.g->error, 2);
-        if (tid == 0) starts[ncell4] = (unsigned short)P.n;
+        if (tid == 0) starts[ncell4] = (unsigned short)(rp.bead_end - rp.bead_begin);
       }
       __syncthreads();
       // ---- scatter to the new order (cell_count: the cells' fill)
       if (tid < nb) {
-        const int c = key[tid], nw_i = starts[c] + atomicAdd(&P.cell_count[c], 1);
+        const int c = key[tid], nw_i = rp.bead_begin + starts[c] + atomicAdd(P.cell_count + rp.cell_begin + c, 1);
         P.tx[nw_i] = st[tid];
         P.ty[nw_i] = st[NB + tid];
         P.tz[nw_i] = st[2 * NB + tid];
@@ -492,7 +510,7 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
       }
       if (tid == 0) {
         slack = 0.0;
-        if (blockIdx.x == 0) P.g->n_rebuilds++;
+        ++rebuilds;
       }
       __syncthreads();
       // ---- lists: a warp takes two neighbouring beads at a time, or one where that leaves warps idle
@@ -517,7 +535,7 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
           const int c = key[q];
           if (c != last_cell) {  // neighbouring beads mostly share it
             const int n0 = rs.ncell[0], n1 = rs.ncell[1], row = c / n0;
-            M = run_stencil(rs, starts, c - row * n0, row % n1, row / n1, seg);
+            M = run_stencil(rs, starts, rp.bead_begin, c - row * n0, row % n1, row / n1, seg);
             last_cell = c;
           }
           const bool pair = q + 1 < end && key[q + 1] == c;
@@ -551,11 +569,11 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
           atomicMax(&P.g->need_nbr, count);
         }
       }
-      for (int c = blockIdx.x * nt + tid; c < ncell; c += gridDim.x * nt) P.cell_count[c] = 0;
+      for (int c = me.index * nt + tid; c < ncell; c += me.ctas * nt) P.cell_count[rp.cell_begin + c] = 0;
       __syncthreads();
     }
     // the counts of the step before this one: read above at the latest
-    for (int c = blockIdx.x * nt + tid; c < ncell; c += gridDim.x * nt) A.cnt[(size_t)((s + 1) & 1) * ncell4 + c] = 0;
+    for (int c = me.index * nt + tid; c < ncell; c += me.ctas * nt) A.cnt[me.cnt + (size_t)((s + 1) & 1) * ncell4 + c] = 0;
     if (tid == 0) {
       sdq[0] = sdq[1] = 0;
       sdu[0] = sdu[1] = 0.0;
@@ -681,28 +699,28 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
       const int par = trials & 1;
       if (tid == 0) {
         if constexpr (MIXED) {
-          atomicAdd((unsigned long long*)&A.sync->dq_pair[par], (unsigned long long)sdq[0]);
-          atomicAdd((unsigned long long*)&A.sync->dq_bond[par], (unsigned long long)sdq[1]);
+          atomicAdd((unsigned long long*)&A.sync[me.rep].dq_pair[par], (unsigned long long)sdq[0]);
+          atomicAdd((unsigned long long*)&A.sync[me.rep].dq_bond[par], (unsigned long long)sdq[1]);
         } else {
-          atomicAdd(&A.sync->du_pair[par], sdu[0]);
-          atomicAdd(&A.sync->du_bond[par], sdu[1]);
+          atomicAdd(&A.sync[me.rep].du_pair[par], sdu[0]);
+          atomicAdd(&A.sync[me.rep].du_bond[par], sdu[1]);
         }
-        if (blockIdx.x == 0) {  // the previous trial's sums: every CTA has read them
-          A.sync->dq_pair[par ^ 1] = A.sync->dq_bond[par ^ 1] = 0;
-          A.sync->du_pair[par ^ 1] = A.sync->du_bond[par ^ 1] = 0.0;
+        if (me.index == 0) {  // the previous trial's sums: every CTA has read them
+          A.sync[me.rep].dq_pair[par ^ 1] = A.sync[me.rep].dq_bond[par ^ 1] = 0;
+          A.sync[me.rep].du_pair[par ^ 1] = A.sync[me.rep].du_bond[par ^ 1] = 0.0;
         }
       }
       if (!barrier(1)) return;
       if (tid == 0) {
-        rs.dUq_pair = __ldcg(&A.sync->dq_pair[par]);
-        rs.dUq_bond = __ldcg(&A.sync->dq_bond[par]);
-        rs.dU_pair = __ldcg(&A.sync->du_pair[par]);
-        rs.dU_bond = __ldcg(&A.sync->du_bond[par]);
+        rs.dUq_pair = __ldcg(&A.sync[me.rep].dq_pair[par]);
+        rs.dUq_bond = __ldcg(&A.sync[me.rep].dq_bond[par]);
+        rs.dU_pair = __ldcg(&A.sync[me.rep].du_pair[par]);
+        rs.dU_bond = __ldcg(&A.sync[me.rep].du_bond[par]);
         rs.accept = 0;
         shift_s = 0.0;
         if (rp.dlxy != 0) {
-          shift_s = decide_trial(rs, rp, T, P.trial_u[(size_t)slot * 2 + 1]);
-          if (blockIdx.x == 0) P.accept_log[slot] = rs.accept;
+          shift_s = decide_trial(rs, rp, T, P.trial_u[((size_t)slot * P.n_rep + me.rep) * 2 + 1]);
+          if (me.index == 0) P.accept_log[(size_t)slot * P.n_rep + me.rep] = rs.accept;
         }
         slack += shift_s;
         ++slot;
@@ -734,7 +752,7 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
       if constexpr (!MIXED) P.d4[cur ^ 1][i] = make_double4(x[0], x[1], x[2], __longlong_as_double((long long)w));
       const int c = cell_of(mn);
       key[tid] = c;
-      if (!last) atomicAdd(A.cnt + (size_t)(s & 1) * ncell4 + c, 1);
+      if (!last) atomicAdd(A.cnt + me.cnt + (size_t)(s & 1) * ncell4 + c, 1);
       if (next_trial && !last) P.refcell[i] = ref_key(x);
     }
     vmax = warp_max(vmax);
@@ -746,8 +764,8 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
       const float bm = warp_max(lane < nw ? smax[lane] : 0.f);
       if ((double)bm + slack > P.half_skin) inc += 1ull << (40 + 8 * (s % 3));
       if (last && lane == 0 && bm > 0.f) atomicMax(&P.g->dmax_bits, __float_as_uint(bm));
-      // CTA 0 clears the field of two steps ago (the next step's), which every CTA has read
-      if (blockIdx.x == 0 && s >= 2) inc -= ((seen >> (40 + 8 * ((s + 1) % 3))) & 0xffull) << (40 + 8 * ((s + 1) % 3));
+      // the first CTA clears the field of two steps ago (the next step's), which every CTA has read
+      if (me.index == 0 && s >= 2) inc -= ((seen >> (40 + 8 * ((s + 1) % 3))) & 0xffull) << (40 + 8 * ((s + 1) % 3));
     }
     if (!barrier(inc)) return;
     if (tid == 0) {
@@ -777,27 +795,36 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
       if constexpr (!MIXED) P.d4[want][i] = P.d4[cur][i];
     }
   }
-  if (blockIdx.x == 0) {
+  if (me.index == 0) {
     for (int k = tid; k < (int)(sizeof(RepState) / 4); k += nt)
-      reinterpret_cast<int*>(P.rs)[k] = reinterpret_cast<const int*>(&rs)[k];
+      reinterpret_cast<int*>(P.rs + me.rep)[k] = reinterpret_cast<const int*>(&rs)[k];
     if (tid == 0) {
-      P.g->slack = slack;
-      P.g->trial_slot = slot;
-      P.g->rebuild = rebuild;
-      P.g->it = it;
-      P.g->last_disp = __uint_as_float(atomicExch(&P.g->dmax_bits, 0u));
+      RunSync& y = A.sync[me.rep];
+      y.slack = slack;
+      y.rebuild = rebuild;
+      y.rebuilds = rebuilds;
     }
   }
   __syncthreads();
   if (tid == 0) {
     __threadfence();
     if (atomicAdd(&A.sync->left, 1u) == gridDim.x - 1) {  // every CTA has passed its last barrier
-      A.sync->arrive = 0;
-      A.sync->left = 0;
-      for (int k = 0; k < 2; ++k) {
-        A.sync->dq_pair[k] = A.sync->dq_bond[k] = 0;
-        A.sync->du_pair[k] = A.sync->du_bond[k] = 0.0;
+      __threadfence();
+      double most = 0.0;
+      int any = 0, count = 0;
+      for (int r = 0; r < P.n_rep; ++r) {
+        RunSync& y = A.sync[r];
+        most = fmax(most, __ldcg(&y.slack));
+        any |= __ldcg(&y.rebuild);
+        count = max(count, __ldcg(&y.rebuilds));
+        y = RunSync{};
       }
+      P.g->slack = most;
+      P.g->rebuild = any;
+      P.g->n_rebuilds += count;
+      P.g->trial_slot = slot;
+      P.g->it = it;
+      P.g->last_disp = __uint_as_float(atomicExch(&P.g->dmax_bits, 0u));
     }
   }
 }

@@ -70,3 +70,34 @@ def test_terms(built):
     a, b = _run(m, True, smd.MIXED, (24, 9)), _run(m, False, smd.MIXED, (24, 9))
     for x, y in zip(a[:3], b[:3]):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("precision", [smd.MIXED, smd.PLAIN_FP64])
+@pytest.mark.parametrize("sizes", [(150, 401, 126, 1300), (2600, 300, 4999, 700), (130,) * 40])
+def test_batch_loop(built, tmp_path, sizes, precision):
+    """A batch's replicas on CTAs of their own: uneven sizes,
+    one replica without a barostat, and few CTAs for many replicas."""
+    ms = []
+    for k, lipids in enumerate(sizes):
+        p = str(tmp_path / f"b{k}.mpd")
+        smd.synth_bilayer(p, 7 + k, lipids, 3.45, 15.0, 0.0 if k == 1 else 0.01, 0.1 * (k % 3))
+        ms.append(smd.read_mpd(p))
+    outs = []
+    for persistent in (True, False):
+        s = smd.System(ms, precision=precision)
+        s.use_graphs(persistent)
+        s.prepare()
+        l0 = s.launches()
+        for k in (1, 8, 31):
+            s.advance(k)
+        outs.append(s.state() + (np.array([s.box(r) for r in range(len(ms))]), s.launches() - l0,
+                                 [s.mc_stats(r) for r in range(len(ms))]))
+        s.close()
+    a, b = outs
+    for x, y in zip(a[:3], b[:3]):
+        if precision == smd.MIXED:
+            assert np.array_equal(x, y)
+        else:
+            assert np.abs(x - y).max() < 1e-9
+    assert a[3] < b[3] / 10
+    assert [m["accepted"] for m in a[4]] == [m["accepted"] for m in b[4]]
