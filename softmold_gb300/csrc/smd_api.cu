@@ -119,7 +119,7 @@ struct smd_system {
   // kRunMaxBeads per replica): CTAs, beads and threads per CTA, lanes per bead
   struct RunLoop {
     int grid = 0;  // 0: not used
-    int beads = 0, threads = 0, lanes = 8;
+    int beads = 0, threads = 0, lanes = 8, warps = 0;
     size_t smem = 0;
     int* cnt = nullptr;
     RunSync* sync = nullptr;
@@ -427,10 +427,10 @@ bool is_trial_step(const smd_system* h, long long it) {
   return h->barostat && (it % h->resize_rate) == 0 && it != 0;
 }
 
-template <bool MIXED, int G>
+template <bool MIXED, int G, int NW>
 int launch_run(smd_system* h, RunArgs a) {
   void* args[] = {&h->P, &a};
-  const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(&k_run<MIXED, G>), dim3(h->run.grid),
+  const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(&k_run<MIXED, G, NW>), dim3(h->run.grid),
                                                     dim3(h->run.threads), args, h->run.smem, h->stream);
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
@@ -439,13 +439,25 @@ int launch_run(smd_system* h, RunArgs a) {
   return check_launch(h);
 }
 
+// The variant a handle's layout takes.
+#define SMD_RUN_VARIANT(h, f, ...)                                                         \
+  [&]() -> int {                                                                           \
+    const auto& r_ = (h)->run;                                                             \
+    if ((h)->mixed) {                                                                      \
+      if (r_.lanes == 32) return f<true, 32, 24>(__VA_ARGS__);                             \
+      if (r_.lanes == 16) return f<true, 16, 24>(__VA_ARGS__);                             \
+      return r_.warps == 28 ? f<true, 8, 28>(__VA_ARGS__) : f<true, 8, 32>(__VA_ARGS__);   \
+    }                                                                                      \
+    if (r_.lanes == 32) return f<false, 32, 24>(__VA_ARGS__);                              \
+    if (r_.lanes == 16) return f<false, 16, 24>(__VA_ARGS__);                              \
+    return r_.warps == 28 ? f<false, 8, 28>(__VA_ARGS__) : f<false, 8, 32>(__VA_ARGS__);   \
+  }()
+
 // `steps` loop iterations (barostat trials included) in one persistent kernel.
 int advance_run(smd_system* h, int steps) {
   const auto& r = h->run;
   const RunArgs a{h->it, h->cur, steps, h->resize_rate, h->barostat ? 1 : 0, r.beads, r.cnt, r.sync, r.place};
-  int rc;
-  if (h->mixed) rc = r.lanes == 32 ? launch_run<true, 32>(h, a) : (r.lanes == 16 ? launch_run<true, 16>(h, a) : launch_run<true, 8>(h, a));
-  else rc = r.lanes == 32 ? launch_run<false, 32>(h, a) : (r.lanes == 16 ? launch_run<false, 16>(h, a) : launch_run<false, 8>(h, a));
+  const int rc = SMD_RUN_VARIANT(h, launch_run, h, a);
   if (rc) return rc;
   for (int k = 0; k < steps; ++k)
     if (is_trial_step(h, h->it + k)) h->trials_used++;
@@ -455,9 +467,9 @@ int advance_run(smd_system* h, int steps) {
 }
 
 // Sets up the persistent loop where the system fits it.
-template <bool MIXED, int G>
+template <bool MIXED, int G, int NW>
 int run_fits_device(smd_system* h, bool* fits) {
-  const void* f = reinterpret_cast<const void*>(&k_run<MIXED, G>);
+  const void* f = reinterpret_cast<const void*>(&k_run<MIXED, G, NW>);
   int dev = 0, limit = 0, coop = 0, per_sm = 0;
   SMD_CUDA(cudaGetDevice(&dev));
   SMD_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -502,7 +514,8 @@ int run_setup(smd_system* h) {
   }
   r.beads = lo;
   r.lanes = r.beads <= 24 ? 32 : (r.beads <= 48 ? 16 : 8);
-  r.threads = std::min(run_threads(r.lanes), std::max(256, (r.beads * r.lanes + r.beads + 63) / 32 * 32));
+  r.warps = run_warps(r.beads, r.lanes);
+  r.threads = 32 * std::min(r.warps, std::max(24, run_tasks(r.beads, r.lanes)));
   if (r.beads > r.threads) return 0;
   r.smem = run_smem(r.beads, cells, h->mixed, r.threads, r.lanes);
   std::vector<RunPlace> place;
@@ -516,8 +529,7 @@ int run_setup(smd_system* h) {
   r.grid = grid;
   bool fits = false;
   int rc;
-  if (h->mixed) rc = r.lanes == 32 ? run_fits_device<true, 32>(h, &fits) : (r.lanes == 16 ? run_fits_device<true, 16>(h, &fits) : run_fits_device<true, 8>(h, &fits));
-  else rc = r.lanes == 32 ? run_fits_device<false, 32>(h, &fits) : (r.lanes == 16 ? run_fits_device<false, 16>(h, &fits) : run_fits_device<false, 8>(h, &fits));
+  rc = SMD_RUN_VARIANT(h, run_fits_device, h, &fits);
   r.grid = 0;
   if (rc || !fits) return rc;
   if ((rc = h->alloc(&r.cnt, (size_t)cnt)) || (rc = h->alloc(&r.sync, (size_t)h->n_rep)) ||

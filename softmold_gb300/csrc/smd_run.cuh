@@ -27,8 +27,18 @@
 
 namespace smd {
 
-// threads per CTA at most: 80 registers per thread, or 64 where many beads want more warps
-__host__ __device__ constexpr int run_threads(int lanes) { return lanes == 8 ? 1024 : 768; }
+// Warps per CTA at most, which set the registers per thread: 24 (80 registers)
+// where a CTA has few beads; with many, 28 (72) or 32 (64), whichever takes
+// their pair and bonded tasks in fewer rounds, 28 if both do: fewer spills then
+// count for more (395 beads per CTA, 112 tasks: 129,000 cycles per step against
+// 137,000; 99 beads, 29 tasks: 48,500 against 45,600).
+__host__ __device__ constexpr int run_tasks(int beads, int lanes) {
+  return (beads * lanes + 31) / 32 + (beads + 31) / 32;
+}
+__host__ __device__ constexpr int run_warps(int beads, int lanes) {
+  const int tasks = run_tasks(beads, lanes);
+  return lanes != 8 ? 24 : (beads <= 896 && (tasks + 27) / 28 == (tasks + 31) / 32 ? 28 : 32);
+}
 // What 16-bit cell starts can count.  It still gains a quarter there (63,654
 // beads: 84 us per step kernel by kernel, 67 here).
 constexpr int kRunMaxBeads = 65000;
@@ -50,6 +60,7 @@ struct RunSync {
   unsigned int left;             // CTAs of the grid that are done with the kernel (first replica's)
   int rebuild, rebuilds;         // the replica's list state at the end, for the last of them
   double slack;
+  unsigned int dmax[3], pad;     // largest displacement (FP32 bits) beyond the margin, by step modulo 3
   long long dq_pair[2], dq_bond[2];  // trial sums, alternating
   double du_pair[2], du_bond[2];
 };
@@ -91,10 +102,10 @@ __device__ __forceinline__ double wrap64(double x, double box) {
 // than 3 cells take every cell once.  seg: first bead less first slot [0, 18),
 // the slot after the last [18, 36), none after the last segment's.  Returns the
 // number of slots.
-__device__ __forceinline__ int run_stencil(const RepState& rs, const unsigned short* starts, int first, int cx,
+__device__ __forceinline__ int run_stencil(const int ncell[3], const unsigned short* starts, int first, int cx,
                                            int cy, int cz, int* seg) {
   const int lane = threadIdx.x & 31;
-  const int n0 = rs.ncell[0], n1 = rs.ncell[1], n2 = rs.ncell[2];
+  const int n0 = ncell[0], n1 = ncell[1], n2 = ncell[2];
   int start = 0, len = 0;
   if (lane < 18) {
     const int t = lane >> 1, half = lane & 1, oy = t % 3 - 1, oz = t / 3 - 1;
@@ -188,15 +199,14 @@ __device__ __forceinline__ void keep_hits(float r2, float lim, int d, int self, 
       : "memory");
 }
 
-// Lists of bead a and (PAIR) of b in the same cell from the stencil's M slots,
-// by one warp.  Distances come from the exact fractional differences, whose
-// wrap is the minimum image, so thin grids need no other path.
-template <bool PAIR>
-__device__ __forceinline__ void run_scan(const uint4* m, const int* seg, int M, uint4 ma, uint4 mb, int ia, float x0,
-                                         float x1, float x2, float lc2, int* oa, int kmax, int& ca, int& cb) {
+// Lists of beads a = ia and b = ia + 1 of the same cell from the stencil's M
+// slots, by one warp.  Distances come from the exact fractional differences,
+// whose wrap is the minimum image, so thin grids need no other path.
+__device__ __forceinline__ void run_scan_pair(const uint4* m, const int* seg, int M, uint4 ma, uint4 mb, int ia,
+                                              float x0, float x1, float x2, float lc2, int* oa, int kmax, int* cnt) {
   const int lane = threadIdx.x & 31;
   const unsigned int below = (1u << lane) - 1u;
-  ca = cb = 0;
+  int ca = 0, cb = 0;
   SlotWalk walk(seg);
   int j = walk.round(0, lane, M);
   uint4 o = m[j];
@@ -209,11 +219,34 @@ __device__ __forceinline__ void run_scan(const uint4* m, const int* seg, int M, 
       o = m[j];
     }
     const float ax = frac_delta(ma.x, c.x, x0), ay = frac_delta(ma.y, c.y, x1), az = frac_delta(ma.z, c.z, x2);
+    const float bx = frac_delta(mb.x, c.x, x0), by = frac_delta(mb.y, c.y, x1), bz = frac_delta(mb.z, c.z, x2);
     keep_hits(ax * ax + ay * ay + az * az, lim, jc - ia, 0, below, jc, oa, kmax, ca);
-    if constexpr (PAIR) {
-      const float bx = frac_delta(mb.x, c.x, x0), by = frac_delta(mb.y, c.y, x1), bz = frac_delta(mb.z, c.z, x2);
-      keep_hits(bx * bx + by * by + bz * bz, lim, jc - ia, 1, below, jc, oa + kmax, kmax, cb);
-    }
+    keep_hits(bx * bx + by * by + bz * bz, lim, jc - ia, 1, below, jc, oa + kmax, kmax, cb);
+  }
+  if (lane == 0) {
+    cnt[0] = ca;
+    cnt[1] = cb;
+  }
+}
+
+// Rounds `part`, part + parts, ... of bead ia's list, by one of the `parts` warps
+// that share it; count (shared memory) starts at 0.
+__device__ __forceinline__ void run_scan_part(const uint4* m, const int* seg, int M, uint4 ma, int ia, int part,
+                                              int parts, float x0, float x1, float x2, float lc2, int* out, int kmax,
+                                              int* count) {
+  const int lane = threadIdx.x & 31;
+  const unsigned int below = (1u << lane) - 1u;
+  SlotWalk walk(seg);
+  for (int k0 = 32 * part; k0 < M; k0 += 32 * parts) {
+    const int j = walk.round(k0, lane, M);
+    const uint4 c = m[j];
+    const float ax = frac_delta(ma.x, c.x, x0), ay = frac_delta(ma.y, c.y, x1), az = frac_delta(ma.z, c.z, x2);
+    const bool hit = k0 + lane < M && j != ia && ax * ax + ay * ay + az * az < lc2;
+    const unsigned int hits = __ballot_sync(0xffffffffu, hit);
+    int at = 0;
+    if (lane == 0 && hits) at = atomicAdd(count, __popc(hits));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(hits & below);
+    if (hit && at < kmax) out[at] = j;
   }
 }
 
@@ -263,20 +296,22 @@ __device__ __forceinline__ void run_scan_group(const uint4* m, const int* seg, i
     if (lane == q && q < n) cnt[q] = count[q];
 }
 
-template <bool MIXED, int G>
-__global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A) {
+template <bool MIXED, int G, int NW>
+__global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
   using R = typename std::conditional<MIXED, float, double>::type;
   using Sum = typename std::conditional<MIXED, long long, double>::type;
   extern __shared__ uint4 run_dyn[];
   __shared__ RepState rs;
   __shared__ __align__(8) R sF[6 * kMaxTypes * kMaxTypes], sU[6 * kMaxTypes * kMaxTypes];
-  __shared__ int wsum[run_threads(G) / 32];
-  __shared__ int segs[run_threads(G) / 32][36];
-  __shared__ float smax[run_threads(G) / 32];
+  __shared__ int wsum[NW];
+  __shared__ int segs[NW][36];
+  __shared__ float smax[NW];
   __shared__ long long sdq[2];
   __shared__ double sdu[2];
   __shared__ double slack, shift_s;
-  __shared__ int rebuild, slot, abort_s;
+  __shared__ int rebuild, slot, abort_s, n_groups;
+  __shared__ int bn[3];     // the list's cell grid, 0 until this launch has built one
+  __shared__ float near_s;  // renewal: beads that moved further get a new list
   __shared__ unsigned long long seen;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
   // kept in shared memory, as what follows from it: registers are short here
@@ -330,6 +365,8 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
     slot = P.g->trial_slot;
     rebuild = P.g->rebuild;
     abort_s = 0;
+    bn[0] = 0;
+    n_groups = 0;
   }
   if (tid < nb) {
     const int i = b0 + tid;
@@ -433,7 +470,8 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
   int trials = 0, rebuilds = 0;
   for (int s = 0; s < A.steps; ++s) {
     const bool last = s + 1 == A.steps;
-    if (rebuild) {
+    bool far = rebuild == 1 && tid < nb;  // the own bead gets a new list
+    if (rebuild == 1) {
       // ---- exclusive scan of the cell counts, by every CTA for itself
       {
         const int4* counts = reinterpret_cast<const int4*>(A.cnt + me.cnt + (size_t)((s + 1) & 1) * ncell4);
@@ -509,58 +547,78 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
         ref[tid] = P.m4[cur][i];
       }
       if (tid == 0) {
+        for (int d = 0; d < 3; ++d) bn[d] = rs.ncell[d];
         slack = 0.0;
         ++rebuilds;
       }
       __syncthreads();
-      // ---- lists: a warp takes two neighbouring beads at a time, or one where that leaves warps idle
-      if (tid < nb) key[tid] = cell_of(ref[tid]);
-      __syncthreads();
+      // ---- lists: a warp takes up to four neighbouring beads of one cell at a time,
+      // fewer where that leaves warps idle
+      const bool offset = rs.ncell[0] >= 5 && rs.ncell[1] >= 5 && rs.ncell[2] >= 5;
+      int* const groups = reinterpret_cast<int*>(fsum);  // first bead and size (free until the force pass)
       {
-        // 1e-5 of the cut: more than the rounding of run_scan_group's squares (offsets
-        // stay within 4.2 cuts); plain form: + the mirror's resolution
-        const float lcut = MIXED ? T.list_cut_f * (1.f + 1e-5f) + 1e-4f
-                                 : T.list_cut_f * (1.f + 1e-5f) + 1e-4f +
-                                       4.f * fmaxf(rs.len_per_frac[0], fmaxf(rs.len_per_frac[1], rs.len_per_frac[2]));
+        const int most = nb <= nw ? 1 : (nb <= 2 * nw || !offset ? 2 : 4);
+        int n = 0, c = 0;
+        if (tid < nb) {
+          const int i = b0 + tid;
+          key[tid] = c = cell_of(ref[tid]);
+          cnt[tid] = 0;
+          const int rank = i - max(rp.bead_begin + starts[c], b0);
+          if (rank % most == 0) n = min(min(most, rp.bead_begin + starts[c + 1] - i), nb - tid);
+        }
+        const unsigned int heads = __ballot_sync(0xffffffffu, n > 0);
+        int at = 0;
+        if (lane == 0 && heads) at = atomicAdd(&n_groups, __popc(heads));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(heads & ((1u << lane) - 1u));
+        if (n > 0) groups[at] = tid | n << 16;
+      }
+    } else if (rebuild == 2) {
+      // ---- a few beads' lists (see the end of the step)
+      far = tid < nb && __int_as_float(cnt[tid]) > near_s;
+      if (far) {
+        cnt[tid] = 0;
+        const uint4 m = P.m4[cur][b0 + tid];
+        key[tid] = (int)__umulhi(m.x, (unsigned)bn[0]) +
+                   bn[0] * ((int)__umulhi(m.y, (unsigned)bn[1]) + bn[1] * (int)__umulhi(m.z, (unsigned)bn[2]));
+      }
+      const unsigned int heads = __ballot_sync(0xffffffffu, far);
+      int at = 0;
+      if (lane == 0 && heads) at = atomicAdd(&n_groups, __popc(heads));
+      at = __shfl_sync(0xffffffffu, at, 0) + __popc(heads & ((1u << lane) - 1u));
+      if (far) reinterpret_cast<int*>(fsum)[at] = tid | 1 << 16;
+    }
+    if (rebuild) {
+      __syncthreads();
+      // rebuild: list_cut, widened by 1e-5 of it, more than the rounding of
+      // run_scan_group's squares (offsets stay within 4.2 cuts); renewal: this
+      // step's range; plain form: + the mirror's resolution
+      {
+        const float range = rebuild == 1 ? T.list_cut_f : T.rcf;
+        const float lcut = range * (1.f + 1e-5f) + 1e-4f +
+                           (MIXED ? 0.f : 4.f * fmaxf(rs.len_per_frac[0], fmaxf(rs.len_per_frac[1], rs.len_per_frac[2])));
         const float lc2 = lcut * lcut;
         const float x0 = rs.len_per_frac[0], x1 = rs.len_per_frac[1], x2 = rs.len_per_frac[2];
-        const bool offset = rs.ncell[0] >= 5 && rs.ncell[1] >= 5 && rs.ncell[2] >= 5;
+        const bool offset = bn[0] >= 5 && bn[1] >= 5 && bn[2] >= 5;
         const uint4* m = P.m4[cur];
-        const int kmax = P.kmax;
+        const int kmax = P.kmax, ng = n_groups;
+        const int* groups = reinterpret_cast<const int*>(fsum);
         int* seg = segs[warp];
-        const int each = nb > nw ? 2 * ((nb + 2 * nw - 1) / (2 * nw)) : 1, end = min((warp + 1) * each, nb);
-        int last_cell = -1, M = 0;
-        for (int q = warp * each; q < end;) {
-          const uint4 ma = ref[q];
-          const int c = key[q];
-          if (c != last_cell) {  // neighbouring beads mostly share it
-            const int n0 = rs.ncell[0], n1 = rs.ncell[1], row = c / n0;
-            M = run_stencil(rs, starts, rp.bead_begin, c - row * n0, row % n1, row / n1, seg);
-            last_cell = c;
-          }
-          const bool pair = q + 1 < end && key[q + 1] == c;
-          const int i = b0 + q;
+        // where there are warps for it, several share a bead's candidates
+        const int parts = max(1, min(8, nw / max(ng, 1)));
+        for (int t = warp; t < ng * parts; t += nw) {
+          const int g = t / parts, q = groups[g] & 0xffff, n = groups[g] >> 16, c = key[q], i = b0 + q;
+          const int row = c / bn[0];
+          const int M = run_stencil(bn, starts, rp.bead_begin, c - row * bn[0], row % bn[1], row / bn[1], seg);
           int* out = P.nbr + (size_t)i * kmax;
-          if (pair && offset) {  // up to four beads at once (the order is by cell)
-            const int n = q + 2 < end && key[q + 2] == c ? (q + 3 < end && key[q + 3] == c ? 4 : 3) : 2;
-            if (n > 2) run_scan_group<4>(m, seg, M, ref + q, n, i, x0, x1, x2, lc2, out, kmax, cnt + q);
-            else run_scan_group<2>(m, seg, M, ref + q, n, i, x0, x1, x2, lc2, out, kmax, cnt + q);
-            q += n;
-            continue;
-          }
-          const uint4 mb = ref[pair ? q + 1 : q];
-          int ca, cb;
-          if (pair) run_scan<true>(m, seg, M, ma, mb, i, x0, x1, x2, lc2, out, kmax, ca, cb);
-          else run_scan<false>(m, seg, M, ma, mb, i, x0, x1, x2, lc2, out, kmax, ca, cb);
-          if (lane == 0) {
-            cnt[q] = ca;
-            if (pair) cnt[q + 1] = cb;
-          }
-          q += pair ? 2 : 1;
+          const uint4 ma = m[i];  // (in a rebuild also ref)
+          if (n > 2) run_scan_group<4>(m, seg, M, ref + q, n, i, x0, x1, x2, lc2, out, kmax, cnt + q);
+          else if (n == 2 && offset) run_scan_group<2>(m, seg, M, ref + q, n, i, x0, x1, x2, lc2, out, kmax, cnt + q);
+          else if (n == 2) run_scan_pair(m, seg, M, ma, ref[q + 1], i, x0, x1, x2, lc2, out, kmax, cnt + q);
+          else run_scan_part(m, seg, M, ma, i, t - g * parts, parts, x0, x1, x2, lc2, out, kmax, cnt + q);
         }
       }
       __syncthreads();
-      if (tid < nb) {
+      if (far) {
         const int count = cnt[tid];
         P.nnbr[b0 + tid] = min(count, P.kmax);
         if (count > *(volatile int*)&P.g->max_nbr) atomicMax(&P.g->max_nbr, count);
@@ -569,7 +627,8 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
           atomicMax(&P.g->need_nbr, count);
         }
       }
-      for (int c = me.index * nt + tid; c < ncell; c += me.ctas * nt) P.cell_count[rp.cell_begin + c] = 0;
+      if (rebuild == 1)
+        for (int c = me.index * nt + tid; c < ncell; c += me.ctas * nt) P.cell_count[rp.cell_begin + c] = 0;
       __syncthreads();
     }
     // the counts of the step before this one: read above at the latest
@@ -748,6 +807,7 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
       const uint4 mn = make_uint4(to_frac(x[0], rs.frac_per_len[0]), to_frac(x[1], rs.frac_per_len[1]),
                                   to_frac(x[2], rs.frac_per_len[2]), w);
       vmax = displacement(ref[tid], mn.x, mn.y, mn.z, rs);
+      cnt[tid] = __float_as_int(vmax);
       P.m4[cur ^ 1][i] = mn;
       if constexpr (!MIXED) P.d4[cur ^ 1][i] = make_double4(x[0], x[1], x[2], __longlong_as_double((long long)w));
       const int c = cell_of(mn);
@@ -758,18 +818,41 @@ __global__ void __launch_bounds__(run_threads(G), 1) k_run(DevPtrs P, RunArgs A)
     vmax = warp_max(vmax);
     if (lane == 0) smax[warp] = vmax;
     __syncthreads();
-    // ---- arrive: a bead beyond the margin (half the skin less the slack) asks for a rebuild
+    // ---- arrive: a bead beyond the margin (half the skin less the slack) asks for new lists
     unsigned long long inc = 1;
     if (warp == 0) {
       const float bm = warp_max(lane < nw ? smax[lane] : 0.f);
-      if ((double)bm + slack > P.half_skin) inc += 1ull << (40 + 8 * (s % 3));
+      if ((double)bm + slack > P.half_skin) {
+        inc += 1ull << (40 + 8 * (s % 3));
+        if (lane == 0) atomicMax(&A.sync[me.rep].dmax[s % 3], __float_as_uint(bm));
+      }
+      if (me.index == 0 && lane == 0) A.sync[me.rep].dmax[(s + 1) % 3] = 0;  // (read two steps ago)
       if (last && lane == 0 && bm > 0.f) atomicMax(&P.g->dmax_bits, __float_as_uint(bm));
       // the first CTA clears the field of two steps ago (the next step's), which every CTA has read
       if (me.index == 0 && s >= 2) inc -= ((seen >> (40 + 8 * ((s + 1) % 3))) & 0xffull) << (40 + 8 * ((s + 1) % 3));
     }
     if (!barrier(inc)) return;
     if (tid == 0) {
-      rebuild = ((seen >> (40 + 8 * (s % 3))) & 0xffull) != 0;
+      // With D the largest displacement, a pair can have come into range unlisted
+      // only if both its beads moved further than the skin less D.  Displacements
+      // are nearly ballistic, so where D first passes half the skin those are the
+      // fastest few beads: they get lists of their own for one step (a renewal,
+      // from the cells of the last build, which must be wide enough), and the
+      // next step rebuilds.  A build then serves three steps instead of two.  (Not
+      // in a trial's step: its size change brings further pairs into range.)
+      int mode = 0;
+      if (rebuild == 2) {
+        mode = 1;
+      } else if (((seen >> (40 + 8 * (s % 3))) & 0xffull) != 0) {
+        const double D = (double)__uint_as_float(__ldcg(&A.sync[me.rep].dmax[s % 3]));
+        const double near = 2.0 * (P.half_skin - slack) - D;
+        bool renew = !last && !next_trial && bn[0] > 0 && near >= 0.5 * D;
+        for (int d = 0; d < 3; ++d) renew = renew && rs.box[d] >= (D + T.rc + 1e-3) * bn[d];
+        mode = renew ? 2 : 1;
+        near_s = (float)(near - 1e-6);
+      }
+      rebuild = mode;
+      n_groups = 0;
     }
     cur ^= 1;
     ++it;

@@ -50,7 +50,7 @@ def test_mixed_loop_bitwise(built, tmp_path, shape, lipids):
     b = _run(m, False, smd.MIXED, cuts)
     for x, y in zip(a[:3], b[:3]):
         assert np.array_equal(x, y)
-    assert a[3] == b[3] and a[4] == b[4] > 0
+    assert a[3] == b[3] and 0 < a[4] <= b[4]  # (the persistent loop renews single lists in between)
     assert np.array_equal(a[5], b[5])  # the list and state it leaves serve the other calls
     assert a[6] < b[6] / 10
 
