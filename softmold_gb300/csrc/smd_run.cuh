@@ -155,14 +155,9 @@ struct SlotWalk {
   const int* seg;
   int t = 0, off, end;
   __device__ __forceinline__ explicit SlotWalk(const int* s) : seg(s), off(s[0]), end(s[18]) {}
-  // bead of slot min(k0 + lane, M - 1); k0 advances by 32 from call to call
+  // bead of slot min(k0 + lane, M - 1); k0 increases from call to call
   __device__ __forceinline__ int round(int k0, int lane, int M) {
     const int g = min(k0 + lane, M - 1);
-    while (end <= k0) {  // (only where the last round ended with the segment)
-      ++t;
-      off = seg[t];
-      end = seg[18 + t];
-    }
     int o = off;
     while (end < k0 + 32) {
       ++t;
@@ -273,7 +268,7 @@ __device__ __forceinline__ void run_scan_group(const uint4* m, const int* seg, i
     fy[q] = -2.f * y;
     fz[q] = -2.f * z;
     lim[q] = q < n ? lc2 - (x * x + y * y + z * z) : -1e30f;  // past the last bead: no hit
-    count[q] = 0;
+    count[q] = q * kmax;
   }
   SlotWalk walk(seg);
   int j = walk.round(0, lane, M);
@@ -288,12 +283,12 @@ __device__ __forceinline__ void run_scan_group(const uint4* m, const int* seg, i
     }
 #pragma unroll
     for (int q = 0; q < Q; ++q)
-      keep_hits(fmaf(fz[q], cz, fmaf(fy[q], cy, fmaf(fx[q], cx, cc))), lim[q], jc - ia, q, below, jc, out + q * kmax,
-                kmax, count[q]);
+      keep_hits(fmaf(fz[q], cz, fmaf(fy[q], cy, fmaf(fx[q], cx, cc))), lim[q], jc - ia, q, below, jc, out,
+                (q + 1) * kmax, count[q]);
   }
 #pragma unroll
   for (int q = 0; q < Q; ++q)
-    if (lane == q && q < n) cnt[q] = count[q];
+    if (lane == q && q < n) cnt[q] = count[q] - q * kmax;
 }
 
 template <bool MIXED, int G, int NW>
