@@ -41,11 +41,27 @@ struct Sum2 {
     lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
     hi = s;
   }
+  __device__ __forceinline__ void add(const Sum2& o) {
+    add(o.hi);
+    lo = __fadd_rn(lo, o.lo);
+  }
+  __device__ __forceinline__ Sum2 from(int x) const {  // lane lane ^ x's
+    Sum2 o;
+    o.hi = __shfl_xor_sync(0xffffffffu, hi, x);
+    o.lo = __shfl_xor_sync(0xffffffffu, lo, x);
+    return o;
+  }
   __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
 struct Sum1 {  // the plain form's sums
   double v = 0.0;
   __device__ __forceinline__ void add(double x) { v += x; }
+  __device__ __forceinline__ void add(const Sum1& o) { v += o.v; }
+  __device__ __forceinline__ Sum1 from(int x) const {
+    Sum1 o;
+    o.v = __shfl_xor_sync(0xffffffffu, v, x);
+    return o;
+  }
   __device__ __forceinline__ double value() const { return v; }
 };
 
@@ -202,132 +218,173 @@ __global__ void __launch_bounds__(kBlock) k_adj_wsort(DevPtrs P, const double* w
     ws[i] = make_double4(w[3 * o], w[3 * o + 1], w[3 * o + 2], 0.0);
 }
 
+// Adds v to *dst once per CTA, where any lane of it has a part: one address
+// takes one atomic after another, 2-3 ns each.  Called by the whole CTA, N
+// quantities at once.
+template <int N>
+__device__ __forceinline__ void adj_add(const double (&v)[N], double* const (&dst)[N]) {
+  __shared__ double part[N][kBlock / 32];
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double x = warp_sum(v[k]);
+    if ((threadIdx.x & 31) == 0) part[k][threadIdx.x >> 5] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x < N) {
+    double x = 0.0;
+    for (int u = 0; u < kBlock / 32; ++u) x += part[threadIdx.x][u];
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (threadIdx.x == k && x != 0.0) atomicAdd(dst[k], x);
+  }
+}
+
 // Pair part of step n: for bead i the non-bonded force F_i, (K w)_i, and the
-// replica sums of U, dU/dUmin and w_i . dF_i/dUmin.  G lanes per bead walk
-// the Verlet list as k_force does.  The mixed form's sums are Sum2: 39 us per
-// pass at 15,000 beads against 92 with each term converted and added in FP64.
-template <bool MIXED, int G>
+// replica sums of U, dU/dUmin and w_i . dF_i/dUmin.  Eight lanes per bead walk
+// the Verlet list in stretches of kPairQueue entries: they first queue the
+// entries in range (about half) by a cheap FP32 test with a slightly wider cut,
+// then take the terms of full groups of queued entries.  The mixed form's sums
+// are Sum2, and the eight sums of a bead end on one lane each by a butterfly
+// that halves what every lane still carries.  At 15,000 beads, per pass: each
+// term converted and added in FP64 92 us, Sum2 39, with the queue, the
+// butterfly and one atomic per CTA 28.
+template <bool MIXED>
 __global__ void __launch_bounds__(kBlock) k_adj_pair(DevPtrs P, int cur, const AdjTables* AT,
                                                      const typename std::conditional<MIXED, float4, double4>::type* ws,
                                                      double* kw, double* fpair, AdjAcc* acc, double dt, double invT) {
+  constexpr int G = 8;
   using R = typename std::conditional<MIXED, float, double>::type;
-  const Tables& T = *P.tab;
-  const int t = blockIdx.x * kBlock + threadIdx.x;
-  const int i = t / G, sub = t % G;
-  const bool active = i < P.n;
   using Sum = typename std::conditional<MIXED, Sum2, Sum1>::type;
-  Sum sF[3], sK[3], su, sut, swft;
-  if (active) {
-    const RepState& rs = P.rs[rep_of(P, i)];
-    const int nn = P.nnbr[i];
-    const int* nb = P.nbr + (size_t)i * P.kmax;
-    const auto wi = ws[i];
-    int ti;
-    R mx, my, mz;
-    uint4 mu = make_uint4(0, 0, 0, 0);
+  __shared__ R tabs[4][6 * kMaxTypes * kMaxTypes];  // F, U and their Umin derivatives
+  __shared__ int queues[kBlock / G][kPairQueue];
+  const Tables& T = *P.tab;
+  for (int k = threadIdx.x; k < 6 * T.nT * T.nT; k += kBlock) {
     if constexpr (MIXED) {
-      mu = P.m4[cur][i];
-      ti = mu.w & 0xff;
+      tabs[0][k] = T.fF[k];
+      tabs[1][k] = T.fU[k];
+      tabs[2][k] = AT->fF[k];
+      tabs[3][k] = AT->fU[k];
     } else {
+      tabs[0][k] = T.dF[k];
+      tabs[1][k] = T.dU[k];
+      tabs[2][k] = AT->dF[k];
+      tabs[3][k] = AT->dU[k];
+    }
+  }
+  __syncthreads();
+  const int t = blockIdx.x * kBlock + threadIdx.x;
+  const int sub = t % G, lane = threadIdx.x & 31;
+  const bool active = t / G < P.n;
+  const int i = active ? t / G : 0, nn = active ? P.nnbr[i] : 0;
+  const unsigned int below = (1u << lane) - 1u, mine = 0xffu << (lane & ~(G - 1));
+  Sum S[8], swft;  // F, K w, U and dU/dUmin (each pair's from both its beads)
+  {
+    const RepState& rs = P.rs[rep_of(P, i)];
+    const int* nb = P.nbr + (size_t)i * P.kmax;
+    int* queue = queues[threadIdx.x / G];
+    const auto wi = ws[i];
+    const uint4 mu = P.m4[cur][i];
+    R mx = 0, my = 0, mz = 0;
+    if constexpr (!MIXED) {
       const double4 me = P.d4[cur][i];
-      ti = __double_as_longlong(me.w) & 0xff;
       mx = me.x;
       my = me.y;
       mz = me.z;
     }
-    const R* rowF;
-    const R* rowU;
-    const R* rowFt;
-    const R* rowUt;
-    if constexpr (MIXED) {
-      rowF = T.fF + 6 * ti * T.nT;
-      rowU = T.fU + 6 * ti * T.nT;
-      rowFt = AT->fF + 6 * ti * T.nT;
-      rowUt = AT->fU + 6 * ti * T.nT;
-    } else {
-      rowF = T.dF + 6 * ti * T.nT;
-      rowU = T.dU + 6 * ti * T.nT;
-      rowFt = AT->dF + 6 * ti * T.nT;
-      rowUt = AT->dU + 6 * ti * T.nT;
-    }
+    const int row = 6 * (mu.w & 0xff) * T.nT;
     const R rc2 = MIXED ? (R)T.rc2f : (R)T.rc2;
-    for (int k = sub; k < nn; k += G) {
-      const int j = __ldg(nb + k);
-      R dx, dy, dz;
-      int tj;
-      if constexpr (MIXED) {
+    const float s0 = rs.len_per_frac[0], s1 = rs.len_per_frac[1], s2 = rs.len_per_frac[2];
+    const float cut = T.rcf * (1.f + 4e-6f) + 4.f * fmaxf(s0, fmaxf(s1, s2)), cut2 = cut * cut;
+    const int longest = __reduce_max_sync(0xffffffffu, nn);
+    for (int base = 0; base < longest; base += kPairQueue) {
+      const int end = min(kPairQueue, longest - base);
+      int queued = 0;
+#pragma unroll 4
+      for (int k0 = 0; k0 < end; k0 += G) {
+        const int k = base + k0 + sub;
+        bool near = false;
+        int j = 0;
+        if (k < nn) {
+          j = __ldg(nb + k);
+          const uint4 o = P.m4[cur][j];
+          const float dx = frac_delta(mu.x, o.x, s0), dy = frac_delta(mu.y, o.y, s1), dz = frac_delta(mu.z, o.z, s2);
+          near = dx * dx + dy * dy + dz * dz < cut2;
+        }
+        const unsigned int hits = __ballot_sync(0xffffffffu, near) & mine;
+        if (near) queue[queued + __popc(hits & below)] = j;
+        queued += __popc(hits);
+      }
+      __syncwarp();
+      for (int k = sub; k < queued; k += G) {
+        const int j = queue[k];
+        R dx, dy, dz;
         const uint4 o = P.m4[cur][j];
-        tj = o.w & 0xff;
-        dx = frac_delta(mu.x, o.x, rs.len_per_frac[0]);
-        dy = frac_delta(mu.y, o.y, rs.len_per_frac[1]);
-        dz = frac_delta(mu.z, o.z, rs.len_per_frac[2]);
-      } else {
-        const double4 o = P.d4[cur][j];
-        tj = __double_as_longlong(o.w) & 0xff;
-        double ox = o.x, oy = o.y, oz = o.z;
-        if (mx - ox > rs.box[0] / 2.0) ox += rs.box[0];
-        if (mx - ox < -rs.box[0] / 2.0) ox -= rs.box[0];
-        if (my - oy > rs.box[1] / 2.0) oy += rs.box[1];
-        if (my - oy < -rs.box[1] / 2.0) oy -= rs.box[1];
-        if (mz - oz > rs.box[2] / 2.0) oz += rs.box[2];
-        if (mz - oz < -rs.box[2] / 2.0) oz -= rs.box[2];
-        dx = mx - ox;
-        dy = my - oy;
-        dz = mz - oz;
+        const int tj = o.w & 0xff;
+        if constexpr (MIXED) {
+          dx = frac_delta(mu.x, o.x, s0);
+          dy = frac_delta(mu.y, o.y, s1);
+          dz = frac_delta(mu.z, o.z, s2);
+        } else {
+          const double4 e = P.d4[cur][j];
+          double ox = e.x, oy = e.y, oz = e.z;
+          if (mx - ox > rs.box[0] / 2.0) ox += rs.box[0];
+          if (mx - ox < -rs.box[0] / 2.0) ox -= rs.box[0];
+          if (my - oy > rs.box[1] / 2.0) oy += rs.box[1];
+          if (my - oy < -rs.box[1] / 2.0) oy -= rs.box[1];
+          if (mz - oz > rs.box[2] / 2.0) oz += rs.box[2];
+          if (mz - oz < -rs.box[2] / 2.0) oz -= rs.box[2];
+          dx = mx - ox;
+          dy = my - oy;
+          dz = mz - oz;
+        }
+        const R r2 = dx * dx + dy * dy + dz * dz;
+        if (!(r2 < rc2)) continue;
+        const R rr = ::sqrt(r2);
+        const R* c = tabs[0] + row + 6 * tj;
+        const int ci = (rr >= c[0]) ? 3 : 0;
+        const R m = c[ci] - rr;
+        const R g = ((c[ci + 1] - c[ci + 2] * m) * m) / rr;
+        // g'(r)/r = -((C1 - 2 C2 m) + g) / r^2
+        const R q = -((c[ci + 1] - (R)2 * c[ci + 2] * m) + g) / r2;
+        const auto wj = ws[j];
+        const R ex = (R)wi.x - (R)wj.x, ey = (R)wi.y - (R)wj.y, ez = (R)wi.z - (R)wj.z;
+        const R dd = q * (dx * ex + dy * ey + dz * ez);
+        S[0].add(g * dx);
+        S[1].add(g * dy);
+        S[2].add(g * dz);
+        S[3].add(g * ex + dd * dx);
+        S[4].add(g * ey + dd * dy);
+        S[5].add(g * ez + dd * dz);
+        S[6].add((R)0.5 * pair_pot<R>(tabs[1] + row + 6 * tj, rr));
+        const R* ct = tabs[2] + row + 6 * tj;
+        if (ct[1] != (R)0 || ct[4] != (R)0) {
+          const R mt = ct[ci] - rr;
+          const R gt = ((ct[ci + 1] - ct[ci + 2] * mt) * mt) / rr;
+          swft.add(gt * (dx * (R)wi.x + dy * (R)wi.y + dz * (R)wi.z));
+          S[7].add((R)0.5 * pair_pot<R>(tabs[3] + row + 6 * tj, rr));
+        }
       }
-      const R r2 = dx * dx + dy * dy + dz * dz;
-      if (!(r2 < rc2)) continue;
-      const R rr = ::sqrt(r2);
-      const R* c = rowF + 6 * tj;
-      const int ci = (rr >= c[0]) ? 3 : 0;
-      const R m = c[ci] - rr;
-      const R g = ((c[ci + 1] - c[ci + 2] * m) * m) / rr;
-      // g'(r)/r = -((C1 - 2 C2 m) + g) / r^2
-      const R q = -((c[ci + 1] - (R)2 * c[ci + 2] * m) + g) / r2;
-      const auto wj = ws[j];
-      const R ex = (R)wi.x - (R)wj.x, ey = (R)wi.y - (R)wj.y, ez = (R)wi.z - (R)wj.z;
-      const R dd = q * (dx * ex + dy * ey + dz * ez);
-      sF[0].add(g * dx);
-      sF[1].add(g * dy);
-      sF[2].add(g * dz);
-      sK[0].add(g * ex + dd * dx);
-      sK[1].add(g * ey + dd * dy);
-      sK[2].add(g * ez + dd * dz);
-      su.add((R)0.5 * pair_pot<R>(rowU + 6 * tj, rr));
-      const R* ct = rowFt + 6 * tj;
-      if (ct[1] != (R)0 || ct[4] != (R)0) {
-        const R mt = ct[ci] - rr;
-        const R gt = ((ct[ci + 1] - ct[ci + 2] * mt) * mt) / rr;
-        swft.add(gt * (dx * (R)wi.x + dy * (R)wi.y + dz * (R)wi.z));
-        sut.add((R)0.5 * pair_pot<R>(rowUt + 6 * tj, rr));
-      }
+      __syncwarp();
     }
   }
-  double F[3], K[3];
-  for (int d = 0; d < 3; ++d) {
-    F[d] = sF[d].value();
-    K[d] = sK[d].value();
-  }
+  // lane sub ends with the group's sum of S[sub]
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) {
-    for (int d = 0; d < 3; ++d) {
-      F[d] += __shfl_xor_sync(0xffffffffu, F[d], o);
-      K[d] += __shfl_xor_sync(0xffffffffu, K[d], o);
+    const bool upper = (sub & o) != 0;
+#pragma unroll
+    for (int k = 0; k < o; ++k) {
+      const Sum give = upper ? S[k] : S[k + o];
+      Sum keep = upper ? S[k + o] : S[k];
+      keep.add(give.from(o));
+      S[k] = keep;
     }
+    swft.add(swft.from(o));
   }
-  if (active && sub == 0) {
-    for (int d = 0; d < 3; ++d) {
-      kw[i + d * P.n] = K[d];
-      fpair[i + d * P.n] = F[d];
-    }
-  }
+  const double mysum = S[0].value();
+  if (active && sub < 6) (sub < 3 ? fpair : kw)[i + (sub % 3) * P.n] = mysum;
   // replica sums (single-system handles): J and the Umin component
-  const double gJ = invT * su.value(), g0 = dt * swft.value() + invT * sut.value();
-  const double sJ = warp_sum(gJ), s0 = warp_sum(g0);
-  if ((threadIdx.x & 31) == 0) {
-    if (sJ != 0.0) atomicAdd(&acc->J, sJ);
-    if (s0 != 0.0) atomicAdd(&acc->grad[0], s0);
-  }
+  const double gJ = sub == 6 ? invT * mysum : 0.0, g0 = sub == 7 ? dt * swft.value() + invT * mysum : 0.0;
+  adj_add<2>({gJ, g0}, {&acc->J, &acc->grad[0]});
 }
 
 // Differences of w along the chain of file-order bead o (file order is chain
@@ -387,14 +444,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_chain(DevPtrs P, int cur, const 
       w_next[3 * o + d] = hb + dt * xb;
     }
   }
-  gJ = warp_sum(gJ);
-  g1 = warp_sum(g1);
-  g2 = warp_sum(g2);
-  if ((threadIdx.x & 31) == 0) {
-    if (gJ != 0.0) atomicAdd(&acc->J, gJ);
-    if (g1 != 0.0) atomicAdd(&acc->grad[1], g1);
-    if (g2 != 0.0) atomicAdd(&acc->grad[2], g2);
-  }
+  adj_add<3>({gJ, g1, g2}, {&acc->J, &acc->grad[1], &acc->grad[2]});
 }
 
 // (K w)_i of the full conservative force at the current positions, file

@@ -1936,11 +1936,11 @@ int adj_pair_pass(smd_system* h, const double* w, double dt, double invT) {
   if (h->mixed) {
     float4* ws = reinterpret_cast<float4*>(A.ws);
     SMD_LAUNCH(h, k_adj_wsort<float4><<<g, kBlock, 0, h->stream>>>(P, w, ws));
-    SMD_LAUNCH(h, (k_adj_pair<true, kLanes><<<gl, kBlock, 0, h->stream>>>(P, h->cur, A.tab, ws, A.kw, A.fpair,
+    SMD_LAUNCH(h, (k_adj_pair<true><<<gl, kBlock, 0, h->stream>>>(P, h->cur, A.tab, ws, A.kw, A.fpair,
                                                                             A.acc, dt, invT)));
   } else {
     SMD_LAUNCH(h, k_adj_wsort<double4><<<g, kBlock, 0, h->stream>>>(P, w, A.ws));
-    SMD_LAUNCH(h, (k_adj_pair<false, kLanes><<<gl, kBlock, 0, h->stream>>>(P, h->cur, A.tab, A.ws, A.kw,
+    SMD_LAUNCH(h, (k_adj_pair<false><<<gl, kBlock, 0, h->stream>>>(P, h->cur, A.tab, A.ws, A.kw,
                                                                              A.fpair, A.acc, dt, invT)));
   }
   return 0;

@@ -1086,23 +1086,48 @@ __device__ __forceinline__ Vec3<RT> term_vec(const DevPtrs& P, int cur, int a, i
   }
 }
 
-// Sum of v over the lanes that belong to the same replica, one atomic per
-// replica present in the warp.  Called by the whole warp.
-__device__ __forceinline__ void warp_atomic_add(double v, double* dst, int r) {
-  const unsigned int peers = __match_any_sync(0xffffffffu, r);
+// Sums over the beads of each replica, of N quantities at once: v[k] to the
+// word w[k] of replica r's state.  A batch adds per warp and replica, a single
+// system per CTA: the sums go to one address each, whose atomics the L2 takes
+// one after another.  (One atomic per warp, after 32 dependent additions, made
+// the pair energies of 29,400 beads take 29 us; so they take 16.)
+// Called by the whole CTA.
+template <int NT, int N, typename V>
+__device__ __forceinline__ void replica_add(const DevPtrs& P, const V (&v)[N], V RepState::*const (&w)[N], int r) {
+  using U = typename std::conditional<std::is_same<V, long long>::value, unsigned long long, double>::type;
   const int lane = threadIdx.x & 31;
-  double acc = 0.0;
-  for (unsigned int rest = peers; rest; rest &= rest - 1) acc += __shfl_sync(peers, v, __ffs(rest) - 1);
-  if (lane == __ffs(peers) - 1 && acc != 0.0) atomicAdd(dst, acc);
-}
-
-__device__ __forceinline__ void warp_atomic_add_q(long long v, long long* dst, int r) {
-  const unsigned int peers = __match_any_sync(0xffffffffu, r);
-  const int lane = threadIdx.x & 31;
-  long long acc = 0;
-  for (unsigned int rest = peers; rest; rest &= rest - 1) acc += __shfl_sync(peers, v, __ffs(rest) - 1);
-  if (lane == __ffs(peers) - 1 && acc != 0)
-    atomicAdd((unsigned long long*)dst, (unsigned long long)acc);
+  auto tree = [](V x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+  };
+  if (P.n_rep > 1) {
+    const unsigned int peers = __match_any_sync(0xffffffffu, r);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      V acc = 0;
+      if (peers == 0xffffffffu) acc = tree(v[k]);
+      else
+        for (unsigned int rest = peers; rest; rest &= rest - 1) acc += __shfl_sync(peers, v[k], __ffs(rest) - 1);
+      if (lane == __ffs(peers) - 1 && acc != 0) atomicAdd((U*)&(P.rs[r].*w[k]), (U)acc);
+    }
+    return;
+  }
+  __shared__ V part[N][NT / 32];
+  __syncthreads();  // (an earlier call's part has been read)
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const V x = tree(v[k]);
+    if (lane == 0) part[k][threadIdx.x >> 5] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x < N) {
+    V acc = 0;
+    for (int u = 0; u < NT / 32; ++u) acc += part[threadIdx.x][u];
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (threadIdx.x == k && acc != 0) atomicAdd((U*)&(P.rs[0].*w[k]), (U)acc);
+  }
 }
 
 // Hash-cell counts of the reference's many-sphere branches for the current
@@ -2021,10 +2046,10 @@ __global__ void __launch_bounds__(kBlock, (MIXED && (FL & F_DU) != 0) ? 4 : 0) k
     }
   }
   if constexpr ((FL & F_DU) != 0) {
-    if constexpr (MIXED) warp_atomic_add_q(dq, &P.rs[r].dUq_pair, r);
-    else warp_atomic_add(dU, &P.rs[r].dU_pair, r);
+    if constexpr (MIXED) replica_add<kBlock, 1, long long>(P, {dq}, {&RepState::dUq_pair}, r);
+    else replica_add<kBlock, 1, double>(P, {dU}, {&RepState::dU_pair}, r);
   }
-  if constexpr ((FL & F_ENERGY) != 0) warp_atomic_add(ep, &P.rs[r].e_pair, r);
+  if constexpr ((FL & F_ENERGY) != 0) replica_add<kBlock, 1, double>(P, {ep}, {&RepState::e_pair}, r);
 }
 
 // Per-bead pass after k_force: CHAIN terms, the total force, the Langevin
@@ -2203,13 +2228,14 @@ __global__ void __launch_bounds__(kBeadBlock) k_integ(DevPtrs P, int cur, StepEn
   if (active) integ_bead<MIXED, FL>(P, cur, i, r, it, fs, dU_bond, e_bond, e_kin, vmax);
   pdl_wait();  // returns at once where integ_bead has waited
   if constexpr ((FL & F_DU) != 0) {
-    if constexpr (MIXED) warp_atomic_add_q(__double2ll_rn(dU_bond * 4294967296.0), &P.rs[r].dUq_bond, r);
-    else warp_atomic_add(dU_bond, &P.rs[r].dU_bond, r);
+    if constexpr (MIXED)
+      replica_add<kBeadBlock, 1, long long>(P, {__double2ll_rn(dU_bond * 4294967296.0)}, {&RepState::dUq_bond}, r);
+    else
+      replica_add<kBeadBlock, 1, double>(P, {dU_bond}, {&RepState::dU_bond}, r);
   }
   if constexpr ((FL & F_ENERGY) != 0) {
-    warp_atomic_add(e_bond, &P.rs[r].e_bond, r);
-    warp_atomic_add(e_kin, &P.rs[r].e_kin, r);
-    if (P.n_sph > 0) warp_atomic_add(e_sph, &P.rs[r].e_sphere, r);
+    replica_add<kBeadBlock, 3, double>(P, {e_bond, e_kin, e_sph},
+                                       {&RepState::e_bond, &RepState::e_kin, &RepState::e_sphere}, r);
   }
   if constexpr ((FL & (F_STOP | F_INIT | F_FORCES | F_ENERGY)) == 0) {
     vmax = warp_max(vmax);
