@@ -123,6 +123,7 @@ struct smd_system {
     size_t smem = 0;
     int* cnt = nullptr;
     RunSync* sync = nullptr;
+    RunTrial* trial = nullptr;
     RunPlace* place = nullptr;
   } run;
   // launch configuration chosen by the autotuner (mixed form): lanes per bead
@@ -456,7 +457,7 @@ int launch_run(smd_system* h, RunArgs a) {
 // `steps` loop iterations (barostat trials included) in one persistent kernel.
 int advance_run(smd_system* h, int steps) {
   const auto& r = h->run;
-  const RunArgs a{h->it, h->cur, steps, h->resize_rate, h->barostat ? 1 : 0, r.beads, r.cnt, r.sync, r.place};
+  const RunArgs a{h->it, h->cur, steps, h->resize_rate, h->barostat ? 1 : 0, r.beads, r.cnt, r.sync, r.trial, r.place};
   const int rc = SMD_RUN_VARIANT(h, launch_run, h, a);
   if (rc) return rc;
   for (int k = 0; k < steps; ++k)
@@ -532,7 +533,8 @@ int run_setup(smd_system* h) {
   rc = SMD_RUN_VARIANT(h, run_fits_device, h, &fits);
   r.grid = 0;
   if (rc || !fits) return rc;
-  if ((rc = h->alloc(&r.cnt, (size_t)cnt)) || (rc = h->alloc(&r.sync, (size_t)h->n_rep)) ||
+  if ((rc = h->alloc(&r.cnt, (size_t)cnt)) || (rc = h->alloc(&r.sync, 1)) ||
+      (rc = h->alloc(&r.trial, (size_t)h->n_rep)) ||
       (rc = h->alloc(&r.place, place.size())))
     return rc;
   SMD_CUDA(cudaMemcpyAsync(r.place, place.data(), place.size() * sizeof(RunPlace), cudaMemcpyHostToDevice, h->stream));

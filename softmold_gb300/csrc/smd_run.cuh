@@ -15,8 +15,8 @@
 // and arrives.  A list rebuild adds one barrier (between the reordering and
 // the stencil scans), a barostat trial one (its summed energy difference).
 // Every barrier waits with a limit.  The CTAs of a batch are dealt out to its
-// replicas, which wait for nobody else: each has its own barrier, its own list
-// rebuilds and its own trials.
+// replicas, which share the barriers and, as kernel by kernel, the decision to
+// rebuild.
 //
 // The arithmetic of a step is that of k_force, k_integ, k_mc and k_finish, and
 // the mixed form's sums are exact in any order, so a mixed run has the same
@@ -51,17 +51,21 @@ struct RunPlace {
   int rep, index, ctas, cnt;
 };
 
-// Words shared by a replica's CTAs in the persistent loop (zero between launches).
+// Grid-wide words of the persistent loop (zero between launches).
 struct RunSync {
   // arrivals in the low 40 bits, then three 8-bit counts (by step modulo 3) of
   // the CTAs with a bead beyond the list's margin: they ride on the arrival,
   // so the barrier itself tells whether the list must be rebuilt
   unsigned long long arrive;
-  unsigned int left;             // CTAs of the grid that are done with the kernel (first replica's)
-  int rebuild, rebuilds;         // the replica's list state at the end, for the last of them
-  double slack;
-  unsigned int dmax[3], pad;     // largest displacement (FP32 bits) beyond the margin, by step modulo 3
-  long long dq_pair[2], dq_bond[2];  // trial sums, alternating
+  unsigned int left;             // CTAs that are done with the kernel
+  // of trial steps, alternating: the largest displacement (FP32 bits) and the
+  // largest change of a pair distance by an accepted trial (FP64 bits)
+  unsigned int dmax[2];
+  unsigned long long shift[2];
+};
+// A replica's trial sums, alternating (zero between launches).
+struct RunTrial {
+  long long dq_pair[2], dq_bond[2];
   double du_pair[2], du_bond[2];
 };
 
@@ -73,7 +77,8 @@ struct RunArgs {
   int barostat;
   int beads;      // beads per CTA
   int* cnt;       // 2 x run_cells(cells) cell counts per replica, zero between launches
-  RunSync* sync;  // per replica
+  RunSync* sync;
+  RunTrial* trial;  // per replica
   const RunPlace* place;  // per CTA
 };
 
@@ -305,8 +310,6 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
   __shared__ double sdu[2];
   __shared__ double slack, shift_s;
   __shared__ int rebuild, slot, abort_s, n_groups;
-  __shared__ int bn[3];     // the list's cell grid, 0 until this launch has built one
-  __shared__ float near_s;  // renewal: beads that moved further get a new list
   __shared__ unsigned long long seen;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
   // kept in shared memory, as what follows from it: registers are short here
@@ -360,7 +363,6 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
     slot = P.g->trial_slot;
     rebuild = P.g->rebuild;
     abort_s = 0;
-    bn[0] = 0;
     n_groups = 0;
   }
   if (tid < nb) {
@@ -386,14 +388,14 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
     __syncthreads();
     ++waited;
     if (tid == 0) {
-      const unsigned long long target = waited * me.ctas;
+      const unsigned long long target = waited * gridDim.x;
       // release: the CTA's writes (ordered before by the block barrier) are
       // visible to whoever sees the arrival; the acquire below is its other end
-      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&A.sync[me.rep].arrive), "l"(inc) : "memory");
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&A.sync->arrive), "l"(inc) : "memory");
       unsigned long long v = 0;
       int polls = 0;
       for (;;) {
-        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&A.sync[me.rep].arrive) : "memory");
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&A.sync->arrive) : "memory");
         if ((v & ((1ull << 40) - 1)) >= target) break;
         if (++polls > kRunSpinLimit) {
           atomicOr(&P.g->error, 8);
@@ -465,8 +467,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
   int trials = 0, rebuilds = 0;
   for (int s = 0; s < A.steps; ++s) {
     const bool last = s + 1 == A.steps;
-    bool far = rebuild == 1 && tid < nb;  // the own bead gets a new list
-    if (rebuild == 1) {
+    if (rebuild) {
       // ---- exclusive scan of the cell counts, by every CTA for itself
       {
         const int4* counts = reinterpret_cast<const int4*>(A.cnt + me.cnt + (size_t)((s + 1) & 1) * ncell4);
@@ -542,7 +543,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
         ref[tid] = P.m4[cur][i];
       }
       if (tid == 0) {
-        for (int d = 0; d < 3; ++d) bn[d] = rs.ncell[d];
+        n_groups = 0;
         slack = 0.0;
         ++rebuilds;
       }
@@ -567,45 +568,25 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
         at = __shfl_sync(0xffffffffu, at, 0) + __popc(heads & ((1u << lane) - 1u));
         if (n > 0) groups[at] = tid | n << 16;
       }
-    } else if (rebuild == 2) {
-      // ---- a few beads' lists (see the end of the step)
-      far = tid < nb && __int_as_float(cnt[tid]) > near_s;
-      if (far) {
-        cnt[tid] = 0;
-        const uint4 m = P.m4[cur][b0 + tid];
-        key[tid] = (int)__umulhi(m.x, (unsigned)bn[0]) +
-                   bn[0] * ((int)__umulhi(m.y, (unsigned)bn[1]) + bn[1] * (int)__umulhi(m.z, (unsigned)bn[2]));
-      }
-      const unsigned int heads = __ballot_sync(0xffffffffu, far);
-      int at = 0;
-      if (lane == 0 && heads) at = atomicAdd(&n_groups, __popc(heads));
-      at = __shfl_sync(0xffffffffu, at, 0) + __popc(heads & ((1u << lane) - 1u));
-      if (far) reinterpret_cast<int*>(fsum)[at] = tid | 1 << 16;
-    }
-    if (rebuild) {
       __syncthreads();
-      // rebuild: list_cut, widened by 1e-5 of it, more than the rounding of
-      // run_scan_group's squares (offsets stay within 4.2 cuts); renewal: this
-      // step's range; plain form: + the mirror's resolution
+      // 1e-5 of the cut: more than the rounding of run_scan_group's squares (offsets
+      // stay within 4.2 cuts); plain form: + the mirror's resolution
       {
-        const float range = rebuild == 1 ? T.list_cut_f : T.rcf;
-        const float lcut = range * (1.f + 1e-5f) + 1e-4f +
+        const float lcut = T.list_cut_f * (1.f + 1e-5f) + 1e-4f +
                            (MIXED ? 0.f : 4.f * fmaxf(rs.len_per_frac[0], fmaxf(rs.len_per_frac[1], rs.len_per_frac[2])));
         const float lc2 = lcut * lcut;
         const float x0 = rs.len_per_frac[0], x1 = rs.len_per_frac[1], x2 = rs.len_per_frac[2];
-        const bool offset = bn[0] >= 5 && bn[1] >= 5 && bn[2] >= 5;
         const uint4* m = P.m4[cur];
         const int kmax = P.kmax, ng = n_groups;
-        const int* groups = reinterpret_cast<const int*>(fsum);
         int* seg = segs[warp];
         // where there are warps for it, several share a bead's candidates
         const int parts = max(1, min(8, nw / max(ng, 1)));
         for (int t = warp; t < ng * parts; t += nw) {
           const int g = t / parts, q = groups[g] & 0xffff, n = groups[g] >> 16, c = key[q], i = b0 + q;
-          const int row = c / bn[0];
-          const int M = run_stencil(bn, starts, rp.bead_begin, c - row * bn[0], row % bn[1], row / bn[1], seg);
+          const int n0 = rs.ncell[0], n1 = rs.ncell[1], row = c / n0;
+          const int M = run_stencil(rs.ncell, starts, rp.bead_begin, c - row * n0, row % n1, row / n1, seg);
           int* out = P.nbr + (size_t)i * kmax;
-          const uint4 ma = m[i];  // (in a rebuild also ref)
+          const uint4 ma = ref[q];
           if (n > 2) run_scan_group<4>(m, seg, M, ref + q, n, i, x0, x1, x2, lc2, out, kmax, cnt + q);
           else if (n == 2 && offset) run_scan_group<2>(m, seg, M, ref + q, n, i, x0, x1, x2, lc2, out, kmax, cnt + q);
           else if (n == 2) run_scan_pair(m, seg, M, ma, ref[q + 1], i, x0, x1, x2, lc2, out, kmax, cnt + q);
@@ -613,7 +594,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
         }
       }
       __syncthreads();
-      if (far) {
+      if (tid < nb) {
         const int count = cnt[tid];
         P.nnbr[b0 + tid] = min(count, P.kmax);
         if (count > *(volatile int*)&P.g->max_nbr) atomicMax(&P.g->max_nbr, count);
@@ -622,8 +603,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
           atomicMax(&P.g->need_nbr, count);
         }
       }
-      if (rebuild == 1)
-        for (int c = me.index * nt + tid; c < ncell; c += me.ctas * nt) P.cell_count[rp.cell_begin + c] = 0;
+      for (int c = me.index * nt + tid; c < ncell; c += me.ctas * nt) P.cell_count[rp.cell_begin + c] = 0;
       __syncthreads();
     }
     // the counts of the step before this one: read above at the latest
@@ -753,30 +733,37 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
       const int par = trials & 1;
       if (tid == 0) {
         if constexpr (MIXED) {
-          atomicAdd((unsigned long long*)&A.sync[me.rep].dq_pair[par], (unsigned long long)sdq[0]);
-          atomicAdd((unsigned long long*)&A.sync[me.rep].dq_bond[par], (unsigned long long)sdq[1]);
+          atomicAdd((unsigned long long*)&A.trial[me.rep].dq_pair[par], (unsigned long long)sdq[0]);
+          atomicAdd((unsigned long long*)&A.trial[me.rep].dq_bond[par], (unsigned long long)sdq[1]);
         } else {
-          atomicAdd(&A.sync[me.rep].du_pair[par], sdu[0]);
-          atomicAdd(&A.sync[me.rep].du_bond[par], sdu[1]);
+          atomicAdd(&A.trial[me.rep].du_pair[par], sdu[0]);
+          atomicAdd(&A.trial[me.rep].du_bond[par], sdu[1]);
         }
-        if (me.index == 0) {  // the previous trial's sums: every CTA has read them
-          A.sync[me.rep].dq_pair[par ^ 1] = A.sync[me.rep].dq_bond[par ^ 1] = 0;
-          A.sync[me.rep].du_pair[par ^ 1] = A.sync[me.rep].du_bond[par ^ 1] = 0.0;
+        if (blockIdx.x == 0) {
+          A.sync->dmax[par ^ 1] = 0;
+          A.sync->shift[par ^ 1] = 0;
+        }
+        if (me.index == 0) {  // the previous trial's words: every CTA has read them
+          A.trial[me.rep].dq_pair[par ^ 1] = A.trial[me.rep].dq_bond[par ^ 1] = 0;
+          A.trial[me.rep].du_pair[par ^ 1] = A.trial[me.rep].du_bond[par ^ 1] = 0.0;
         }
       }
       if (!barrier(1)) return;
       if (tid == 0) {
-        rs.dUq_pair = __ldcg(&A.sync[me.rep].dq_pair[par]);
-        rs.dUq_bond = __ldcg(&A.sync[me.rep].dq_bond[par]);
-        rs.dU_pair = __ldcg(&A.sync[me.rep].du_pair[par]);
-        rs.dU_bond = __ldcg(&A.sync[me.rep].du_bond[par]);
+        rs.dUq_pair = __ldcg(&A.trial[me.rep].dq_pair[par]);
+        rs.dUq_bond = __ldcg(&A.trial[me.rep].dq_bond[par]);
+        rs.dU_pair = __ldcg(&A.trial[me.rep].du_pair[par]);
+        rs.dU_bond = __ldcg(&A.trial[me.rep].du_bond[par]);
         rs.accept = 0;
         shift_s = 0.0;
         if (rp.dlxy != 0) {
           shift_s = decide_trial(rs, rp, T, P.trial_u[((size_t)slot * P.n_rep + me.rep) * 2 + 1]);
-          if (me.index == 0) P.accept_log[(size_t)slot * P.n_rep + me.rep] = rs.accept;
+          if (me.index == 0) {
+            P.accept_log[(size_t)slot * P.n_rep + me.rep] = rs.accept;
+            if (rs.accept)
+              atomicMax(&A.sync->shift[par], (unsigned long long)__double_as_longlong(shift_s));
+          }
         }
-        slack += shift_s;
         ++slot;
       }
       __syncthreads();
@@ -802,7 +789,6 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
       const uint4 mn = make_uint4(to_frac(x[0], rs.frac_per_len[0]), to_frac(x[1], rs.frac_per_len[1]),
                                   to_frac(x[2], rs.frac_per_len[2]), w);
       vmax = displacement(ref[tid], mn.x, mn.y, mn.z, rs);
-      cnt[tid] = __float_as_int(vmax);
       P.m4[cur ^ 1][i] = mn;
       if constexpr (!MIXED) P.d4[cur ^ 1][i] = make_double4(x[0], x[1], x[2], __longlong_as_double((long long)w));
       const int c = cell_of(mn);
@@ -817,37 +803,24 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
     unsigned long long inc = 1;
     if (warp == 0) {
       const float bm = warp_max(lane < nw ? smax[lane] : 0.f);
-      if ((double)bm + slack > P.half_skin) {
+      if (trial) {  // (the slack is not known yet)
+        if (lane == 0 && bm > 0.f) atomicMax(&A.sync->dmax[(trials - 1) & 1], __float_as_uint(bm));
+      } else if ((double)bm + slack > P.half_skin) {
         inc += 1ull << (40 + 8 * (s % 3));
-        if (lane == 0) atomicMax(&A.sync[me.rep].dmax[s % 3], __float_as_uint(bm));
       }
-      if (me.index == 0 && lane == 0) A.sync[me.rep].dmax[(s + 1) % 3] = 0;  // (read two steps ago)
       if (last && lane == 0 && bm > 0.f) atomicMax(&P.g->dmax_bits, __float_as_uint(bm));
       // the first CTA clears the field of two steps ago (the next step's), which every CTA has read
-      if (me.index == 0 && s >= 2) inc -= ((seen >> (40 + 8 * ((s + 1) % 3))) & 0xffull) << (40 + 8 * ((s + 1) % 3));
+      if (blockIdx.x == 0 && s >= 2) inc -= ((seen >> (40 + 8 * ((s + 1) % 3))) & 0xffull) << (40 + 8 * ((s + 1) % 3));
     }
     if (!barrier(inc)) return;
     if (tid == 0) {
-      // With D the largest displacement, a pair can have come into range unlisted
-      // only if both its beads moved further than the skin less D.  Displacements
-      // are nearly ballistic, so where D first passes half the skin those are the
-      // fastest few beads: they get lists of their own for one step (a renewal,
-      // from the cells of the last build, which must be wide enough), and the
-      // next step rebuilds.  A build then serves three steps instead of two.  (Not
-      // in a trial's step: its size change brings further pairs into range.)
-      int mode = 0;
-      if (rebuild == 2) {
-        mode = 1;
-      } else if (((seen >> (40 + 8 * (s % 3))) & 0xffull) != 0) {
-        const double D = (double)__uint_as_float(__ldcg(&A.sync[me.rep].dmax[s % 3]));
-        const double near = 2.0 * (P.half_skin - slack) - D;
-        bool renew = !last && !next_trial && bn[0] > 0 && near >= 0.5 * D;
-        for (int d = 0; d < 3; ++d) renew = renew && rs.box[d] >= (D + T.rc + 1e-3) * bn[d];
-        mode = renew ? 2 : 1;
-        near_s = (float)(near - 1e-6);
+      if (trial) {
+        const int par = (trials - 1) & 1;
+        slack += __longlong_as_double((long long)__ldcg(&A.sync->shift[par]));
+        rebuild = (double)__uint_as_float(__ldcg(&A.sync->dmax[par])) + slack > P.half_skin;
+      } else {
+        rebuild = ((seen >> (40 + 8 * (s % 3))) & 0xffull) != 0;
       }
-      rebuild = mode;
-      n_groups = 0;
     }
     cur ^= 1;
     ++it;
@@ -876,30 +849,17 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
   if (me.index == 0) {
     for (int k = tid; k < (int)(sizeof(RepState) / 4); k += nt)
       reinterpret_cast<int*>(P.rs + me.rep)[k] = reinterpret_cast<const int*>(&rs)[k];
-    if (tid == 0) {
-      RunSync& y = A.sync[me.rep];
-      y.slack = slack;
-      y.rebuild = rebuild;
-      y.rebuilds = rebuilds;
-    }
   }
   __syncthreads();
   if (tid == 0) {
     __threadfence();
     if (atomicAdd(&A.sync->left, 1u) == gridDim.x - 1) {  // every CTA has passed its last barrier
       __threadfence();
-      double most = 0.0;
-      int any = 0, count = 0;
-      for (int r = 0; r < P.n_rep; ++r) {
-        RunSync& y = A.sync[r];
-        most = fmax(most, __ldcg(&y.slack));
-        any |= __ldcg(&y.rebuild);
-        count = max(count, __ldcg(&y.rebuilds));
-        y = RunSync{};
-      }
-      P.g->slack = most;
-      P.g->rebuild = any;
-      P.g->n_rebuilds += count;
+      *A.sync = RunSync{};
+      for (int r = 0; r < P.n_rep; ++r) A.trial[r] = RunTrial{};
+      P.g->slack = slack;
+      P.g->rebuild = rebuild;
+      P.g->n_rebuilds += rebuilds;
       P.g->trial_slot = slot;
       P.g->it = it;
       P.g->last_disp = __uint_as_float(atomicExch(&P.g->dmax_bits, 0u));

@@ -50,7 +50,7 @@ def test_mixed_loop_bitwise(built, tmp_path, shape, lipids):
     b = _run(m, False, smd.MIXED, cuts)
     for x, y in zip(a[:3], b[:3]):
         assert np.array_equal(x, y)
-    assert a[3] == b[3] and 0 < a[4] <= b[4]  # (the persistent loop renews single lists in between)
+    assert a[3] == b[3] and a[4] == b[4] > 0
     assert np.array_equal(a[5], b[5])  # the list and state it leaves serve the other calls
     assert a[6] < b[6] / 10
 
@@ -91,7 +91,7 @@ def test_batch_loop(built, tmp_path, sizes, precision):
         for k in (1, 8, 31):
             s.advance(k)
         outs.append(s.state() + (np.array([s.box(r) for r in range(len(ms))]), s.launches() - l0,
-                                 [s.mc_stats(r) for r in range(len(ms))]))
+                                 [s.mc_stats(r) for r in range(len(ms))], s.rebuilds()))
         s.close()
     a, b = outs
     for x, y in zip(a[:3], b[:3]):
@@ -101,3 +101,4 @@ def test_batch_loop(built, tmp_path, sizes, precision):
             assert np.abs(x - y).max() < 1e-9
     assert a[3] < b[3] / 10
     assert [m["accepted"] for m in a[4]] == [m["accepted"] for m in b[4]]
+    assert a[5] == b[5] > 0
