@@ -115,6 +115,9 @@ struct smd_system {
     int kernels = 0;  // kernel nodes outside the conditional bodies
   } graph[2];
   bool use_graphs = true;
+  // the rebuild flag is known to be clear: read back so by the last call, and
+  // nothing launched since moves a bead.  Its list kernels would all return at once.
+  bool list_ok = false;
   // the persistent loop kernel (no spheres, no BOND / BEND or field terms, up to
   // kRunMaxBeads per replica): CTAs, beads and threads per CTA, lanes per bead
   struct RunLoop {
@@ -297,12 +300,14 @@ int launch_rebuild(smd_system* h, cudaStream_t st, int cur, int in_graph) {
 int rebuild_kernels(const smd_system* h) { return h->n_cells <= kScanOneMax ? 4 : 6; }
 
 int rebuild_if_needed(smd_system* h, bool clear_after = false) {
+  if (h->list_ok) return 0;
   if (int rc = launch_rebuild(h, h->stream, h->cur, 0)) return rc;
   if (clear_after) SMD_LAUNCH(h, k_set_rebuild<<<1, 1, 0, h->stream>>>(h->P.g, 0));
   return 0;
 }
 
 int force_rebuild(smd_system* h) {
+  h->list_ok = false;
   SMD_LAUNCH(h, k_set_rebuild<<<1, 1, 0, h->stream>>>(h->P.g, 1));
   return rebuild_if_needed(h, true);
 }
@@ -338,6 +343,7 @@ template <int FL>
 int launch_step(smd_system* h, StepEnd se = StepEnd{0, 0, 1, 0, 0}) {
   auto& P = h->P;
   constexpr bool kLoopStep = (FL & (F_FORCES | F_ENERGY | F_INIT)) == 0;
+  if constexpr (kLoopStep) h->list_ok = false;
   // the loop's two integrator variants also come without the field-term
   // call, whose out-of-line ABI costs them registers and a stack frame
   constexpr bool kHot = FL == 0 || FL == (F_STOP | F_DU);
@@ -412,6 +418,7 @@ int launch_force_only(smd_system* h) {
 // mode bit 0: restart half-kick; bit 1: completes a stopped loop step.
 int launch_finish(smd_system* h, int mode, int apply_mc, StepEnd se) {
   auto& P = h->P;
+  h->list_ok = false;
   if (h->mixed)
     SMD_LAUNCH(h, k_finish<true><<<h->bead_grid(), kBeadBlock, 0, h->stream>>>(P, h->cur, mode, apply_mc, se));
   else
@@ -456,6 +463,7 @@ int launch_run(smd_system* h, RunArgs a) {
 
 // `steps` loop iterations (barostat trials included) in one persistent kernel.
 int advance_run(smd_system* h, int steps) {
+  h->list_ok = false;
   const auto& r = h->run;
   const RunArgs a{h->it, h->cur, steps, h->resize_rate, h->barostat ? 1 : 0, r.beads, r.cnt, r.sync, r.trial, r.place};
   const int rc = SMD_RUN_VARIANT(h, launch_run, h, a);
@@ -624,8 +632,7 @@ int grow_list(smd_system* h, int need) {
       cudaGraphExecDestroy(gr.exec);
       gr.exec = nullptr;
     }
-  SMD_LAUNCH(h, k_set_rebuild<<<1, 1, 0, h->stream>>>(h->P.g, 1));
-  return rebuild_if_needed(h, true);
+  return force_rebuild(h);
 }
 
 // Device staging for the state copies: the host side moves one contiguous
@@ -635,10 +642,15 @@ int xfer_buffer(smd_system* h) {
   return h->alloc(&h->xfer, (size_t)h->n * 6);
 }
 
-int read_error(smd_system* h) {
-  Global g;
-  SMD_CUDA(cudaMemcpyAsync(&g, h->P.g, sizeof(Global), cudaMemcpyDeviceToHost, h->stream));
+int read_global(smd_system* h, Global* g) {
+  SMD_CUDA(cudaMemcpyAsync(g, h->P.g, sizeof(Global), cudaMemcpyDeviceToHost, h->stream));
   SMD_CUDA(cudaStreamSynchronize(h->stream));
+  return 0;
+}
+
+// What a call ends with: the device's errors from a read-back of its words.
+int check_global(smd_system* h, const Global& g) {
+  h->list_ok = g.rebuild == 0;
   h->graph_builds = g.graph_builds;
   if (g.n_occ > 0) h->occ_est = g.n_occ;
   if (g.error & 8) return fail(11, "the persistent loop kernel gave up waiting for its CTAs (the handle's state is lost)");
@@ -657,6 +669,11 @@ int read_error(smd_system* h) {
     SMD_CUDA(cudaStreamSynchronize(h->stream));
   }
   return 0;
+}
+int read_error(smd_system* h) {
+  Global g;
+  if (int rc = read_global(h, &g)) return rc;
+  return check_global(h, g);
 }
 
 // Range of the reference's hash cells for a residue above the brute-force
@@ -1222,42 +1239,37 @@ int smd_set_state(smd_system* h, const double* pos, const double* vel) {
   double* vs = h->xfer + n3;
   if (pos) SMD_CUDA(cudaMemcpyAsync(xs, pos, n3 * sizeof(double), cudaMemcpyHostToDevice, h->stream));
   if (vel) SMD_CUDA(cudaMemcpyAsync(vs, vel, n3 * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  // One round trip: a refused state (bit 2 of the error word) is not loaded,
+  // and a new configuration may be denser than the list was sized for, so the
+  // list is built here; if a bead overflowed, it grows to the count and is
+  // built again.
   SMD_LAUNCH(h, k_state_check<<<h->grid(), kBlock, 0, h->stream>>>(P, pos ? xs : nullptr, vel ? vs : nullptr));
-  {
-    Global g;
-    SMD_CUDA(cudaMemcpyAsync(&g, P.g, sizeof(Global), cudaMemcpyDeviceToHost, h->stream));
-    SMD_CUDA(cudaStreamSynchronize(h->stream));
-    if (g.error & 4) {
-      g.error &= ~4;
-      SMD_CUDA(cudaMemcpy(P.g, &g, sizeof(Global), cudaMemcpyHostToDevice));
-      return fail(9, "smd_set_state: a position outside its replica's box or not finite, or a velocity that is "
-                     "not finite (the handle's state is unchanged)");
-    }
-  }
   SMD_LAUNCH(h, k_state_load<<<h->grid(), kBlock, 0, h->stream>>>(P, pos ? xs : nullptr, vel ? vs : nullptr));
   if (pos) {
     if (h->mixed)
       SMD_LAUNCH(h, k_mirror<true><<<h->grid(), kBlock, 0, h->stream>>>(P, h->cur));
     else
       SMD_LAUNCH(h, k_mirror<false><<<h->grid(), kBlock, 0, h->stream>>>(P, h->cur));
-    SMD_LAUNCH(h, k_set_rebuild<<<1, 1, 0, h->stream>>>(P.g, 1));
+    h->list_ok = false;
+    if (int rc = rebuild_if_needed(h, true)) return rc;  // (k_state_load set the flag)
   }
-  if (pos) {
-    // a new configuration may be denser than the list was sized for: build,
-    // and if a bead overflowed, grow the list to its count and build again
-    if (int rc = force_rebuild(h)) return rc;
-    Global g;
-    SMD_CUDA(cudaMemcpyAsync(&g, P.g, sizeof(Global), cudaMemcpyDeviceToHost, h->stream));
-    SMD_CUDA(cudaStreamSynchronize(h->stream));
-    if (g.error & 1) {
-      const int need = std::max(g.need_nbr, g.max_nbr);
-      g.error &= ~1;
-      g.need_nbr = 0;
-      SMD_CUDA(cudaMemcpy(P.g, &g, sizeof(Global), cudaMemcpyHostToDevice));
-      if (int rc = grow_list(h, need)) return rc;
-    }
+  Global g;
+  if (int rc = read_global(h, &g)) return rc;
+  if (g.error & 4) {
+    g.error &= ~4;
+    SMD_CUDA(cudaMemcpy(P.g, &g, sizeof(Global), cudaMemcpyHostToDevice));
+    return fail(9, "smd_set_state: a position outside its replica's box or not finite, or a velocity that is "
+                   "not finite (the handle's state is unchanged)");
   }
-  return read_error(h);  // synchronises the stream
+  if (pos && (g.error & 1)) {
+    const int need = std::max(g.need_nbr, g.max_nbr);
+    g.error &= ~1;
+    g.need_nbr = 0;
+    SMD_CUDA(cudaMemcpy(P.g, &g, sizeof(Global), cudaMemcpyHostToDevice));
+    if (int rc = grow_list(h, need)) return rc;
+    return read_error(h);
+  }
+  return check_global(h, g);
 }
 
 int smd_get_box(smd_system* h, int replica, double box[3]) {
@@ -1277,6 +1289,7 @@ int smd_set_box(smd_system* h, int replica, const double box[3]) {
   RepState rs;
   SMD_CUDA(cudaMemcpyAsync(&rs, h->P.rs + replica, sizeof(RepState), cudaMemcpyDeviceToHost, h->stream));
   SMD_CUDA(cudaStreamSynchronize(h->stream));
+  h->list_ok = false;
   for (int k = 0; k < 3; ++k) rs.box[k] = box[k];
   derive_box(rs, h->rp[replica].cell_cap, h->tab.list_cut, h->tab.rc);
   SMD_CUDA(cudaMemcpyAsync(h->P.rs + replica, &rs, sizeof(RepState), cudaMemcpyHostToDevice, h->stream));
@@ -1296,8 +1309,7 @@ static int compute_forces_impl(smd_system* h, double* out, bool pair_only) {
   rc = pair_only ? launch_step<F_FORCES | F_PAIRONLY>(h) : launch_step<F_FORCES>(h);
   if (rc) return rc;
   SMD_CUDA(cudaMemcpyAsync(out, h->P.force_out, 3 * h->n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-  SMD_CUDA(cudaStreamSynchronize(h->stream));
-  return read_error(h);
+  return read_error(h);  // its synchronisation also completes the copy above
 }
 
 int smd_compute_forces(smd_system* h, double* out) { return compute_forces_impl(h, out, false); }
@@ -1553,16 +1565,14 @@ int autotune(smd_system* h, bool force) {
   for (int v = 0; v < 3; ++v) {
     h->tune.list = v;
     int rc = time_ms(h, [&]() -> int {
-      SMD_LAUNCH(h, k_set_rebuild<<<1, 1, 0, h->stream>>>(P.g, 1));
-      return rebuild_if_needed(h, true);
+      return force_rebuild(h);
     }, 3, &h->tune.ms_list[v]);
     if (rc) return rc;
     if (h->tune.ms_list[v] < h->tune.ms_list[best_list]) best_list = v;
   }
   h->tune.list = best_list;
   // leave a list built by the chosen kernel
-  SMD_LAUNCH(h, k_set_rebuild<<<1, 1, 0, h->stream>>>(P.g, 1));
-  if (int rc = rebuild_if_needed(h, true)) return rc;
+  if (int rc = force_rebuild(h)) return rc;
   const int lanes[3] = {4, 8, 16};
   int best_lanes = 1;
   for (int v = 0; v < 3; ++v) {
@@ -1623,6 +1633,7 @@ int smd_advance(smd_system* h, int steps, int flags) {
       if (graph_fits(h, h->it, left)) {
         auto& g = h->graph[h->cur];
         if (!g.exec && (rc = capture_period(h, h->cur))) return rc;
+        h->list_ok = false;
         SMD_CUDA(cudaGraphLaunch(g.exec, h->stream));
         h->launches += g.kernels;
         h->it += h->resize_rate;
@@ -1952,6 +1963,7 @@ int adj_pair_pass(smd_system* h, const double* w, double dt, double invT) {
 // rebuilt when they moved too far from its build positions (force: always).
 int adj_load(smd_system* h, const double* xs, const double* vs, bool force) {
   auto& P = h->P;
+  h->list_ok = false;
   if (h->mixed)
     SMD_LAUNCH(h, k_adj_load<true><<<h->grid(), kBlock, 0, h->stream>>>(P, h->cur, xs, vs));
   else

@@ -2635,7 +2635,8 @@ __global__ void __launch_bounds__(kBlock) k_state_check(DevPtrs P, const double*
 
 __global__ void __launch_bounds__(kBlock) k_state_load(DevPtrs P, const double* xs, const double* vs) {
   const int i = blockIdx.x * kBlock + threadIdx.x;
-  if (i >= P.n) return;
+  if (i >= P.n || (P.g->error & 4)) return;  // (k_state_check refused it)
+  if (xs && i == 0) P.g->rebuild = 1;
   const int o = P.orig[i];
   if (xs) {
     P.x[i] = xs[3 * o];
