@@ -461,11 +461,17 @@ int launch_run(smd_system* h, RunArgs a) {
     return r_.warps == 28 ? f<false, 8, 28>(__VA_ARGS__) : f<false, 8, 32>(__VA_ARGS__);   \
   }()
 
-// `steps` loop iterations (barostat trials included) in one persistent kernel.
-int advance_run(smd_system* h, int steps) {
+// Whether the persistent loop can take this handle's next steps.
+bool run_ready(const smd_system* h) {
+  return h->run.grid && h->use_graphs && !h->profile && !h->ext_noise_pending && !h->meas.tracking;
+}
+
+// `steps` loop iterations (barostat trials included) in one persistent kernel;
+// save: the positions after each of them (3n values in file order), or null.
+int advance_run(smd_system* h, int steps, double* save = nullptr) {
   h->list_ok = false;
   const auto& r = h->run;
-  const RunArgs a{h->it, h->cur, steps, h->resize_rate, h->barostat ? 1 : 0, r.beads, r.cnt, r.sync, r.trial, r.place};
+  const RunArgs a{h->it, h->cur, steps, h->resize_rate, h->barostat ? 1 : 0, r.beads, r.cnt, r.sync, r.trial, r.place, save};
   const int rc = SMD_RUN_VARIANT(h, launch_run, h, a);
   if (rc) return rc;
   for (int k = 0; k < steps; ++k)
@@ -1625,7 +1631,7 @@ int smd_advance(smd_system* h, int steps, int flags) {
     for (int s = 0; s < chunk; ++s) {
       // the last step of a stopping call runs alone (it stops after its second half-kick)
       const int left = chunk - s - ((stop_at_measure && done + chunk == steps) ? 1 : 0);
-      if (h->run.grid && left > 0 && h->use_graphs && !h->profile && !h->ext_noise_pending && !h->meas.tracking) {
+      if (left > 0 && run_ready(h)) {
         if ((rc = advance_run(h, left))) return rc;
         s += left - 1;
         continue;
@@ -1969,7 +1975,7 @@ int adj_load(smd_system* h, const double* xs, const double* vs, bool force) {
   else
     SMD_LAUNCH(h, k_adj_load<false><<<h->grid(), kBlock, 0, h->stream>>>(P, h->cur, xs, vs));
   if (force) SMD_LAUNCH(h, k_set_rebuild<<<1, 1, 0, h->stream>>>(P.g, 1));
-  return rebuild_if_needed(h, true);
+  return rebuild_if_needed(h, force);  // (k_adj_load decides anew each time)
 }
 
 int adj_check_handle(smd_system* h) {
@@ -2082,11 +2088,15 @@ int smd_adjoint(smd_system* h, const smd_adjoint_spec* spec, smd_adjoint_result*
       if (int r = adj_load(h, x, x + n3, true)) return r;
       h->it = cp_it[c];
       SMD_LAUNCH(h, k_set_counters<<<1, 1, 0, h->stream>>>(P.g, h->it, 1, 0, 0));
-      for (int m = 0; m < len; ++m) {  // recompute x_n of the segment
+      // recompute x_n of the segment (the persistent loop saves them as it goes)
+      const bool whole = len > 1 && run_ready(h);
+      for (int m = 0; m < (whole ? 1 : len); ++m) {
         SMD_LAUNCH(h, k_state_save<<<h->grid(), kBlock, 0, h->stream>>>(P, seg + (size_t)m * n3, nullptr));
-        if (m + 1 < len)
+        if (m + 1 < len && !whole)
           if (int r = smd_advance(h, 1, SMD_ASYNC)) return r;
       }
+      if (whole)
+        if (int r = advance_run(h, len - 1, seg + n3)) return r;
       for (int m = len - 1; m >= 0; --m) {
         if (int r = adj_load(h, seg + (size_t)m * n3, nullptr, false)) return r;
         if (int r = adj_pair_pass(h, w, dt, invT)) return r;

@@ -80,6 +80,7 @@ struct RunArgs {
   RunSync* sync;
   RunTrial* trial;  // per replica
   const RunPlace* place;  // per CTA
+  double* save;   // positions after every step in file order (3n each), or null
 };
 
 // Shared memory per CTA beyond the static part.
@@ -786,6 +787,10 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
         }
       }
       for (int d = 0; d < 3; ++d) st[d * NB + tid] = x[d];
+      if (A.save) {
+        double* to = A.save + 3 * ((size_t)s * P.n + orig[tid]);
+        for (int d = 0; d < 3; ++d) to[d] = x[d];
+      }
       const uint4 mn = make_uint4(to_frac(x[0], rs.frac_per_len[0]), to_frac(x[1], rs.frac_per_len[1]),
                                   to_frac(x[2], rs.frac_per_len[2]), w);
       vmax = displacement(ref[tid], mn.x, mn.y, mn.z, rs);
