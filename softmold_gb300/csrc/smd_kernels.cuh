@@ -703,22 +703,29 @@ __global__ void __launch_bounds__(kOctThreads) k_nbr_cells_oct(DevPtrs P, int cu
 // ---- Flat stencil.  The CTA stages the stencil's beads as FP32
 // offsets from the cell centre (exact 32-bit fractional differences, scaled
 // once), one x-row segment after another with no per-candidate search, and
-// each warp tests one bead of the cell against every staged candidate.  Few
-// barriers and 16 KB of shared memory per CTA: at the ~30 beads of an
-// occupied membrane cell this costs fewer instructions than filtering the
-// stencil per octant first.
+// each warp tests its share of the cell's beads, four at a time, against every
+// staged candidate.  Few barriers and 20 KB of shared memory per CTA: at the
+// ~30 beads of an occupied membrane cell this costs fewer instructions than
+// filtering the stencil per octant first.  With c the candidate's offset and x
+// the bead's,
+//   |c - x|^2 < L^2  <=>  |c|^2 - 2 x . c < L^2 - |x|^2,
+// three FMAs and a comparison.  Two beads at a time, six operations per
+// distance and a branch around every store took 101 us per build of 120,001
+// beads, this 84; the compaction of the hits (ballot, two counts, the store)
+// is now most of it.
 //
-// Both forms build their lists here.  The plain form's list is a filter only
-// (its pair passes test every entry's FP64 distance), so FP32 tests of the
-// fractional mirror serve it with a cut widened by the mirror's resolution and
-// the FP32 rounding of the offsets.  Testing in FP64 took 594 us per build of
-// an 18,003-bead vesicle, bound by the FP64 pipe.
-constexpr int kFlatChunk = 1024;  // staged candidates per pass (16 KB)
+// Both forms build their lists here.  The list is a filter (the pair passes
+// test every entry's distance), so FP32 tests of the fractional mirror serve
+// with a wider cut: by 1e-5 of the cut, twice the rounding of the expanded
+// square (offsets stay within 3.5 cuts on grids of three cells and more), and
+// in the plain form by the mirror's resolution.  Testing in FP64 took 594 us
+// per build of an 18,003-bead vesicle, bound by the FP64 pipe.
+constexpr int kFlatChunk = 640;  // staged candidates per pass (12.5 KB)
 
 // One bead (one warp) against mpad staged candidates (a multiple of 32):
-// appends the hits within lc2 to the bead's list from position count.
-template <bool THIN>
-__device__ __forceinline__ int flat_scan(const float4* stage, int mpad, float xi, float yi, float zi, int i,
+// appends the hits within lc2 to the bead's list from position count.  Thin
+// boxes (fewer than 3 cells on an axis) take the minimum image per pair.
+__device__ __forceinline__ int flat_scan_thin(const float4* stage, const int* stj, int mpad, float xi, float yi, float zi, int i,
                                          float lc2, float bx, float by, float bz, int* out, int count, int kmax,
                                          int lane) {
   const unsigned int below = (1u << lane) - 1u;
@@ -726,14 +733,11 @@ __device__ __forceinline__ int flat_scan(const float4* stage, int mpad, float xi
   for (int k0 = 0; k0 < mpad; k0 += 32) {
     const float4 cj = stage[k0 + lane];
     float dx = xi - cj.x, dy = yi - cj.y, dz = zi - cj.z;
-    if constexpr (THIN) {  // fewer than 3 cells on an axis: minimum image per pair
-      dx -= bx * rintf(dx / bx);
-      dy -= by * rintf(dy / by);
-      dz -= bz * rintf(dz / bz);
-    }
-    const int j = __float_as_int(cj.w);
-    bool hit = (dx * dx + dy * dy + dz * dz < lc2) & (j != i);
-    if constexpr (THIN) hit = hit & (j >= 0);  // the minimum image can fold a sentinel back
+    dx -= bx * rintf(dx / bx);
+    dy -= by * rintf(dy / by);
+    dz -= bz * rintf(dz / bz);
+    const int j = stj[k0 + lane];  // -1: a sentinel, which the minimum image can fold back
+    const bool hit = (dx * dx + dy * dy + dz * dz < lc2) & (j != i) & (j >= 0);
     const unsigned int hits = __ballot_sync(0xffffffffu, hit);
     if (hits) {
       const int slot = count + __popc(hits & below);
@@ -744,42 +748,68 @@ __device__ __forceinline__ int flat_scan(const float4* stage, int mpad, float xi
   return count;
 }
 
-// Two beads (one warp) against the same staged candidates: one shared load
-// and one loop step serve both.  Appends as flat_scan does, per bead.
-template <bool THIN>
-__device__ __forceinline__ void flat_scan2(const float4* stage, int mpad, float xa, float ya, float za, int ia,
-                                           float xb, float yb, float zb, int ib, float lc2, float bx, float by,
-                                           float bz, int* outa, int* outb, int& ca, int& cb, int kmax, int lane) {
+// Appends j to the list at out for the lanes with r2 < lim and d != self, in
+// lane order: a ballot, two counts and a predicated store (a branch around the
+// store costs three instructions more).
+__device__ __forceinline__ void keep_hits(float r2, float lim, int d, int self, unsigned int below, int j, int* out,
+                                          int kmax, int& count) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t.reg .b32 h, b;\n\t.reg .b64 a;\n\t"
+      "setp.lt.f32 p, %1, %2;\n\t"
+      "setp.ne.and.s32 p, %3, %4, p;\n\t"
+      "vote.sync.ballot.b32 h, p, 0xffffffff;\n\t"
+      "and.b32 b, h, %5;\n\t"
+      "popc.b32 b, b;\n\t"
+      "add.s32 b, b, %0;\n\t"
+      "setp.lt.and.s32 p, b, %6, p;\n\t"
+      "mad.wide.s32 a, b, 4, %7;\n\t"
+      "@p st.global.u32 [a], %8;\n\t"
+      "popc.b32 h, h;\n\t"
+      "add.s32 %0, %0, h;\n\t"
+      "}"
+      : "+r"(count)
+      : "f"(r2), "f"(lim), "r"(d), "r"(self), "r"(below), "r"(kmax), "l"(__cvta_generic_to_global(out)), "r"(j)
+      : "memory");
+}
+
+// Beads i .. i + n - 1 (n <= Q, one warp) against the mpad staged candidates:
+// one shared load and one loop step serve them all.  Appends as
+// flat_scan_thin does, per bead.
+template <int Q>
+__device__ __forceinline__ void flat_beads(const DevPtrs& P, const float4* stage, const int* stj, int mpad, int i,
+                                           int n, unsigned int crx, unsigned int cry, unsigned int crz, float sx,
+                                           float sy, float sz, float lc2, int* cnt, int lane) {
   const unsigned int below = (1u << lane) - 1u;
-#pragma unroll 2
-  for (int k0 = 0; k0 < mpad; k0 += 32) {
-    const float4 cj = stage[k0 + lane];
-    const int j = __float_as_int(cj.w);
-    float dx = xa - cj.x, dy = ya - cj.y, dz = za - cj.z;
-    float ex = xb - cj.x, ey = yb - cj.y, ez = zb - cj.z;
-    if constexpr (THIN) {
-      dx -= bx * rintf(dx / bx);
-      dy -= by * rintf(dy / by);
-      dz -= bz * rintf(dz / bz);
-      ex -= bx * rintf(ex / bx);
-      ey -= by * rintf(ey / by);
-      ez -= bz * rintf(ez / bz);
-    }
-    bool ha = (dx * dx + dy * dy + dz * dz < lc2) & (j != ia);
-    bool hb = (ex * ex + ey * ey + ez * ez < lc2) & (j != ib);
-    if constexpr (THIN) {
-      ha = ha & (j >= 0);
-      hb = hb & (j >= 0);
-    }
-    const unsigned int hitsa = __ballot_sync(0xffffffffu, ha), hitsb = __ballot_sync(0xffffffffu, hb);
-    if (hitsa | hitsb) {
-      const int sa = ca + __popc(hitsa & below), sb = cb + __popc(hitsb & below);
-      if (ha && sa < kmax) outa[sa] = j;
-      if (hb && sb < kmax) outb[sb] = j;
-      ca += __popc(hitsa);
-      cb += __popc(hitsb);
+  const int kmax = P.kmax;
+  float4 f[Q];  // -2 x and lc2 - |x|^2
+  int count[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    f[q] = make_float4(0.f, 0.f, 0.f, -1.f);  // past the last bead: no hit
+    count[q] = q * kmax;
+    if (q < n) {
+      const uint4 mi = P.mt[i + q];
+      const float x = (float)(int)(mi.x - crx) * sx, y = (float)(int)(mi.y - cry) * sy,
+                  z = (float)(int)(mi.z - crz) * sz;
+      f[q] = make_float4(-2.f * x, -2.f * y, -2.f * z, lc2 - (x * x + y * y + z * z));
+      count[q] += cnt[q];
     }
   }
+  int* out = P.nbr + (size_t)i * kmax;
+  for (int k = lane; k < mpad; k += 32) {
+    const float4 c = stage[k];
+    const int j = stj[k];
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      keep_hits(fmaf(f[q].z, c.z, fmaf(f[q].y, c.y, fmaf(f[q].x, c.x, c.w))), f[q].w, j - i, q, below, j, out,
+                (q + 1) * kmax, count[q]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if (lane == q && q < n) cnt[q] = count[q] - q * kmax;
+  __syncwarp();
 }
 
 template <bool MIXED, int NT>
@@ -788,7 +818,8 @@ __device__ __forceinline__ void nbr_cell_flat(const DevPtrs& P, int cur, int c) 
   if (s0 >= e0) return;
   __shared__ int seg_s[18], seg_len[18], seg_p[19];
   __shared__ int cnt[kNbrMaxCell];
-  __shared__ float4 stage[kFlatChunk];
+  __shared__ float4 stage[kFlatChunk];  // offset and its square
+  __shared__ int stj[kFlatChunk];
   // every thread derives the cell's context itself (the same few loads)
   const CellCtx q = cell_ctx(P, c, s0, e0);
   const RepState& rs = P.rs[q.r];
@@ -801,7 +832,9 @@ __device__ __forceinline__ void nbr_cell_flat(const DevPtrs& P, int cur, int c) 
                      crz = cell_centre_frac(q.cz, q.n2);
   __syncthreads();  // the previous cell of this CTA is done with the shared arrays
   copy_back<MIXED, NT>(P, cur, q);
-  if (threadIdx.x < 32) stencil_warp(P, q, seg_s, seg_p, seg_len);
+  if (threadIdx.x < 32) {
+    stencil_warp(P, q, seg_s, seg_p, seg_len);
+  }
   for (int b = threadIdx.x; b < nb; b += NT) cnt[b] = 0;
   __syncthreads();
   const int nseg = seg_len[0];
@@ -809,10 +842,9 @@ __device__ __forceinline__ void nbr_cell_flat(const DevPtrs& P, int cur, int c) 
   const float sx = rs.len_per_frac[0], sy = rs.len_per_frac[1], sz = rs.len_per_frac[2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kmax = P.kmax;
-  float lcut = P.tab->list_cut_f + 1e-4f;
-  // plain form: + the mirror's truncation (one unit per axis and pair) and the
-  // offsets' rounding (under 1e-6 of the cell size, itself under 2 list_cut)
-  if constexpr (!MIXED) lcut += 4e-6f * P.tab->list_cut_f + 4.f * fmaxf(sx, fmaxf(sy, sz));
+  float lcut = P.tab->list_cut_f * (1.f + 1e-5f) + 1e-4f;
+  // plain form: + the mirror's truncation (one unit per axis and pair)
+  if constexpr (!MIXED) lcut += 4.f * fmaxf(sx, fmaxf(sy, sz));
   const float lc2 = lcut * lcut;
   const bool thin = q.n0 < 3 || q.n1 < 3 || q.n2 < 3;
   const float bx = sx * 4294967296.0f, by = sy * 4294967296.0f, bz = sz * 4294967296.0f;
@@ -820,66 +852,46 @@ __device__ __forceinline__ void nbr_cell_flat(const DevPtrs& P, int cur, int c) 
     const int m = min(kFlatChunk, M - base);
     const int mpad = (m + 31) & ~31;
     if (base > 0) __syncthreads();  // every warp is done with the previous chunk
-    // stage the chunk: thread t takes slots base + t, + NT, ...; the bead of a
-    // slot comes from the segment table, and four loads are issued together
-    // (a small system has few cells per SM, so their latency is not hidden
-    // by other CTAs)
-    {
-      constexpr int kBatch = 4;
-      int t = 0;  // segment of this thread's next slot (slots only increase)
-      for (int k0 = threadIdx.x; k0 < m; k0 += kBatch * NT) {
-        int jj[kBatch];
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-          const int g = base + k0 + u * NT;
-          jj[u] = -1;
-          if (k0 + u * NT < m) {
-            while (seg_p[t + 1] <= g) ++t;
-            jj[u] = seg_s[t] + (g - seg_p[t]);
-          }
-        }
-        uint4 mj[kBatch];
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u)
-          if (jj[u] >= 0) mj[u] = P.mt[jj[u]];
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u)
-          if (jj[u] >= 0)
-            stage[k0 + u * NT] = make_float4((float)(int)(mj[u].x - crx) * sx, (float)(int)(mj[u].y - cry) * sy,
-                                             (float)(int)(mj[u].z - crz) * sz, __int_as_float(jj[u]));
+    // stage the chunk, a segment per warp and turn, two loads in flight
+    for (int t = warp; t < nseg; t += NT / 32) {
+      const int lo = max(seg_p[t] - base, 0), hi = min(seg_p[t + 1] - base, m), j0 = seg_s[t] - (seg_p[t] - base);
+      for (int k0 = lo + lane; k0 < hi; k0 += 64) {
+        const bool two = k0 + 32 < hi;
+        const uint4 m0 = P.mt[j0 + k0], m1 = P.mt[two ? j0 + k0 + 32 : j0 + k0];
+        auto put = [&](int k, const uint4& mj) {
+          const float x = (float)(int)(mj.x - crx) * sx, y = (float)(int)(mj.y - cry) * sy,
+                      z = (float)(int)(mj.z - crz) * sz;
+          stage[k] = make_float4(x, y, z, x * x + y * y + z * z);
+          stj[k] = j0 + k;
+        };
+        put(k0, m0);
+        if (two) put(k0 + 32, m1);
       }
     }
-    // far sentinels complete the last round of 32 (index -1 matches no bead)
-    for (int k = m + threadIdx.x; k < mpad; k += NT) stage[k] = make_float4(1e30f, 1e30f, 1e30f, __int_as_float(-1));
+    // far sentinels complete the last round of 32
+    for (int k = m + threadIdx.x; k < mpad; k += NT) {
+      stage[k] = make_float4(0.f, 0.f, 0.f, 1e30f);
+      stj[k] = -1;
+    }
     __syncthreads();
-    // beads in pairs (b, b + NT/32): warp w takes 2w, 2w+1 of every 2*NT/32
-    for (int b = 2 * warp; b < nb; b += 2 * (NT / 32)) {
-      const int i = q.s + b;
-      const uint4 mi = P.mt[i];
-      const float xi = (float)(int)(mi.x - crx) * sx, yi = (float)(int)(mi.y - cry) * sy,
-                  zi = (float)(int)(mi.z - crz) * sz;
-      int* out = P.nbr + (size_t)i * kmax;
-      if (b + 1 < nb) {
-        const int i2 = i + 1;
-        const uint4 m2 = P.mt[i2];
-        const float x2 = (float)(int)(m2.x - crx) * sx, y2 = (float)(int)(m2.y - cry) * sy,
-                    z2 = (float)(int)(m2.z - crz) * sz;
-        int ca = cnt[b], cb = cnt[b + 1];
-        if (thin)
-          flat_scan2<true>(stage, mpad, xi, yi, zi, i, x2, y2, z2, i2, lc2, bx, by, bz, out, out + kmax, ca, cb, kmax,
-                           lane);
-        else
-          flat_scan2<false>(stage, mpad, xi, yi, zi, i, x2, y2, z2, i2, lc2, bx, by, bz, out, out + kmax, ca, cb, kmax,
-                            lane);
-        if (lane == 0) {
-          cnt[b] = ca;
-          cnt[b + 1] = cb;
-        }
-      } else {
-        const int count = thin ? flat_scan<true>(stage, mpad, xi, yi, zi, i, lc2, bx, by, bz, out, cnt[b], kmax, lane)
-                               : flat_scan<false>(stage, mpad, xi, yi, zi, i, lc2, bx, by, bz, out, cnt[b], kmax, lane);
+    // each warp takes an equal share of the beads
+    const int last = nb * (warp + 1) / (NT / 32);
+    for (int b = nb * warp / (NT / 32); b < last;) {
+      const int i = q.s + b, left = last - b;
+      if (thin) {
+        const uint4 mi = P.mt[i];
+        const int count =
+            flat_scan_thin(stage, stj, mpad, (float)(int)(mi.x - crx) * sx, (float)(int)(mi.y - cry) * sy,
+                           (float)(int)(mi.z - crz) * sz, i, lc2, bx, by, bz, P.nbr + (size_t)i * kmax, cnt[b], kmax, lane);
+        __syncwarp();
         if (lane == 0) cnt[b] = count;
+        ++b;
+        continue;
       }
+      const int n = left > 2 ? min(left, 4) : left;
+      if (n > 2) flat_beads<4>(P, stage, stj, mpad, i, n, crx, cry, crz, sx, sy, sz, lc2, cnt + b, lane);
+      else flat_beads<2>(P, stage, stj, mpad, i, n, crx, cry, crz, sx, sy, sz, lc2, cnt + b, lane);
+      b += n;
     }
   }
   __syncthreads();
@@ -887,7 +899,7 @@ __device__ __forceinline__ void nbr_cell_flat(const DevPtrs& P, int cur, int c) 
 }
 
 template <bool MIXED, int NT>
-__global__ void __launch_bounds__(NT, 768 / NT) k_nbr_cells_flat(DevPtrs P, int cur) {
+__global__ void __launch_bounds__(NT, 1024 / NT) k_nbr_cells_flat(DevPtrs P, int cur) {
   pdl_wait();  // the reordered state
   if (!P.g->rebuild) return;
   list_build_begin(P);

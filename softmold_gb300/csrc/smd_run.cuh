@@ -175,31 +175,6 @@ struct SlotWalk {
   }
 };
 
-// Appends j to the list at out for the lanes with r2 < lim and d != self, in
-// lane order: a ballot, two counts and a predicated store (a branch around the
-// store costs three instructions more).
-__device__ __forceinline__ void keep_hits(float r2, float lim, int d, int self, unsigned int below, int j, int* out,
-                                          int kmax, int& count) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t.reg .b32 h, b;\n\t.reg .b64 a;\n\t"
-      "setp.lt.f32 p, %1, %2;\n\t"
-      "setp.ne.and.s32 p, %3, %4, p;\n\t"
-      "vote.sync.ballot.b32 h, p, 0xffffffff;\n\t"
-      "and.b32 b, h, %5;\n\t"
-      "popc.b32 b, b;\n\t"
-      "add.s32 b, b, %0;\n\t"
-      "setp.lt.and.s32 p, b, %6, p;\n\t"
-      "mad.wide.s32 a, b, 4, %7;\n\t"
-      "@p st.global.u32 [a], %8;\n\t"
-      "popc.b32 h, h;\n\t"
-      "add.s32 %0, %0, h;\n\t"
-      "}"
-      : "+r"(count)
-      : "f"(r2), "f"(lim), "r"(d), "r"(self), "r"(below), "r"(kmax), "l"(__cvta_generic_to_global(out)), "r"(j)
-      : "memory");
-}
-
 // Lists of beads a = ia and b = ia + 1 of the same cell from the stencil's M
 // slots, by one warp.  Distances come from the exact fractional differences,
 // whose wrap is the minimum image, so thin grids need no other path.
