@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(kOctThreads) k_nbr_cells_oct(DevPtrs P, int cu
 // offsets from the cell centre (exact 32-bit fractional differences, scaled
 // once), one x-row segment after another with no per-candidate search, and
 // each warp tests its share of the cell's beads, four at a time, against every
-// staged candidate.  Few barriers and 20 KB of shared memory per CTA: at the
+// staged candidate.  Few barriers and 17 KB of shared memory per CTA: at the
 // ~30 beads of an occupied membrane cell this costs fewer instructions than
 // filtering the stencil per octant first.  With c the candidate's offset and x
 // the bead's,
@@ -716,18 +716,31 @@ __global__ void __launch_bounds__(kOctThreads) k_nbr_cells_oct(DevPtrs P, int cu
 //
 // Both forms build their lists here.  The list is a filter (the pair passes
 // test every entry's distance), so FP32 tests of the fractional mirror serve
-// with a wider cut: by 1e-5 of the cut, twice the rounding of the expanded
-// square (offsets stay within 3.5 cuts on grids of three cells and more), and
-// in the plain form by the mirror's resolution.  Testing in FP64 took 594 us
+// with a wider cut (list_reach), and in the plain form by the mirror's
+// resolution too.  Testing in FP64 took 594 us
 // per build of an 18,003-bead vesicle, bound by the FP64 pipe.
+// The list cut widened by more than FP32 tests can be off.  In cells of width w
+// an expanded square's terms stay below 36 w^2 (offsets from a bead of the
+// stencil's middle cell; from its centre, half that), its rounding below 2e-5
+// w^2 or 1e-5 w^2 / L of the distance.
+template <bool MIXED>
+__device__ __forceinline__ float list_reach(const RepState& rs, float cut) {
+  float w = 0.f;
+  for (int d = 0; d < 3; ++d) w = fmaxf(w, rs.len_per_frac[d] * (4294967296.f / (float)rs.ncell[d]));
+  float reach = cut + 1e-4f + 1e-5f * w * w / cut;
+  // the mirror's truncation (one unit per axis and pair)
+  if constexpr (!MIXED) reach += 4.f * fmaxf(rs.len_per_frac[0], fmaxf(rs.len_per_frac[1], rs.len_per_frac[2]));
+  return reach;
+}
+
 constexpr int kFlatChunk = 640;  // staged candidates per pass (12.5 KB)
 
 // One bead (one warp) against mpad staged candidates (a multiple of 32):
 // appends the hits within lc2 to the bead's list from position count.  Thin
 // boxes (fewer than 3 cells on an axis) take the minimum image per pair.
-__device__ __forceinline__ int flat_scan_thin(const float4* stage, const int* stj, int mpad, float xi, float yi, float zi, int i,
-                                         float lc2, float bx, float by, float bz, int* out, int count, int kmax,
-                                         int lane) {
+__device__ __forceinline__ int flat_scan_thin(const float4* stage, const int* stj, int mpad, float xi, float yi,
+                                              float zi, int i, float lc2, float bx, float by, float bz, int* out,
+                                              int count, int kmax, int lane) {
   const unsigned int below = (1u << lane) - 1u;
 #pragma unroll 4
   for (int k0 = 0; k0 < mpad; k0 += 32) {
@@ -842,9 +855,7 @@ __device__ __forceinline__ void nbr_cell_flat(const DevPtrs& P, int cur, int c) 
   const float sx = rs.len_per_frac[0], sy = rs.len_per_frac[1], sz = rs.len_per_frac[2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kmax = P.kmax;
-  float lcut = P.tab->list_cut_f * (1.f + 1e-5f) + 1e-4f;
-  // plain form: + the mirror's truncation (one unit per axis and pair)
-  if constexpr (!MIXED) lcut += 4.f * fmaxf(sx, fmaxf(sy, sz));
+  const float lcut = list_reach<MIXED>(rs, P.tab->list_cut_f);
   const float lc2 = lcut * lcut;
   const bool thin = q.n0 < 3 || q.n1 < 3 || q.n2 < 3;
   const float bx = sx * 4294967296.0f, by = sy * 4294967296.0f, bz = sz * 4294967296.0f;

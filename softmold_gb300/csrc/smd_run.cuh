@@ -545,11 +545,8 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
         if (n > 0) groups[at] = tid | n << 16;
       }
       __syncthreads();
-      // 1e-5 of the cut: more than the rounding of run_scan_group's squares (offsets
-      // stay within 4.2 cuts); plain form: + the mirror's resolution
       {
-        const float lcut = T.list_cut_f * (1.f + 1e-5f) + 1e-4f +
-                           (MIXED ? 0.f : 4.f * fmaxf(rs.len_per_frac[0], fmaxf(rs.len_per_frac[1], rs.len_per_frac[2])));
+        const float lcut = list_reach<MIXED>(rs, T.list_cut_f);
         const float lc2 = lcut * lcut;
         const float x0 = rs.len_per_frac[0], x1 = rs.len_per_frac[1], x2 = rs.len_per_frac[2];
         const uint4* m = P.m4[cur];
