@@ -61,22 +61,21 @@ PERIOD = 8         # MD steps of one barostat period (resizeRate, MD.cpp:67)
 STEP_MD = 10 * PERIOD  # MD steps per bench step (20 bench steps take over 100 ms)
 SMS = 152          # GB300 streaming multiprocessors
 ISSUE_PER_SM_CLK = 4  # warp instructions issued per SM and clock (four schedulers)
-# DRAM bytes and warp instructions per bead and MD step of the mixed step,
-# summed over every kernel of the step with its launches per MD step, from ncu
-# captures of the workload (metrics dram__bytes_read.sum, dram__bytes_write.sum,
-# smsp__inst_executed.sum per kernel).  "warm": one pass per launch with the
-# caches as the previous kernels left them (--cache-control none), the traffic
-# of the bench's L2-resident loop; "cold": every launch after an L2 flush, each
-# kernel's whole working set from DRAM (an upper bound).  The commands and the
-# per-kernel tables are in profiles/step_traffic_warm_bilayer60k.md and
-# profiles/step_traffic_bilayer60k.md.  Traffic is a named constant because ncu
-# cannot run inside the timed region.
+# DRAM bytes and warp instructions per bead and MD step of the mixed step, from
+# ncu captures of the workload (metrics dram__bytes_read.sum,
+# dram__bytes_write.sum, smsp__inst_executed.sum).  "warm" and the instructions:
+# 80 steps of the persistent loop with the caches as the previous kernels left
+# them (--cache-control none); "cold": the same step launched kernel by kernel,
+# every launch after an L2 flush, each kernel's whole working set from DRAM (an
+# upper bound).  The commands and the tables are in
+# profiles/run_loop_bilayer60k.md and profiles/step_traffic_bilayer60k.md.
+# Traffic is a named constant because ncu cannot run inside the timed region.
 STEP_PROFILE = {
-    "bilayer20k": {"dram_bytes_per_bead_step": 54.0, "dram_bytes_per_bead_step_cold": 773.0,
-                   "warp_inst_per_bead_step": 618.0,
-                   "source": "profiles/step_traffic_warm_bilayer60k.md (ncu --cache-control none: the bench's "
-                             "L2-resident loop; traffic and instructions) and profiles/step_traffic_bilayer60k.md "
-                             "(ncu, caches flushed per launch: an upper bound on traffic)"},
+    "bilayer20k": {"dram_bytes_per_bead_step": 13.6, "dram_bytes_per_bead_step_cold": 773.0,
+                   "warp_inst_per_bead_step": 693.0,
+                   "source": "profiles/run_loop_bilayer60k.md (ncu --cache-control none: the persistent loop; "
+                             "traffic and instructions) and profiles/step_traffic_bilayer60k.md (ncu, kernel by "
+                             "kernel, caches flushed per launch: an upper bound on traffic)"},
 }
 
 

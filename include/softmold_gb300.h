@@ -196,8 +196,9 @@ int smd_autotune(smd_system* h, int force, int* lanes, int* list_kernel, float* 
 int smd_set_tuning(smd_system* h, int lanes, int list_kernel);
 
 /* Launch mode of smd_advance: on = 1 (default) runs a stretch of steps of a
- * small or mid-size system as one persistent cooperative kernel, and each
- * barostat period of any other as one CUDA graph whose list builds are
+ * system or batch of up to 65,000 beads per replica (without spheres, BOND / BEND
+ * or field terms) as one persistent cooperative kernel, and each barostat
+ * period of any other as one CUDA graph whose list builds are
  * conditional nodes; on = 0 launches the same work kernel by kernel (profilers
  * that cannot see kernel nodes inside graphs with conditional nodes still see
  * each kernel).  No reference counterpart: the reference launches nothing. */
