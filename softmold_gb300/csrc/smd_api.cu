@@ -502,30 +502,24 @@ int run_fits_device(smd_system* h, bool* fits) {
 int run_setup(smd_system* h) {
   auto& r = h->run;
   r.grid = 0;
-  if (h->n_rep > h->sms || h->n_sph > 0 || h->n_terms > 0) return 0;
+  const int ctas = std::min(h->sms, 255);  // (the barrier counts them in 8 bits)
+  if (h->n_rep > ctas || h->n_sph > 0 || h->n_terms > 0) return 0;
   int cells = 0, most = 0;  // of the largest replica
   for (int k = 0; k < h->n_rep; ++k) {
     cells = std::max(cells, h->rp[k].cell_cap);
     most = std::max(most, h->rp[k].bead_end - h->rp[k].bead_begin);
   }
   if (most > kRunMaxBeads || cells > kRunCells) return 0;
-  // the fewest beads per CTA that leave every replica CTAs of its own (at most
-  // 255 each: the barrier counts them in 8 bits)
-  auto ctas_at = [&](int beads, int* largest) {
+  // the fewest beads per CTA that leave every replica CTAs of its own
+  auto ctas_at = [&](int beads) {
     long long sum = 0;
-    for (int k = 0; k < h->n_rep; ++k) {
-      const int c = (h->rp[k].bead_end - h->rp[k].bead_begin + beads - 1) / beads;
-      *largest = std::max(*largest, c);
-      sum += c;
-    }
+    for (int k = 0; k < h->n_rep; ++k) sum += (h->rp[k].bead_end - h->rp[k].bead_begin + beads - 1) / beads;
     return sum;
   };
   int lo = 8, hi = std::max(8, most);
   while (lo < hi) {
     const int mid = (lo + hi) / 2;
-    int largest = 0;
-    const long long sum = ctas_at(mid, &largest);
-    if (sum <= h->sms && largest <= 255) hi = mid; else lo = mid + 1;
+    if (ctas_at(mid) <= ctas) hi = mid; else lo = mid + 1;
   }
   r.beads = lo;
   r.lanes = r.beads <= 24 ? 32 : (r.beads <= 48 ? 16 : 8);
