@@ -378,7 +378,7 @@ int launch_step(smd_system* h, StepEnd se = StepEnd{0, 0, 1, 0, 0}) {
     } else {
       SMD_PDL_INTEG(h, (k_integ<true, FL | F_FIELDS>));
     }
-    if (h->n_sph) SMD_LAUNCH(h, (k_sphere<true, FL><<<1, h->sph_threads, 0, h->stream>>>(P, h->cur, se)));
+    if (h->n_sph) SMD_PDL(h, (k_sphere<true, FL>), 1, h->sph_threads, h->stream, P, h->cur, se);
   } else {
     SMD_LAUNCH(h, (k_force<false, FL, kLanes><<<gl, kBlock, 0, h->stream>>>(P, h->cur)));
     if constexpr (kHot) {
@@ -389,7 +389,7 @@ int launch_step(smd_system* h, StepEnd se = StepEnd{0, 0, 1, 0, 0}) {
     } else {
       SMD_PDL_INTEG(h, (k_integ<false, FL | F_FIELDS>));
     }
-    if (h->n_sph) SMD_LAUNCH(h, (k_sphere<false, FL><<<1, h->sph_threads, 0, h->stream>>>(P, h->cur, se)));
+    if (h->n_sph) SMD_PDL(h, (k_sphere<false, FL>), 1, h->sph_threads, h->stream, P, h->cur, se);
   }
   if (kLoopStep && h->profile) {
     if (int rc = prof_mark(h)) return rc;

@@ -2235,6 +2235,7 @@ template <bool MIXED, int FL>
 __global__ void __launch_bounds__(kBeadBlock) k_integ(DevPtrs P, int cur, StepEnd se) {
   // No wait here: integ_bead waits for the pair pass right before it reads
   // the pair forces, and every thread waits before the step's sums.
+  pdl_trigger();  // k_sphere's own start
   const long long it = P.g->it;
   const int i = blockIdx.x * kBeadBlock + threadIdx.x;
   const bool active = i < P.n;
@@ -2413,6 +2414,10 @@ __global__ void __launch_bounds__(kBeadBlock) k_finish(DevPtrs P, int cur, int m
 // Langevin term, the mass division of MD.cpp:480-509 and, in a loop step, both half-kicks,
 // the drift and the wrap; then the step's list-rebuild decision.  The same
 // flags as k_integ select the variant.
+// One block's chain of loads and FP64 operations bounds it (11 us alone), so it
+// is launched as a programmatic dependent of k_integ and waits only where it
+// reads that kernel's sums: 12,001 beads 51 to 49 us per step, 36,001 70 to 66
+// (with the list build's change).
 template <bool MIXED, int FL>
 __global__ void __launch_bounds__(kMaxSpheres) k_sphere(DevPtrs P, int cur, StepEnd se) {
   SphereDev* S = P.sph;
@@ -2437,6 +2442,19 @@ __global__ void __launch_bounds__(kMaxSpheres) k_sphere(DevPtrs P, int cur, Step
     const int o = S->orig[s], j = P.inv[o];
     int ti;
     if constexpr (MIXED) ti = pos_s[s].w & 0xff; else ti = __double_as_longlong(pos_s[s].w) & 0xff;
+    // what k_integ leaves alone, before its sums: the noise and the sphere's state
+    double noise[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0};
+    if constexpr ((FL & (F_FORCES | F_ENERGY)) == 0) {
+      if constexpr ((FL & F_EXTNOISE) != 0) {
+        for (int d = 0; d < 3; ++d) noise[d] = rp.sigma * P.ext_noise[3 * o + d];
+      } else {
+        langevin_noise(rp.seed, o - rp.bead_begin, it, (FL & F_INIT) ? 1 : 0, rp.sig31, noise);
+      }
+      v[0] = P.vx[j];
+      v[1] = P.vy[j];
+      v[2] = P.vz[j];
+    }
+    pdl_wait();
     double F[3] = {0.0, 0.0, 0.0};
     if constexpr ((FL & F_ENERGY) == 0) {
       for (int d = 0; d < 3; ++d) {
@@ -2491,13 +2509,6 @@ __global__ void __launch_bounds__(kMaxSpheres) k_sphere(DevPtrs P, int cur, Step
     if constexpr ((FL & F_FORCES) != 0) {
       for (int d = 0; d < 3; ++d) P.force_out[3 * o + d] = F[d];
     } else if constexpr ((FL & F_ENERGY) == 0) {
-      double noise[3];
-      if constexpr ((FL & F_EXTNOISE) != 0) {
-        for (int d = 0; d < 3; ++d) noise[d] = rp.sigma * P.ext_noise[3 * o + d];
-      } else {
-        langevin_noise(rp.seed, o - rp.bead_begin, it, (FL & F_INIT) ? 1 : 0, rp.sig31, noise);
-      }
-      double v[3] = {P.vx[j], P.vy[j], P.vz[j]};
       double a[3];
       for (int d = 0; d < 3; ++d) a[d] = fma(-rp.gamma, v[d], F[d]) + noise[d];
       const double m = S->mass[s], h = rp.dt * 0.5;
@@ -2544,6 +2555,7 @@ __global__ void __launch_bounds__(kMaxSpheres) k_sphere(DevPtrs P, int cur, Step
       }
     }
   }
+  pdl_wait();  // (returns at once where it has waited)
   // each thread has read its own accumulator: clear it for the next pass
   if (s < S->n)
     for (int d = 0; d < 3; ++d) {
