@@ -712,16 +712,20 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
           atomicAdd(&A.trial[me.rep].du_pair[par], sdu[0]);
           atomicAdd(&A.trial[me.rep].du_bond[par], sdu[1]);
         }
-        if (blockIdx.x == 0) {
-          A.sync->dmax[par ^ 1] = 0;
-          A.sync->shift[par ^ 1] = 0;
-        }
-        if (me.index == 0) {  // the previous trial's words: every CTA has read them
+        if (me.index == 0) {  // the previous trial's words: every CTA read them before the barrier that ended its step
           A.trial[me.rep].dq_pair[par ^ 1] = A.trial[me.rep].dq_bond[par ^ 1] = 0;
           A.trial[me.rep].du_pair[par ^ 1] = A.trial[me.rep].du_bond[par ^ 1] = 0.0;
         }
       }
       if (!barrier(1)) return;
+      // Past this barrier every CTA has read the previous trial's largest
+      // displacement and shift (after the barrier that ended its step, the last
+      // one before this where a period is one step); they are added to again
+      // after the barrier that ends this step.
+      if (tid == 0 && blockIdx.x == 0) {
+        A.sync->dmax[par ^ 1] = 0;
+        A.sync->shift[par ^ 1] = 0;
+      }
       if (tid == 0) {
         rs.dUq_pair = __ldcg(&A.trial[me.rep].dq_pair[par]);
         rs.dUq_bond = __ldcg(&A.trial[me.rep].dq_bond[par]);
