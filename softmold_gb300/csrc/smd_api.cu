@@ -152,7 +152,10 @@ struct smd_system {
       (void)cudaGetLastError();  // not the next launch's error
       return fail(100 + (int)e, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
-    e = cudaMemset(q, 0, bytes);
+    // On the handle's stream, as every later use of the array: that stream does
+    // not wait for the legacy one, where a clear could still be on its way when
+    // the array's first contents arrive.
+    e = cudaMemsetAsync(q, 0, bytes, stream);
     if (e != cudaSuccess) {
       (void)cudaGetLastError();
       cudaFree(q);
@@ -193,6 +196,13 @@ int check_launch(smd_system* h) {
   if (e != cudaSuccess) return fail(200 + (int)e, std::string("kernel launch: ") + cudaGetErrorString(e));
   h->launches++;
   return 0;
+}
+
+// Host data to the device, on the handle's stream and complete on return: a
+// copy on the legacy stream is not ordered with that stream's kernels.
+cudaError_t upload(cudaStream_t st, void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(st);
 }
 
 // Launch with programmatic stream serialization: the kernel may start while
@@ -545,8 +555,7 @@ int run_setup(smd_system* h) {
       (rc = h->alloc(&r.trial, (size_t)h->n_rep)) ||
       (rc = h->alloc(&r.place, place.size())))
     return rc;
-  SMD_CUDA(cudaMemcpyAsync(r.place, place.data(), place.size() * sizeof(RunPlace), cudaMemcpyHostToDevice, h->stream));
-  SMD_CUDA(cudaStreamSynchronize(h->stream));
+  SMD_CUDA(upload(h->stream, r.place, place.data(), place.size() * sizeof(RunPlace)));
   r.grid = grid;
   return 0;
 }
@@ -1092,9 +1101,9 @@ int smd_create_batch(const smd_system_desc* descs, int n_rep, int precision, smd
     sd.all_partners = (sd.nanocore || sd.n > kBeadBrute) ? 1 : 0;
     sd.grid = sd.nanocore ? (sd.n > kCoreBrute ? 1 : 0) : (sd.n > kBeadBrute ? 1 : 0);
     sd.grid_len = 2.0 * sphere_grid_range(d0);
-    SMD_CUDA(cudaMemcpy(P.sph, &sd, sizeof sd, cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(dC, d0.sphere_consts, nc * sizeof(double), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(fC, cf.data(), nc * sizeof(float), cudaMemcpyHostToDevice));
+    SMD_CUDA(upload(h->stream, P.sph, &sd, sizeof sd));
+    SMD_CUDA(upload(h->stream, dC, d0.sphere_consts, nc * sizeof(double)));
+    SMD_CUDA(upload(h->stream, fC, cf.data(), nc * sizeof(float)));
     P.sphC = dC;
     P.sphCf = fC;
     P.n_sph = sd.n;
@@ -1115,8 +1124,8 @@ int smd_create_batch(const smd_system_desc* descs, int n_rep, int precision, smd
       int* doff = nullptr;
       int4* dterms = nullptr;
       if ((rc = h->alloc(&doff, total + 1)) || (rc = h->alloc(&dterms, flat.size()))) return rc;
-      SMD_CUDA(cudaMemcpy(doff, off.data(), (total + 1) * sizeof(int), cudaMemcpyHostToDevice));
-      SMD_CUDA(cudaMemcpy(dterms, flat.data(), flat.size() * sizeof(int4), cudaMemcpyHostToDevice));
+      SMD_CUDA(upload(h->stream, doff, off.data(), (total + 1) * sizeof(int)));
+      SMD_CUDA(upload(h->stream, dterms, flat.data(), flat.size() * sizeof(int4)));
       P.term_off = doff;
       P.terms = dterms;
       P.n_terms = (int)flat.size();
@@ -1158,21 +1167,21 @@ int smd_create_batch(const smd_system_desc* descs, int n_rep, int precision, smd
         }
       }
     }
-    SMD_CUDA(cudaMemcpy(P.x, hx.data(), total * sizeof(double), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(P.y, hy.data(), total * sizeof(double), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(P.z, hz.data(), total * sizeof(double), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(P.vx, hvx.data(), total * sizeof(double), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(P.vy, hvy.data(), total * sizeof(double), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(P.vz, hvz.data(), total * sizeof(double), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(P.orig, orig.data(), total * sizeof(int), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(P.inv, orig.data(), total * sizeof(int), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(P.cinfo, cinfo.data(), total * sizeof(int), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(P.m4[0], m4.data(), total * sizeof(uint4), cudaMemcpyHostToDevice));
+    SMD_CUDA(upload(h->stream, P.x, hx.data(), total * sizeof(double)));
+    SMD_CUDA(upload(h->stream, P.y, hy.data(), total * sizeof(double)));
+    SMD_CUDA(upload(h->stream, P.z, hz.data(), total * sizeof(double)));
+    SMD_CUDA(upload(h->stream, P.vx, hvx.data(), total * sizeof(double)));
+    SMD_CUDA(upload(h->stream, P.vy, hvy.data(), total * sizeof(double)));
+    SMD_CUDA(upload(h->stream, P.vz, hvz.data(), total * sizeof(double)));
+    SMD_CUDA(upload(h->stream, P.orig, orig.data(), total * sizeof(int)));
+    SMD_CUDA(upload(h->stream, P.inv, orig.data(), total * sizeof(int)));
+    SMD_CUDA(upload(h->stream, P.cinfo, cinfo.data(), total * sizeof(int)));
+    SMD_CUDA(upload(h->stream, P.m4[0], m4.data(), total * sizeof(uint4)));
     if (!h->mixed)
-      SMD_CUDA(cudaMemcpy(P.d4[0], d4.data(), total * sizeof(double4), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(P.rp, h->rp.data(), n_rep * sizeof(RepParams), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(P.rs, rs.data(), n_rep * sizeof(RepState), cudaMemcpyHostToDevice));
-    SMD_CUDA(cudaMemcpy(tdev, &T, sizeof(Tables), cudaMemcpyHostToDevice));
+      SMD_CUDA(upload(h->stream, P.d4[0], d4.data(), total * sizeof(double4)));
+    SMD_CUDA(upload(h->stream, P.rp, h->rp.data(), n_rep * sizeof(RepParams)));
+    SMD_CUDA(upload(h->stream, P.rs, rs.data(), n_rep * sizeof(RepState)));
+    SMD_CUDA(upload(h->stream, tdev, &T, sizeof(Tables)));
   }
   if ((rc = run_setup(h.get()))) return rc;
   // ---- size the Verlet list: count pass with zero capacity, then the build
@@ -1193,7 +1202,7 @@ int smd_create_batch(const smd_system_desc* descs, int n_rep, int precision, smd
   g.it = h->it;
   g.trial_slot = 0;
   g.graph_builds = 0;
-  SMD_CUDA(cudaMemcpy(P.g, &g, sizeof(Global), cudaMemcpyHostToDevice));
+  SMD_CUDA(upload(h->stream, P.g, &g, sizeof(Global)));
   if ((rc = rebuild_if_needed(h.get()))) return rc;
   if ((rc = read_error(h.get()))) return rc;
   *out = h.release();
@@ -1257,7 +1266,7 @@ int smd_set_state(smd_system* h, const double* pos, const double* vel) {
   if (int rc = read_global(h, &g)) return rc;
   if (g.error & 4) {
     g.error &= ~4;
-    SMD_CUDA(cudaMemcpy(P.g, &g, sizeof(Global), cudaMemcpyHostToDevice));
+    SMD_CUDA(upload(h->stream, P.g, &g, sizeof(Global)));
     return fail(9, "smd_set_state: a position outside its replica's box or not finite, or a velocity that is "
                    "not finite (the handle's state is unchanged)");
   }
@@ -1265,7 +1274,7 @@ int smd_set_state(smd_system* h, const double* pos, const double* vel) {
     const int need = std::max(g.need_nbr, g.max_nbr);
     g.error &= ~1;
     g.need_nbr = 0;
-    SMD_CUDA(cudaMemcpy(P.g, &g, sizeof(Global), cudaMemcpyHostToDevice));
+    SMD_CUDA(upload(h->stream, P.g, &g, sizeof(Global)));
     if (int rc = grow_list(h, need)) return rc;
     return read_error(h);
   }
@@ -1585,7 +1594,7 @@ int autotune(smd_system* h, bool force) {
   h->tune.done = true;
   h->launches = saved;  // tuning launches are not step work
   SMD_CUDA(cudaStreamSynchronize(h->stream));
-  SMD_CUDA(cudaMemcpy(&P.g->n_rebuilds, &rebuilds0, sizeof rebuilds0, cudaMemcpyHostToDevice));
+  SMD_CUDA(upload(h->stream, &P.g->n_rebuilds, &rebuilds0, sizeof rebuilds0));
   drop_graphs(h);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -1830,8 +1839,8 @@ int smd_set_msd_groups(smd_system* h, int n_groups, const int* offsets, const in
     if (int rc = h->alloc(&off, (size_t)n_groups + 1)) return rc;
     if (int rc = h->alloc(&bd, (size_t)std::max(total, 1))) return rc;
     if (int rc = h->alloc(&out, (size_t)n_groups)) return rc;
-    SMD_CUDA(cudaMemcpy(off, offsets, sizeof(int) * ((size_t)n_groups + 1), cudaMemcpyHostToDevice));
-    if (total > 0) SMD_CUDA(cudaMemcpy(bd, beads, sizeof(int) * (size_t)total, cudaMemcpyHostToDevice));
+    SMD_CUDA(upload(h->stream, off, offsets, sizeof(int) * ((size_t)n_groups + 1)));
+    if (total > 0) SMD_CUDA(upload(h->stream, bd, beads, sizeof(int) * (size_t)total));
     M.off = off;
     M.beads = bd;
     M.msd = out;
