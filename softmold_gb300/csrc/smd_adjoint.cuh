@@ -19,8 +19,8 @@
 // constants 1 and 3 (include/MD.h:384-431, 683-789), so their derivatives
 // are the same kernels evaluated with derivative rows or unit constants.
 //
-// MIXED: pair terms in FP32 from the exact fractional mirror, summed as pairs
-// of FP32 (TwoSum), the adjoint state in FP64.  PLAIN: FP64 throughout.  The
+// MIXED: pair terms in FP32 from the exact fractional mirror, summed in three
+// FP32 words (Sum3, more bits than FP64), the adjoint state in FP64.  PLAIN: FP64 throughout.  The
 // CHAIN terms are FP64 in both, their K w the directional derivative of the
 // force formulas, written out.
 #pragma once
@@ -29,29 +29,38 @@
 
 namespace smd {
 
-// A sum of FP32 terms held as an unevaluated pair hi + lo (Knuth's TwoSum: the
-// rounding error of each addition, exact, is added to lo).  Its error, some
-// 2^-45 of the terms' magnitude, is far below the terms' own FP32 rounding, and
-// its seven FP32 instructions cost a tenth of an FP64 conversion and addition.
-struct Sum2 {
-  float hi = 0.f, lo = 0.f;
-  __device__ __forceinline__ void add(float x) {
-    const float s = __fadd_rn(hi, x);
-    const float b = __fsub_rn(s, hi);
-    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
-    hi = s;
+// A sum of FP32 terms held as three FP32 words (Knuth's TwoSum, cascaded: the
+// rounding error of each addition to a word, exact, is added to the next one;
+// Ogita, Rump and Oishi's K-fold summation with K = 3).  Its error is some
+// n^2 2^-70 of the terms' magnitude, below that of FP64 additions: on 52 terms
+// of which 40 cancel, in units of 2^-53 of the terms' total, FP64 0.42 at most,
+// three words 1e-6, two words 21.  Thirteen FP32 instructions a term cost a
+// fifth of an FP64 conversion and addition (two FP64 instructions).
+struct Sum3 {
+  float hi = 0.f, mid = 0.f, lo = 0.f;
+  // a + b in a, its rounding error returned
+  static __device__ __forceinline__ float two_sum(float& a, float b) {
+    const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+    a = s;
+    return e;
   }
-  __device__ __forceinline__ void add(const Sum2& o) {
+  __device__ __forceinline__ void add(float x) { lo = __fadd_rn(lo, two_sum(mid, two_sum(hi, x))); }
+  __device__ __forceinline__ void add(const Sum3& o) {
     add(o.hi);
-    lo = __fadd_rn(lo, o.lo);
+    lo = __fadd_rn(lo, __fadd_rn(two_sum(mid, o.mid), o.lo));
   }
-  __device__ __forceinline__ Sum2 from(int x) const {  // lane lane ^ x's
-    Sum2 o;
+  __device__ __forceinline__ Sum3 from(int x) const {  // lane lane ^ x's
+    Sum3 o;
     o.hi = __shfl_xor_sync(0xffffffffu, hi, x);
+    o.mid = __shfl_xor_sync(0xffffffffu, mid, x);
     o.lo = __shfl_xor_sync(0xffffffffu, lo, x);
     return o;
   }
-  __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+  // (an infinite or undefined sum is hi alone: the lower words of one are NaN)
+  __device__ __forceinline__ double value() const {
+    return isfinite(hi) ? (double)hi + ((double)mid + (double)lo) : (double)hi;
+  }
 };
 struct Sum1 {  // the plain form's sums
   double v = 0.0;
@@ -244,17 +253,19 @@ __device__ __forceinline__ void adj_add(const double (&v)[N], double* const (&ds
 // the Verlet list in stretches of kPairQueue entries: they first queue the
 // entries in range (about half) by a cheap FP32 test with a slightly wider cut,
 // then take the terms of full groups of queued entries.  The mixed form's sums
-// are Sum2, and the eight sums of a bead end on one lane each by a butterfly
+// are Sum3, and the eight sums of a bead end on one lane each by a butterfly
 // that halves what every lane still carries.  At 15,000 beads, per pass: each
-// term converted and added in FP64 92 us, Sum2 39, with the queue, the
-// butterfly and one atomic per CTA 28.
+// term converted and added in FP64 92 us, with Sum3, the queue, the butterfly and one
+// atomic per CTA 35.  The mixed form is held to three CTAs per SM (80 registers;
+// left to itself it takes 84, two CTAs and 45 us; four CTAs spill, 35 here and 5 %
+// more for a 10,000-lipid call).
 template <bool MIXED>
-__global__ void __launch_bounds__(kBlock) k_adj_pair(DevPtrs P, int cur, const AdjTables* AT,
+__global__ void __launch_bounds__(kBlock, MIXED ? 3 : 1) k_adj_pair(DevPtrs P, int cur, const AdjTables* AT,
                                                      const typename std::conditional<MIXED, float4, double4>::type* ws,
                                                      double* kw, double* fpair, AdjAcc* acc, double dt, double invT) {
   constexpr int G = 8;
   using R = typename std::conditional<MIXED, float, double>::type;
-  using Sum = typename std::conditional<MIXED, Sum2, Sum1>::type;
+  using Sum = typename std::conditional<MIXED, Sum3, Sum1>::type;
   __shared__ R tabs[4][6 * kMaxTypes * kMaxTypes];  // F, U and their Umin derivatives
   __shared__ int queues[kBlock / G][kPairQueue];
   const Tables& T = *P.tab;
