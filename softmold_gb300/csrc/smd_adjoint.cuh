@@ -82,9 +82,12 @@ struct Sum1 {  // the plain form's sums
 // for a bend of unit vectors a, b (lengths p, q), c = a . b, m = c0 - c:
 //   g1 = (m/p)(b - a c) on the first bead, g2 = (m/q)(a - b c) off the third,
 //   the second taking g2 - g1, with a' = (t_a - a (a . t_a)) / p and so on.
-// One reciprocal root per vector serves everything: the same terms by dual
-// numbers through sqrt and divisions took 1,280 FP64 instructions per warp and
-// 95 us at 15,000 beads, these 260 and 24 us.
+// One reciprocal root per vector serves everything, its quotients rounded by a
+// residual step: the same terms by dual numbers through sqrt and divisions took
+// 1,280 FP64 instructions per warp and 95 us at 15,000 beads, these 28 us with
+// the same error (3.91e-16 and 2.46e-16 of the rms derivative for a bilayer and
+// a vesicle, the dual numbers 3.92e-16 and 2.45e-16; with plain products by the
+// reciprocal 24 us, but 3.97e-16 and 2.63e-16).
 struct ChainDual {
   double fb[3] = {0, 0, 0}, tb[3] = {0, 0, 0};  // bonds: force, derivative
   double fn[3] = {0, 0, 0}, tn[3] = {0, 0, 0};  // bends
@@ -98,18 +101,19 @@ __device__ __forceinline__ double dot3(const double a[3], const double b[3]) {
 template <bool SUMS>
 __device__ __forceinline__ void chain_dual(const Vec3<double> e[4], const double t[4][3], const bool valid[4],
                                            const double* cd, ChainDual& c) {
-  double u[4][3], ri[4];  // unit vectors and reciprocal lengths
+  double u[4][3], rr[4], ri[4];  // unit vectors, lengths and their reciprocals
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    u[k][0] = u[k][1] = u[k][2] = ri[k] = 0.0;
+    u[k][0] = u[k][1] = u[k][2] = rr[k] = ri[k] = 0.0;
     if (!valid[k]) continue;
     const double d[3] = {e[k].x, e[k].y, e[k].z};
     const double r2 = dot3(d, d);
-    ri[k] = rsqrt(r2);
-    for (int a = 0; a < 3; ++a) u[k][a] = d[a] * ri[k];
+    const double r = rr[k] = root64(r2, ri[k]);
+    ri[k] = recip64(r, ri[k]);
+    for (int a = 0; a < 3; ++a) u[k][a] = div64(d[a], r, ri[k]);
     if (k == 1 || k == 2) {  // bonds (p-1, p) as second, (p, p+1) as first
       const double sg = k == 1 ? -1.0 : 1.0;
-      const double l = cd[0], lr = l * ri[k], A = sg * (lr - 1.0);
+      const double l = cd[0], lr = div64(l, r, ri[k]), A = sg * (lr - 1.0);
       const double B = sg * lr * dot3(u[k], t[k]);  // (l/r)(u . t)
       for (int a = 0; a < 3; ++a) {
         if constexpr (SUMS) c.fb[a] = fma(A, d[a], c.fb[a]);
@@ -117,7 +121,7 @@ __device__ __forceinline__ void chain_dual(const Vec3<double> e[4], const double
       }
       if constexpr (SUMS) {
         if (k == 2) {
-          const double x = fma(r2, ri[k], -l);
+          const double x = r - l;
           c.ub = 0.5 * x * x;
         }
       }
@@ -137,16 +141,17 @@ __device__ __forceinline__ void chain_dual(const Vec3<double> e[4], const double
       tb[x] = k == 0 ? t[1][x] : (k == 1 ? t[2][x] : t[3][x]);
     }
     const double ia = k == 0 ? ri[0] : (k == 1 ? ri[1] : ri[2]), ib = k == 0 ? ri[1] : (k == 1 ? ri[2] : ri[3]);
+    const double ra = k == 0 ? rr[0] : (k == 1 ? rr[1] : rr[2]), rb = k == 0 ? rr[1] : (k == 1 ? rr[2] : rr[3]);
     const double cs = dot3(a, b), m = cd[2] - cs;
     const double pa = dot3(a, ta), pb = dot3(b, tb);  // rates of the lengths
     double da[3], db[3];
     for (int x = 0; x < 3; ++x) {
-      da[x] = fma(-a[x], pa, ta[x]) * ia;
-      db[x] = fma(-b[x], pb, tb[x]) * ib;
+      da[x] = div64(fma(-a[x], pa, ta[x]), ra, ia);
+      db[x] = div64(fma(-b[x], pb, tb[x]), rb, ib);
     }
     const double dc = dot3(da, b) + dot3(a, db);
-    const double ma = m * ia, mb = m * ib;
-    const double na = fma(-ma, pa, -dc) * ia, nb = fma(-mb, pb, -dc) * ib;  // rates of m/p, m/q
+    const double ma = div64(m, ra, ia), mb = div64(m, rb, ib);
+    const double na = div64(fma(-ma, pa, -dc), ra, ia), nb = div64(fma(-mb, pb, -dc), rb, ib);  // rates of m/p, m/q
     const double s1 = k == 0 ? 0.0 : (k == 1 ? -1.0 : 1.0), s2 = k == 0 ? -1.0 : (k == 1 ? 1.0 : 0.0);
     for (int x = 0; x < 3; ++x) {
       const double va = fma(-a[x], cs, b[x]), vb = fma(-b[x], cs, a[x]);
