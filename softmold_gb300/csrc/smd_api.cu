@@ -471,6 +471,19 @@ int launch_run(smd_system* h, RunArgs a) {
     return r_.warps == 28 ? f<false, 8, 28>(__VA_ARGS__) : f<false, 8, 32>(__VA_ARGS__);   \
   }()
 
+// Whether the caller is capturing the handle's stream.  A captured advance is
+// replayed from other states, so what the host knows now (the step number that
+// the persistent loop is launched with, a rebuild flag that was read back
+// clear) must not shape what is recorded.
+bool being_captured(const smd_system* h) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->stream, &status) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return status != cudaStreamCaptureStatusNone;
+}
+
 // Whether the persistent loop can take this handle's next steps.
 bool run_ready(const smd_system* h) {
   return h->run.grid && h->use_graphs && !h->profile && !h->ext_noise_pending && !h->meas.tracking;
@@ -1627,6 +1640,8 @@ int smd_advance(smd_system* h, int steps, int flags) {
   // sparser than the running membrane and favours other kernels)
   if (!h->tune.done && h->it - h->first_step[0] >= 256 && autotune_enabled() && (rc = autotune(h, false)))
     return rc;
+  const bool captured = being_captured(h);
+  if (captured) h->list_ok = false;
   int done = 0;
   while (done < steps) {
     const int chunk = std::min(steps - done, kTrialChunk * std::max(1, h->resize_rate) / 2);
@@ -1634,7 +1649,7 @@ int smd_advance(smd_system* h, int steps, int flags) {
     for (int s = 0; s < chunk; ++s) {
       // the last step of a stopping call runs alone (it stops after its second half-kick)
       const int left = chunk - s - ((stop_at_measure && done + chunk == steps) ? 1 : 0);
-      if (left > 0 && run_ready(h)) {
+      if (left > 0 && !captured && run_ready(h)) {
         if ((rc = advance_run(h, left))) return rc;
         s += left - 1;
         continue;
