@@ -195,13 +195,23 @@ int smd_autotune(smd_system* h, int force, int* lanes, int* list_kernel, float* 
  * 16; list_kernel 0, 1 or 2) and marks the handle tuned. */
 int smd_set_tuning(smd_system* h, int lanes, int list_kernel);
 
-/* Launch mode of smd_advance: on = 1 (default) runs a stretch of steps of a
- * system or batch of up to 65,000 beads per replica (without spheres, BOND / BEND
- * or field terms) as one persistent cooperative kernel, and each barostat
- * period of any other as one CUDA graph whose list builds are
- * conditional nodes; on = 0 launches the same work kernel by kernel (profilers
- * that cannot see kernel nodes inside graphs with conditional nodes still see
- * each kernel).  No reference counterpart: the reference launches nothing. */
+/* Launch mode of smd_advance.  on = 1 (default): a stretch of steps runs as one
+ * persistent cooperative kernel where the handle allows it, that is a system
+ * or batch without spheres, BOND / BEND or field terms, of up to 65,000 beads
+ * and 81,920 list cells per replica, no more replicas than the GPU has SMs and
+ * no more beads per CTA than it has threads (some 155,000 beads on 152 SMs).  It
+ * does not while diffusion is tracked (smd_start_diffusion), under smd_profile,
+ * for the steps of a noise upload, for the last step of a SMD_STOP_AT_MEASURE
+ * call, while the caller captures the handle's stream, or beside the advances of
+ * two other handles on the GPU (of one, above 36,000 beads, plain form 3,000): those
+ * share the SMs, where persistent loops queue behind one another.  Everything
+ * else runs each barostat period as one CUDA graph whose list builds are
+ * conditional nodes.  The persistent loop takes every SM for its stretch: other
+ * work of the caller on the GPU waits for it, up to 4,096 steps at a time.
+ * on = 0 launches the same work kernel by kernel (profilers that cannot see
+ * kernel nodes inside graphs with conditional nodes still see each kernel), and
+ * leaves the SMs to others between kernels.  Mixed runs are bitwise the same
+ * either way.  No reference counterpart: the reference launches nothing. */
 int smd_use_graphs(smd_system* h, int on);
 
 /* Waits for the handle's stream and reports any device-side error. */

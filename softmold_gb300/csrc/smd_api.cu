@@ -142,6 +142,13 @@ struct smd_system {
   cudaStream_t side = nullptr;  // captures the conditional bodies
   long long graph_builds = 0;   // device count of list builds run inside graphs
   double* xfer = nullptr;       // 6n doubles: file-order positions and velocities for host copies
+  int device = 0;
+  // this handle among those whose advances may still run (advance_begin)
+  struct Flight {
+    bool in_call = false;         // inside a call; otherwise `done` tells
+    cudaEvent_t done = nullptr;   // behind the last asynchronous advance
+    int others = 0;               // most others seen beside the last advance (up to 2)
+  } flight;
 
   template <typename T>
   int alloc(T** p, size_t count) {
@@ -165,7 +172,10 @@ struct smd_system {
     *p = (T*)q;
     return 0;
   }
+  void leave_flight();
   ~smd_system() {
+    leave_flight();
+    if (flight.done) cudaEventDestroy(flight.done);
     if (stream) cudaStreamSynchronize(stream);
     for (auto& g : graph)
       if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -482,6 +492,86 @@ bool being_captured(const smd_system* h) {
     return false;
   }
   return status != cudaStreamCaptureStatusNone;
+}
+
+// Handles whose advances may still run, in the order of their starts.  The
+// persistent loop takes all SMs for a stretch of steps, so the loops of several
+// handles run one after another, where their single kernels run side by side.
+// Each advance therefore looks at how many others it overlaps.
+struct InFlight {
+  std::mutex mu;
+  std::vector<smd_system*> handles;
+};
+InFlight& in_flight() {  // (outlives every handle)
+  static InFlight* f = new InFlight;
+  return *f;
+}
+
+// Enters h's advance and returns how many other handles' advances on its
+// device it overlaps, up to two: those that run now or, if more, those that ran
+// beside its previous one (the first of several asynchronous calls meets none).
+int advance_begin(smd_system* h) {
+  InFlight& f = in_flight();
+  std::lock_guard<std::mutex> lock(f.mu);
+  // an event query from this thread does not disturb a capture of another one
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  smd_system* beside[2];
+  int now = 0;
+  size_t kept = 0;
+  for (smd_system* o : f.handles) {
+    if (o == h) continue;
+    if (now < 2 && o->device == h->device) {
+      if (!o->flight.in_call && cudaEventQuery(o->flight.done) != cudaErrorNotReady) continue;  // done
+      beside[now++] = o;
+    }
+    f.handles[kept++] = o;
+  }
+  f.handles.resize(kept);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (now) (void)cudaGetLastError();  // "not ready" is no launch's error
+  for (int k = 0; k < now; ++k) beside[k]->flight.others = std::max(beside[k]->flight.others, now);
+  const int others = std::max(now, h->flight.others);
+  h->flight.others = now;
+  h->flight.in_call = true;
+  f.handles.push_back(h);
+  return others;
+}
+
+// Leaves it: at once, or when the device has done what was queued.
+void advance_end(smd_system* h, bool queued) {
+  InFlight& f = in_flight();
+  std::lock_guard<std::mutex> lock(f.mu);
+  if (queued && (h->flight.done || cudaEventCreateWithFlags(&h->flight.done, cudaEventDisableTiming) == cudaSuccess) &&
+      cudaEventRecord(h->flight.done, h->stream) == cudaSuccess) {
+    h->flight.in_call = false;
+    return;
+  }
+  if (queued) (void)cudaGetLastError();
+  h->flight.in_call = false;
+  f.handles.erase(std::remove(f.handles.begin(), f.handles.end(), h), f.handles.end());
+}
+
+struct AdvanceScope {  // an advance that fails, or has been waited for, is over
+  smd_system* h;
+  ~AdvanceScope() {
+    if (h) advance_end(h, false);
+  }
+  void queued() {
+    if (h) advance_end(h, true);
+    h = nullptr;
+  }
+};
+
+// Whether an advance beside `others` others leaves the loop to its single
+// kernels.  us per step of all handles together, loop and kernels, two handles:
+// mixed 3,822 beads 31 and 39, 15,000 41 and 54, 29,400 70 and 71, 45,000 93 and
+// 87, 60,000 122 and 109; plain 1,176 beads 61 and 70, 4,611 105 and 100.  Three:
+// mixed 1,176 beads 36 and 38, 3,822 47 and 42, 15,000 62 and 64, 29,400 104 and
+// 93; plain 1,176 beads 92 and 73.  Eight: mixed 1,176 beads 94 and 47, 15,000 167
+// and 120; plain 1,176 beads 245 and 101.
+bool shares_device(const smd_system* h, int others) {
+  return others >= 2 || (others == 1 && h->n > (h->mixed ? 36000 : 3000));
 }
 
 // Whether the persistent loop can take this handle's next steps.
@@ -811,6 +901,8 @@ int validate(const smd_system_desc& d, std::string& why) {
 
 }  // namespace
 
+void smd_system::leave_flight() { advance_end(this, false); }
+
 extern "C" {
 
 int smd_last_error(char* buf, size_t len) {
@@ -1043,6 +1135,7 @@ int smd_create_batch(const smd_system_desc* descs, int n_rep, int precision, smd
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
       h->sms = sms;
+    h->device = dev;
   }
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(2, "cudaStreamCreate failed");
@@ -1642,14 +1735,18 @@ int smd_advance(smd_system* h, int steps, int flags) {
     return rc;
   const bool captured = being_captured(h);
   if (captured) h->list_ok = false;
+  AdvanceScope scope{captured ? nullptr : h};
   int done = 0;
   while (done < steps) {
+    // a long call looks again at every chunk, once the one before is through
+    if (done > 0 && !captured && h->run.grid) SMD_CUDA(cudaStreamSynchronize(h->stream));
+    const bool loop = !captured && !shares_device(h, advance_begin(h));
     const int chunk = std::min(steps - done, kTrialChunk * std::max(1, h->resize_rate) / 2);
     if ((rc = stage_trials(h, h->it, chunk))) return rc;
     for (int s = 0; s < chunk; ++s) {
       // the last step of a stopping call runs alone (it stops after its second half-kick)
       const int left = chunk - s - ((stop_at_measure && done + chunk == steps) ? 1 : 0);
-      if (left > 0 && !captured && run_ready(h)) {
+      if (left > 0 && loop && run_ready(h)) {
         if ((rc = advance_run(h, left))) return rc;
         s += left - 1;
         continue;
@@ -1691,7 +1788,10 @@ int smd_advance(smd_system* h, int steps, int flags) {
     }
     done += chunk;
   }
-  if (async) return 0;
+  if (async) {
+    scope.queued();
+    return 0;
+  }
   return smd_sync(h);
 }
 
@@ -2107,7 +2207,8 @@ int smd_adjoint(smd_system* h, const smd_adjoint_spec* spec, smd_adjoint_result*
       h->it = cp_it[c];
       SMD_LAUNCH(h, k_set_counters<<<1, 1, 0, h->stream>>>(P.g, h->it, 1, 0, 0));
       // recompute x_n of the segment (the persistent loop saves them as it goes)
-      const bool whole = len > 1 && run_ready(h);
+      AdvanceScope scope{h};
+      const bool whole = len > 1 && !shares_device(h, advance_begin(h)) && run_ready(h);
       for (int m = 0; m < (whole ? 1 : len); ++m) {
         SMD_LAUNCH(h, k_state_save<<<h->grid(), kBlock, 0, h->stream>>>(P, seg + (size_t)m * n3, nullptr));
         if (m + 1 < len && !whole)
@@ -2115,6 +2216,7 @@ int smd_adjoint(smd_system* h, const smd_adjoint_spec* spec, smd_adjoint_result*
       }
       if (whole)
         if (int r = advance_run(h, len - 1, seg + n3)) return r;
+      scope.queued();
       for (int m = len - 1; m >= 0; --m) {
         if (int r = adj_load(h, seg + (size_t)m * n3, nullptr, false)) return r;
         if (int r = adj_pair_pass(h, w, dt, invT)) return r;
