@@ -1354,10 +1354,10 @@ int smd_set_state(smd_system* h, const double* pos, const double* vel) {
   double* vs = h->xfer + n3;
   if (pos) SMD_CUDA(cudaMemcpyAsync(xs, pos, n3 * sizeof(double), cudaMemcpyHostToDevice, h->stream));
   if (vel) SMD_CUDA(cudaMemcpyAsync(vs, vel, n3 * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  // One round trip: a refused state (bit 2 of the error word) is not loaded,
-  // and a new configuration may be denser than the list was sized for, so the
-  // list is built here; if a bead overflowed, it grows to the count and is
-  // built again.
+  // One round trip: a refused state (bit 2 of the error word) is not loaded and
+  // nothing is rebuilt for it.  A new configuration may be denser than the list
+  // was sized for, so the list is built here; if a bead overflowed, it grows to
+  // the count and is built again.
   SMD_LAUNCH(h, k_state_check<<<h->grid(), kBlock, 0, h->stream>>>(P, pos ? xs : nullptr, vel ? vs : nullptr));
   SMD_LAUNCH(h, k_state_load<<<h->grid(), kBlock, 0, h->stream>>>(P, pos ? xs : nullptr, vel ? vs : nullptr));
   if (pos) {
@@ -1372,7 +1372,9 @@ int smd_set_state(smd_system* h, const double* pos, const double* vel) {
   if (int rc = read_global(h, &g)) return rc;
   if (g.error & 4) {
     g.error &= ~4;
+    if (pos) g.rebuild = g.held_rebuild;
     SMD_CUDA(upload(h->stream, P.g, &g, sizeof(Global)));
+    h->list_ok = g.rebuild == 0;
     return fail(9, "smd_set_state: a position outside its replica's box or not finite, or a velocity that is "
                    "not finite (the handle's state is unchanged)");
   }

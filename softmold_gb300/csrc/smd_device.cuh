@@ -151,7 +151,8 @@ struct Global {  // single instance
   float last_disp;
   unsigned int blocks_done;    // last-block counter
   int rebuild;                 // 1: rebuild the Verlet list before the next force pass
-  int error;                   // bit 0: list overflow, bit 1: cell overflow (>kMaxCell), bit 2: refused set_state input
+  int error;                   // bit 0: list overflow, bit 1: cell overflow (>kMaxCell), bit 2: refused set_state input,
+                               // bit 3: the persistent loop gave up waiting for its CTAs
   int need_nbr;                // largest neighbour count seen on overflow
   int max_nbr;                 // largest neighbour count of any list build so far
   int trial_slot;              // staged barostat trial used by the next MC step
@@ -159,6 +160,7 @@ struct Global {  // single instance
   long long graph_builds;      // list builds run inside graph conditional bodies
   int n_occ;                   // occupied list cells of the current build
   int next_cell;               // work queue of the list kernels over occ[]
+  int held_rebuild;            // the rebuild flag of before a refused set_state
 };
 
 // Bookkeeping of the kernel that completes a step (its last block): advance

@@ -2616,7 +2616,7 @@ __global__ void __launch_bounds__(kMaxSpheres) k_sphere(DevPtrs P, int cur, Step
 template <bool MIXED>
 __global__ void __launch_bounds__(kBlock) k_mirror(DevPtrs P, int cur) {
   const int i = blockIdx.x * kBlock + threadIdx.x;
-  if (i >= P.n) return;
+  if (i >= P.n || (P.g->error & 4)) return;  // (a refused state is not loaded)
   const int r = rep_of(P, i);
   const RepState& rs = P.rs[r];
   P.m4[cur][i] = make_uint4(to_frac(P.x[i], rs.frac_per_len[0]), to_frac(P.y[i], rs.frac_per_len[1]),
@@ -2670,7 +2670,14 @@ __global__ void __launch_bounds__(kBlock) k_state_check(DevPtrs P, const double*
 
 __global__ void __launch_bounds__(kBlock) k_state_load(DevPtrs P, const double* xs, const double* vs) {
   const int i = blockIdx.x * kBlock + threadIdx.x;
-  if (i >= P.n || (P.g->error & 4)) return;  // (k_state_check refused it)
+  if (i >= P.n) return;
+  if (P.g->error & 4) {  // k_state_check refused it: a pending rebuild waits for the next call
+    if (xs && i == 0) {
+      P.g->held_rebuild = P.g->rebuild;
+      P.g->rebuild = 0;
+    }
+    return;
+  }
   if (xs && i == 0) P.g->rebuild = 1;
   const int o = P.orig[i];
   if (xs) {
