@@ -635,6 +635,12 @@ int run_setup(smd_system* h) {
     if (ctas_at(mid) <= ctas) hi = mid; else lo = mid + 1;
   }
   r.beads = lo;
+  // Lanes per bead, so that few beads still make tasks for the warps.  us per step
+  // with 32, 16 and 8 lanes by beads per CTA, mixed form: 8 12.2 / 12.5 / 14.2, 16
+  // 14.5 / 14.8 / 16.1, 24 15.6 / 15.9 / 17.1, 28 16.4 / 15.2 / 16.5, 40 18.0 / 16.9
+  // / 18.0, 46 18.2 / 17.1 / 18.0, 52 19.5 / 19.0 / 18.4, 60 20.7 / 20.1 / 19.5.  The
+  // plain form, bound by FP64, would take fewer lanes sooner: 8 31.1 / 27.6 / 34.2,
+  // 16 42.8 / 37.7 / 37.4, 24 50.0 / 45.3 / 42.1, 46 75.0 / 64.2 / 60.3.
   r.lanes = r.beads <= 24 ? 32 : (r.beads <= 48 ? 16 : 8);
   r.warps = run_warps(r.beads, r.lanes);
   r.threads = 32 * std::min(r.warps, std::max(24, run_tasks(r.beads, r.lanes)));
@@ -983,7 +989,6 @@ int smd_create_batch(const smd_system_desc* descs, int n_rep, int precision, smd
   T.rcf = (float)d0.cutoff;
   T.rc2f = (float)(d0.cutoff * d0.cutoff);
   T.list_cut = d0.cutoff + h->skin;
-  T.list_cut2 = T.list_cut * T.list_cut;
   T.list_cut_f = (float)T.list_cut;
   double maxF = 1.0;
   for (int k = 0; k < d0.n_types * d0.n_types; ++k) {

@@ -179,8 +179,7 @@ struct Tables {  // force/potential tables (float and double) in constant-like m
   int n_sets;
   float rc2f, rcf;
   double rc2, rc;
-  double list_cut2;  // (rc+skin)^2
-  double list_cut;
+  double list_cut;   // rc + skin
   float list_cut_f;
   float fscale;      // fixed-point scale of one pair force (2^k)
   double inv_fscale;
@@ -279,13 +278,6 @@ __device__ __forceinline__ int cell_coord(double p, double cs, int n) {
   int c = int(p / cs);
   c = (c >= n) ? c - 1 : c;
   return c;
-}
-
-// Cell coordinate on the Verlet-list grid, clamped into [0, n) so that a bead
-// outside the box (a blown-up run) can never index outside the cell arrays.
-__device__ __forceinline__ int list_cell_coord(double p, double cs, int n) {
-  int c = cell_coord(p, cs, n);
-  return c < 0 ? 0 : (c >= n ? n - 1 : c);
 }
 
 __device__ __forceinline__ unsigned int to_frac(double x, double frac_per_len) {
@@ -410,15 +402,6 @@ __device__ __forceinline__ void trial_box(const double box[3], double dlxy, doub
 }
 
 // ------------------------------------------------------------------ potentials
-// Pair force magnitude with the reference's table index trick
-// (include/MD.h:811-825): force on i = mag * d.
-template <typename R>
-__device__ __forceinline__ R pair_mag(const R* c, R r) {
-  int ci = int(r / c[0]) * 3;
-  ci = ci > 3 ? 3 : ci;  // rows hold two segments; the tables use rc = 2 rm
-  R m = c[ci] - r;
-  return ((c[ci + 1] - c[ci + 2] * m) * m) / r;
-}
 // Pair potential (include/MD.h:913-926).
 template <typename R>
 __device__ __forceinline__ R pair_pot(const R* c, R r) {

@@ -716,10 +716,11 @@ __global__ void __launch_bounds__(kOctThreads) k_nbr_cells_oct(DevPtrs P, int cu
 //
 // Both forms build their lists here.  The list is a filter (the pair passes
 // test every entry's distance), so FP32 tests of the fractional mirror serve
-// with a wider cut (list_reach), and in the plain form by the mirror's
-// resolution too.  Testing in FP64 took 594 us
-// per build of an 18,003-bead vesicle, bound by the FP64 pipe.
-// The list cut widened by more than FP32 tests can be off.  In cells of width w
+// with a wider cut (list_reach).  Testing in FP64 took 594 us per build of an
+// 18,003-bead vesicle, bound by the FP64 pipe.
+
+// The list cut widened by more than FP32 tests can be off, and in the plain form
+// by the mirror's resolution.  In cells of width w
 // an expanded square's terms stay below 36 w^2 (offsets from a bead of the
 // stencil's middle cell; from its centre, half that), its rounding below 2e-5
 // w^2 or 1e-5 w^2 / L of the distance.

@@ -5,9 +5,10 @@
 // step kernels and, every second step, four list kernels of 5-25 us each that
 // keep at most a tenth of the chip's warps busy.  At tens of thousands the
 // launches' starts and tails, the reordered state's way through memory and one
-// list cell per CTA still cost a quarter of a step.  us per step, kernel by
-// kernel and here: 1,176 beads 35 and 14, 15,000 41 and 23, 24,000 54 and 31,
-// 33,000 64 and 37, 60,000 83 and 63.  Here every CTA owns a contiguous range of the
+// list cell per CTA still cost a quarter of a step.  us per step at a skin of
+// 0.5, kernel by kernel and here: 1,176 beads 32 and 12, 15,000 41 and 21, 22,500
+// 51 and 32, 29,400 57 and 35, 45,000 63 and 47, 60,000 75 and 61 (57 at a skin
+// of 0.42).  Here every CTA owns a contiguous range of the
 // cell-sorted beads and keeps their positions, velocities and bookkeeping in
 // shared memory; only the position mirror goes through global memory.  A step
 // is one grid barrier: each CTA forms its beads' pair sums (and beside them
@@ -30,8 +31,13 @@ namespace smd {
 // Warps per CTA at most, which set the registers per thread: 24 (80 registers)
 // where a CTA has few beads; with many, 28 (72) or 32 (64), whichever takes
 // their pair and bonded tasks in fewer rounds, 28 if both do: fewer spills then
-// count for more (395 beads per CTA, 112 tasks: 129,000 cycles per step against
-// 137,000; 99 beads, 29 tasks: 48,500 against 45,600).
+// count for more.  us per step with 28 and 32 warps, by beads per CTA (tasks),
+// bilayers in the mixed form: 60 (17) 19.4 and 19.8, 79 (23) 20.8 and 21.1, 98
+// (29) 21.7 and 22.0, 109 (32) 26.9 and 23.9, 119 (34) 29.0 and 26.4 (the rule
+// takes 28), 139 (40) 30.4 and 32.1, 168 (48) 32.8 and 34.2, 198 (57) 35.2 and
+// 35.8, 227 (65) 40.2 and 37.2, 257 (74) 44.6 and 46.3, 297 (85) 46.7 and 48.3,
+// 336 (95) 55.2 and 52.3, 390 (111) 59.5 and 61.9, 422 (120) 64.0 and 63.7.  The
+// plain form, bound by FP64, differs by 1 % (227: 234 and 229, the others 28).
 __host__ __device__ constexpr int run_tasks(int beads, int lanes) {
   return (beads * lanes + 31) / 32 + (beads + 31) / 32;
 }
@@ -399,7 +405,6 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
       k |= (unsigned long long)(ref_cell_coord(x[d], rs.ref_cs[d], rs.ref_inv_cs[d], rs.refn[d]) & 0x1fffff) << (21 * d);
     return k;
   };
-  // the trial of a barostat step: every CTA draws it into its own copy
   // exclusive sum of v over the block's threads, and the total (scratch: 32
   // words; the caller synchronises before it is used again)
   auto block_scan = [&](int v, int* scratch, int& total) {
@@ -421,6 +426,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
     const int before = __shfl_sync(0xffffffffu, t, warp > 0 ? warp - 1 : 0);
     return (warp > 0 ? before : 0) + x - v;
   };
+  // the trial of a barostat step: every CTA draws it into its own copy
   auto draw = [&]() {
     if (tid == 0) draw_trial(rs, rp, P.trial_u[((size_t)slot * P.n_rep + me.rep) * 2]);
   };
