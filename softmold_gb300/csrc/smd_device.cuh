@@ -183,7 +183,7 @@ struct Tables {  // force/potential tables (float and double) in constant-like m
   float list_cut_f;
   float fscale;      // fixed-point scale of one pair force (2^k)
   double inv_fscale;
-  float fF[6 * kMaxTypes * kMaxTypes];
+  alignas(64) float fF[6 * kMaxTypes * kMaxTypes];  // (8 bytes lower, a small system's step took 1 % more)
   float fU[6 * kMaxTypes * kMaxTypes];
   double dF[6 * kMaxTypes * kMaxTypes];
   double dU[6 * kMaxTypes * kMaxTypes];

@@ -727,8 +727,9 @@ __global__ void __launch_bounds__(NW * 32, 1) k_run(DevPtrs P, RunArgs A) {
       // Past this barrier every CTA has read the previous trial's largest
       // displacement and shift (after the barrier that ended its step, the last
       // one before this where a period is one step); they are added to again
-      // after the barrier that ends this step.
-      if (tid == 0 && blockIdx.x == 0) {
+      // after the barrier that ends this step.  (Not by thread 0, whose decision
+      // the whole CTA waits for.)
+      if (tid == 32 && blockIdx.x == 0) {
         A.sync->dmax[par ^ 1] = 0;
         A.sync->shift[par ^ 1] = 0;
       }
