@@ -109,7 +109,6 @@ __device__ __forceinline__ void chain_dual(const Vec3<double> e[4], const double
     const double d[3] = {e[k].x, e[k].y, e[k].z};
     const double r2 = dot3(d, d);
     const double r = rr[k] = root64(r2, ri[k]);
-    ri[k] = recip64(r, ri[k]);
     for (int a = 0; a < 3; ++a) u[k][a] = div64(d[a], r, ri[k]);
     if (k == 1 || k == 2) {  // bonds (p-1, p) as second, (p, p+1) as first
       const double sg = k == 1 ? -1.0 : 1.0;

@@ -18,11 +18,9 @@ __device__ __forceinline__ double root64(double r2, double& rinv) {
   return __double_as_longlong(r2) != 0 ? fma(fma(-r, r, r2), 0.5 * rinv, r) : 0.0;  // coincident beads
 }
 
-// 1 / r for r = root64(r2) from the reciprocal root, and a / r from 1 / r: one
-// Newton step and one residual step (Markstein, "Computation of elementary
-// functions on the IBM RISC System/6000 processor", 1990), which round them as
-// the division does but for rare last-bit cases.
-__device__ __forceinline__ double recip64(double r, double rinv) { return fma(fma(-r, rinv, 1.0), rinv, rinv); }
+// a / r for r = root64(r2) from the reciprocal root: one residual step
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990) rounds it as the division does but for rare last-bit cases.
 __device__ __forceinline__ double div64(double a, double r, double rinv) {
   const double q = a * rinv;
   return fma(fma(-q, r, a), rinv, q);
