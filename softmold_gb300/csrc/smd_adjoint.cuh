@@ -84,8 +84,8 @@ struct Sum1 {  // the plain form's sums
 //   the second taking g2 - g1, with a' = (t_a - a (a . t_a)) / p and so on.
 // One reciprocal root per vector serves everything, its quotients rounded by a
 // residual step: the same terms by dual numbers through sqrt and divisions took
-// 1,280 FP64 instructions per warp and 95 us at 15,000 beads, these 28 us with
-// the same error (3.91e-16 and 2.46e-16 of the rms derivative for a bilayer and
+// 1,280 FP64 instructions per warp and 95 us at 15,000 beads, these 28 us in the
+// same CTAs of 256 threads (17 in CTAs of 64) with the same error (3.91e-16 and 2.46e-16 of the rms derivative for a bilayer and
 // a vesicle, the dual numbers 3.92e-16 and 2.45e-16; with plain products by the
 // reciprocal 24 us, but 3.97e-16 and 2.63e-16).
 struct ChainDual {
@@ -234,9 +234,9 @@ __global__ void __launch_bounds__(kBlock) k_adj_wsort(DevPtrs P, const double* w
 // Adds v to *dst once per CTA, where any lane of it has a part: one address
 // takes one atomic after another, 2-3 ns each.  Called by the whole CTA, N
 // quantities at once.
-template <int N>
+template <int NT, int N>
 __device__ __forceinline__ void adj_add(const double (&v)[N], double* const (&dst)[N]) {
-  __shared__ double part[N][kBlock / 32];
+  __shared__ double part[N][NT / 32];
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     const double x = warp_sum(v[k]);
@@ -245,7 +245,7 @@ __device__ __forceinline__ void adj_add(const double (&v)[N], double* const (&ds
   __syncthreads();
   if (threadIdx.x < N) {
     double x = 0.0;
-    for (int u = 0; u < kBlock / 32; ++u) x += part[threadIdx.x][u];
+    for (int u = 0; u < NT / 32; ++u) x += part[threadIdx.x][u];
 #pragma unroll
     for (int k = 0; k < N; ++k)
       if (threadIdx.x == k && x != 0.0) atomicAdd(dst[k], x);
@@ -260,20 +260,24 @@ __device__ __forceinline__ void adj_add(const double (&v)[N], double* const (&ds
 // are Sum3, and the eight sums of a bead end on one lane each by a butterfly
 // that halves what every lane still carries.  At 15,000 beads, per pass: each
 // term converted and added in FP64 92 us, with Sum3, the queue, the butterfly and one
-// atomic per CTA 35.  The mixed form is held to three CTAs per SM (80 registers;
-// left to itself it takes 84, two CTAs and 45 us; four CTAs spill, 35 here and 5 %
-// more for a 10,000-lipid call).
+// atomic per CTA 30.  Sum3's words take 84 registers, which leave an SM 20 warps;
+// CTAs of 128 threads held to seven per SM (72 registers) leave it 28 and a finer
+// last wave.  A 40-step call at 15,000 and 18,300 beads (chain pass in CTAs of 256):
+// 5.61 and 6.77 ms, with six per SM (80 registers) 5.75 and 6.92, with eight (64,
+// 92 bytes spilled) 5.72 and 6.56 but 2 % more at 1,176 and 24,000, as three CTAs
+// of 256 threads 5.74 and 6.95.
+constexpr int kAdjThreads = 128;
 template <bool MIXED>
-__global__ void __launch_bounds__(kBlock, MIXED ? 3 : 1) k_adj_pair(DevPtrs P, int cur, const AdjTables* AT,
+__global__ void __launch_bounds__(kAdjThreads, MIXED ? 7 : 1) k_adj_pair(DevPtrs P, int cur, const AdjTables* AT,
                                                      const typename std::conditional<MIXED, float4, double4>::type* ws,
                                                      double* kw, double* fpair, AdjAcc* acc, double dt, double invT) {
   constexpr int G = 8;
   using R = typename std::conditional<MIXED, float, double>::type;
   using Sum = typename std::conditional<MIXED, Sum3, Sum1>::type;
   __shared__ R tabs[4][6 * kMaxTypes * kMaxTypes];  // F, U and their Umin derivatives
-  __shared__ int queues[kBlock / G][kPairQueue];
+  __shared__ int queues[kAdjThreads / G][kPairQueue];
   const Tables& T = *P.tab;
-  for (int k = threadIdx.x; k < 6 * T.nT * T.nT; k += kBlock) {
+  for (int k = threadIdx.x; k < 6 * T.nT * T.nT; k += kAdjThreads) {
     if constexpr (MIXED) {
       tabs[0][k] = T.fF[k];
       tabs[1][k] = T.fU[k];
@@ -287,7 +291,7 @@ __global__ void __launch_bounds__(kBlock, MIXED ? 3 : 1) k_adj_pair(DevPtrs P, i
     }
   }
   __syncthreads();
-  const int t = blockIdx.x * kBlock + threadIdx.x;
+  const int t = blockIdx.x * kAdjThreads + threadIdx.x;
   const int sub = t % G, lane = threadIdx.x & 31;
   const bool active = t / G < P.n;
   const int i = active ? t / G : 0, nn = active ? P.nnbr[i] : 0;
@@ -399,7 +403,7 @@ __global__ void __launch_bounds__(kBlock, MIXED ? 3 : 1) k_adj_pair(DevPtrs P, i
   if (active && sub < 6) (sub < 3 ? fpair : kw)[i + (sub % 3) * P.n] = mysum;
   // replica sums (single-system handles): J and the Umin component
   const double gJ = sub == 6 ? invT * mysum : 0.0, g0 = sub == 7 ? dt * swft.value() + invT * mysum : 0.0;
-  adj_add<2>({gJ, g0}, {&acc->J, &acc->grad[0]});
+  adj_add<kAdjThreads, 2>({gJ, g0}, {&acc->J, &acc->grad[0]});
 }
 
 // Differences of w along the chain of file-order bead o (file order is chain
@@ -415,11 +419,15 @@ __device__ __forceinline__ void chain_tangents(const double* w, int o, const boo
 //   xbar += dt (K w)_i - invT F_i, hbar = (1 - gamma dt) w_i,
 //   w_next = hbar + dt xbar.
 // Adds invT U_chain and the kbond / kbend components to the accumulators.
+// Bound by FP64: 15,000 beads are 59 CTAs of 256 threads, on as many SMs, 28 us;
+// CTAs of 64 reach every SM's pipe, 17 us (a 40-step call of 1,176, 15,000 and
+// 24,000 beads: 4.14, 5.61 and 7.25 ms against 3.65, 5.21 and 6.99).
+constexpr int kChainThreads = 64;
 template <bool MIXED>
-__global__ void __launch_bounds__(kBlock) k_adj_chain(DevPtrs P, int cur, const double* w, double* w_next,
+__global__ void __launch_bounds__(kChainThreads) k_adj_chain(DevPtrs P, int cur, const double* w, double* w_next,
                                                       double* xbar, double* hbar, const double* kw,
                                                       const double* fpair, AdjAcc* acc, double dt, double invT) {
-  const int i = blockIdx.x * kBlock + threadIdx.x;
+  const int i = blockIdx.x * kChainThreads + threadIdx.x;
   double gJ = 0.0, g1 = 0.0, g2 = 0.0;
   if (i < P.n) {
     const Tables& T = *P.tab;
@@ -459,7 +467,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_chain(DevPtrs P, int cur, const 
       w_next[3 * o + d] = hb + dt * xb;
     }
   }
-  adj_add<3>({gJ, g1, g2}, {&acc->J, &acc->grad[1], &acc->grad[2]});
+  adj_add<kChainThreads, 3>({gJ, g1, g2}, {&acc->J, &acc->grad[1], &acc->grad[2]});
 }
 
 // (K w)_i of the full conservative force at the current positions, file

@@ -2076,16 +2076,16 @@ int adj_alloc(smd_system* h) {
 int adj_pair_pass(smd_system* h, const double* w, double dt, double invT) {
   auto& P = h->P;
   auto& A = h->adj;
-  const int g = h->grid(), gl = h->grid_lanes();
+  const int g = h->grid(), gl = (int)((8LL * h->n + kAdjThreads - 1) / kAdjThreads);
   if (h->mixed) {
     float4* ws = reinterpret_cast<float4*>(A.ws);
     SMD_LAUNCH(h, k_adj_wsort<float4><<<g, kBlock, 0, h->stream>>>(P, w, ws));
-    SMD_LAUNCH(h, (k_adj_pair<true><<<gl, kBlock, 0, h->stream>>>(P, h->cur, A.tab, ws, A.kw, A.fpair,
-                                                                            A.acc, dt, invT)));
+    SMD_LAUNCH(h, (k_adj_pair<true><<<gl, kAdjThreads, 0, h->stream>>>(P, h->cur, A.tab, ws, A.kw, A.fpair, A.acc, dt,
+                                                                       invT)));
   } else {
     SMD_LAUNCH(h, k_adj_wsort<double4><<<g, kBlock, 0, h->stream>>>(P, w, A.ws));
-    SMD_LAUNCH(h, (k_adj_pair<false><<<gl, kBlock, 0, h->stream>>>(P, h->cur, A.tab, A.ws, A.kw,
-                                                                             A.fpair, A.acc, dt, invT)));
+    SMD_LAUNCH(h, (k_adj_pair<false><<<gl, kAdjThreads, 0, h->stream>>>(P, h->cur, A.tab, A.ws, A.kw, A.fpair, A.acc,
+                                                                        dt, invT)));
   }
   return 0;
 }
@@ -2227,11 +2227,12 @@ int smd_adjoint(smd_system* h, const smd_adjoint_spec* spec, smd_adjoint_result*
       for (int m = len - 1; m >= 0; --m) {
         if (int r = adj_load(h, seg + (size_t)m * n3, nullptr, false)) return r;
         if (int r = adj_pair_pass(h, w, dt, invT)) return r;
+        const int gc = (h->n + kChainThreads - 1) / kChainThreads;
         if (h->mixed)
-          SMD_LAUNCH(h, k_adj_chain<true><<<h->grid(), kBlock, 0, h->stream>>>(P, h->cur, w, wn, A.xbar, A.hbar,
-                                                                               A.kw, A.fpair, A.acc, dt, invT));
+          SMD_LAUNCH(h, k_adj_chain<true><<<gc, kChainThreads, 0, h->stream>>>(P, h->cur, w, wn, A.xbar, A.hbar, A.kw,
+                                                                               A.fpair, A.acc, dt, invT));
         else
-          SMD_LAUNCH(h, k_adj_chain<false><<<h->grid(), kBlock, 0, h->stream>>>(P, h->cur, w, wn, A.xbar, A.hbar,
+          SMD_LAUNCH(h, k_adj_chain<false><<<gc, kChainThreads, 0, h->stream>>>(P, h->cur, w, wn, A.xbar, A.hbar,
                                                                                 A.kw, A.fpair, A.acc, dt, invT));
         std::swap(w, wn);
       }
