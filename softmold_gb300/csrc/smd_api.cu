@@ -513,23 +513,29 @@ InFlight& in_flight() {  // (outlives every handle)
 int advance_begin(smd_system* h) {
   InFlight& f = in_flight();
   std::lock_guard<std::mutex> lock(f.mu);
-  // an event query from this thread does not disturb a capture of another one
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  cudaThreadExchangeStreamCaptureMode(&mode);
   smd_system* beside[2];
   int now = 0;
   size_t kept = 0;
+  // an event query from a thread in the relaxed mode does not disturb another thread's capture
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  bool queried = false;
   for (smd_system* o : f.handles) {
     if (o == h) continue;
     if (now < 2 && o->device == h->device) {
-      if (!o->flight.in_call && cudaEventQuery(o->flight.done) != cudaErrorNotReady) continue;  // done
+      if (!o->flight.in_call) {
+        if (!queried) cudaThreadExchangeStreamCaptureMode(&mode);
+        queried = true;
+        if (cudaEventQuery(o->flight.done) != cudaErrorNotReady) continue;  // done
+      }
       beside[now++] = o;
     }
     f.handles[kept++] = o;
   }
   f.handles.resize(kept);
-  cudaThreadExchangeStreamCaptureMode(&mode);
-  if (now) (void)cudaGetLastError();  // "not ready" is no launch's error
+  if (queried) {
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    (void)cudaGetLastError();  // "not ready" is no launch's error
+  }
   for (int k = 0; k < now; ++k) beside[k]->flight.others = std::max(beside[k]->flight.others, now);
   const int others = std::max(now, h->flight.others);
   h->flight.others = now;
@@ -1746,7 +1752,8 @@ int smd_advance(smd_system* h, int steps, int flags) {
   int done = 0;
   while (done < steps) {
     // a long call looks again at every chunk, once the one before is through
-    if (done > 0 && !captured && h->run.grid) SMD_CUDA(cudaStreamSynchronize(h->stream));
+    // (an asynchronous one does not wait)
+    if (done > 0 && !async && h->run.grid) SMD_CUDA(cudaStreamSynchronize(h->stream));
     const bool loop = !captured && !shares_device(h, advance_begin(h));
     const int chunk = std::min(steps - done, kTrialChunk * std::max(1, h->resize_rate) / 2);
     if ((rc = stage_trials(h, h->it, chunk))) return rc;
