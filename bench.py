@@ -8,21 +8,22 @@ mixed precision.  Seeded synthetic input built in the reference generator's
 geometry, equilibrated for 1,000 untimed steps.
 
 One bench step = 80 MD loop iterations (MD.cpp:335-729), ten barostat
-periods of resizeRate 8, on the device-resident state, launched as one CUDA
-graph per period; L2 is flushed (256 MiB write) between timed steps and every
-step is bracketed by CUDA events on the library's stream.  `e2e` runs the same
-metric through the C ABI with host buffers: per e2e step the state is
-uploaded, 48 iterations are advanced, the energies are measured and the state
-is read back.
+periods of resizeRate 8, on the device-resident state, in one launch of the
+persistent loop (batch64 and sphere80k: one CUDA graph per period); L2 is
+flushed (256 MiB write) between timed steps and every step is bracketed by CUDA
+events on the library's stream.  `e2e` runs the same metric through the C ABI
+with host buffers: per e2e step the state is uploaded, 48 iterations are
+advanced, the energies are measured and the state is read back.
 
 `roofline` is the whole MD step against HBM: 176 algorithmic bytes per
 bead-step (x and v FP64 read and write, the 16-byte position mirror written
 and read, the int64 force accumulator written and read) times the measured
 bead-steps/s, over the measured copy bandwidth.  `kernels` gives the same
-figure for the pair pass + integrator alone, timed per launch with CUDA
-events, and `issue` the instruction-issue bound of the step from the warp
-instructions the committed ncu capture counted.  `force_err` is the mixed
-form's force error against the oracle's FP64 forces on the bench's own state.
+figure for the pair pass + integrator alone, launched kernel by kernel in a
+pass of their own and timed per launch with CUDA events, and `issue` the
+instruction-issue bound of the step from the warp instructions the committed
+ncu capture counted.  `force_err` is the mixed form's force error against the
+oracle's FP64 forces on the bench's own state.
 
 Other workloads (--workload): vesicle5k (15,000-bead vesicle, no barostat),
 batch64 (64 independent bilayers of 1,000-8,000 lipids and tension 0-1, one
@@ -62,20 +63,15 @@ STEP_MD = 10 * PERIOD  # MD steps per bench step (20 bench steps take over 100 m
 SMS = 152          # GB300 streaming multiprocessors
 ISSUE_PER_SM_CLK = 4  # warp instructions issued per SM and clock (four schedulers)
 # DRAM bytes and warp instructions per bead and MD step of the mixed step, from
-# ncu captures of the workload (metrics dram__bytes_read.sum,
-# dram__bytes_write.sum, smsp__inst_executed.sum).  "warm" and the instructions:
-# 80 steps of the persistent loop with the caches as the previous kernels left
-# them (--cache-control none); "cold": the same step launched kernel by kernel,
-# every launch after an L2 flush, each kernel's whole working set from DRAM (an
-# upper bound).  The commands and the tables are in
-# profiles/run_loop_bilayer60k.md and profiles/step_traffic_bilayer60k.md.
-# Traffic is a named constant because ncu cannot run inside the timed region.
+# an ncu capture of the workload (metrics dram__bytes_read.sum,
+# dram__bytes_write.sum, smsp__inst_executed.sum): 80 steps of the persistent
+# loop with the caches as the previous kernels left them (--cache-control none).
+# The command and the table are in profiles/run_loop_bilayer60k.md.  Traffic is a
+# named constant because ncu cannot run inside the timed region.
 STEP_PROFILE = {
-    "bilayer20k": {"dram_bytes_per_bead_step": 13.6, "dram_bytes_per_bead_step_cold": 773.0,
-                   "warp_inst_per_bead_step": 693.0,
+    "bilayer20k": {"dram_bytes_per_bead_step": 13.6, "warp_inst_per_bead_step": 693.0,
                    "source": "profiles/run_loop_bilayer60k.md (ncu --cache-control none: the persistent loop; "
-                             "traffic and instructions) and profiles/step_traffic_bilayer60k.md (ncu, kernel by "
-                             "kernel, caches flushed per launch: an upper bound on traffic)"},
+                             "traffic and instructions)"},
 }
 
 
@@ -572,9 +568,7 @@ def main():
     prof = STEP_PROFILE.get(args.workload)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": prof["dram_bytes_per_bead_step"] * n if prof else None,
-                "traffic_cold": prof["dram_bytes_per_bead_step_cold"] * n if prof else None,
-                "traffic_per": "MD step, every kernel of the step (DRAM read + write); traffic with the caches "
-                               "as the step leaves them, traffic_cold with L2 flushed before every launch",
+                "traffic_per": "MD step (DRAM read + write) with the caches as the steps before leave them",
                 "alg_bytes_per_bead_step": ALG_BYTES_PER_BEAD_STEP, "alg_bytes_per_md_step": ALG_BYTES_PER_BEAD_STEP * n,
                 "kernel": "the whole MD step (every kernel, list builds and barostat passes included)",
                 "peak_source": f"{peak_kind} hbm_gbs"}
@@ -584,7 +578,9 @@ def main():
         kernels = {"k_force + k_integ": {
             "avg_us_per_md_step": avg_us, "achieved_gbs": ALG_BYTES_PER_BEAD_STEP * n / (avg_us * 1e3),
             "frac": ALG_BYTES_PER_BEAD_STEP * n / (avg_us * 1e3) / peak, "launch_pairs": kernel_launches,
-            "share_of_step": avg_us / us_md_step}}
+            "launched": "kernel by kernel, in a pass of their own"}}
+        if launches >= K * STEP_MD:  # (the persistent loop launches neither)
+            kernels["k_force + k_integ"]["share_of_step"] = avg_us / us_md_step
     issue = None
     if prof and clocks.get("sm_mhz"):
         inst = prof["warp_inst_per_bead_step"] * n  # per MD step
